@@ -6,6 +6,8 @@ fails, an exception is raised.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -147,6 +149,23 @@ class PeerReduceParams(C.Structure):
 
 
 _lib = None
+_native = None
+
+
+def native():
+    """The native host path of ``ops`` (csrc/binding.cpp), loaded once; raises if it has not been built."""
+    global _native
+    if _native is None:
+        import torch  # noqa: F401  (its libraries are what the module is linked against)
+        path = os.path.join(HERE, "_native.so")
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: build it with `python -m xlstm_b200.build` (there is no fallback implementation)")
+        lib()
+        loader = importlib.machinery.ExtensionFileLoader("xlstm_b200._native", path)
+        spec = importlib.util.spec_from_file_location("xlstm_b200._native", path, loader=loader)
+        _native = importlib.util.module_from_spec(spec)
+        loader.exec_module(_native)
+    return _native
 
 
 def lib() -> C.CDLL:

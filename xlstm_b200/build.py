@@ -1,11 +1,14 @@
-"""Ahead-of-time build of the C-ABI shared library (in-tree, sm_100a only).
+"""Ahead-of-time build of the C-ABI shared library and its Python binding (in-tree, sm_100a only).
 
-    python -m xlstm_b200.build            # -> xlstm_b200/libxlstm_b200.so
+    python -m xlstm_b200.build            # -> xlstm_b200/libxlstm_b200.so, xlstm_b200/_native.so
 
 nvcc cross-compiles for sm_100a without a GPU.  The library has no link-time
 dependency on libcuda (the one driver entry point it needs, the tensor-map
 encoder, is looked up at run time) and links the CUDA runtime statically, so
-it loads on a machine without a driver; only launching needs a B200.
+it loads on a machine without a driver; only launching needs a B200.  The
+binding (`csrc/binding.cpp`, the native host path of `ops.py`) is linked
+against it and against the installed PyTorch.  Sources are compiled one by
+one, in parallel, into `build/`, so a change recompiles only what it touches.
 """
 from __future__ import annotations
 
@@ -13,15 +16,19 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
+OBJ = os.path.join(HERE, "..", "build")
+HEADER = os.path.join(HERE, "..", "include", "xlstm_b200.h")
 LIB = os.path.join(HERE, "libxlstm_b200.so")
+NATIVE = os.path.join(HERE, "_native.so")
 SOURCES = ["capi.cu", "mlstm_step.cu", "mlstm_recurrent.cu", "mlstm_chunkwise.cu", "slstm_fwd.cu", "slstm_bwd.cu", "layer_adjacent.cu", "greedy_head.cu", "peer_reduce.cu", "headwise_proj.cu"]
-NVCC_FLAGS = [
-    "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "--shared", "-Xcompiler", "-fPIC",
-]
+BINDING = "binding.cpp"
+ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+NVCC_FLAGS = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 
 
 def _nvcc() -> str:
@@ -31,26 +38,58 @@ def _nvcc() -> str:
     return cand
 
 
+def _run(cmd) -> str:
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed:\n" + res.stdout + res.stderr)
+    return res.stderr
+
+
+def _newer(deps, target) -> bool:
+    return not os.path.exists(target) or any(os.path.getmtime(d) > os.path.getmtime(target) for d in deps)
+
+
+def _headers():
+    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] + [HEADER]
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
-        return True
-    t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(HERE, "..", "include", "xlstm_b200.h")]
-    return any(os.path.getmtime(d) > t for d in deps)
+    cu = [os.path.join(CSRC, s) for s in SOURCES] + _headers()
+    return _newer(cu, LIB) or _newer([os.path.join(CSRC, BINDING), HEADER], NATIVE)
+
+
+def _binding_command(obj: str):
+    import torch
+    inc = os.path.join(os.path.dirname(torch.__file__), "include")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    return ["g++", "-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", inc,
+            "-I", os.path.join(inc, "torch", "csrc", "api", "include"), "-I", cuda, "-I", sysconfig.get_paths()["include"], "-c",
+            os.path.join(CSRC, BINDING), "-o", obj]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB
-    cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB] + [os.path.join(CSRC, s) for s in SOURCES]
-    if verbose:
-        cmd.insert(1, "-Xptxas")
-        cmd.insert(2, "-v")
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    if verbose:
-        print(res.stderr)
+    import torch
+    os.makedirs(OBJ, exist_ok=True)
+    extra = ["-Xptxas", "-v"] if verbose else []
+    jobs, objs = [], []
+    for s in SOURCES:
+        src, obj = os.path.join(CSRC, s), os.path.join(OBJ, s + ".o")
+        objs.append(obj)
+        if force or _newer([src, *_headers()], obj):
+            jobs.append([_nvcc(), *extra, *NVCC_FLAGS, "-c", src, "-o", obj])
+    bobj = os.path.join(OBJ, BINDING + ".o")
+    if force or _newer([os.path.join(CSRC, BINDING), HEADER], bobj):
+        jobs.append(_binding_command(bobj))
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        for log in pool.map(_run, jobs):
+            if verbose:
+                print(log)
+    _run([_nvcc(), *ARCH, "--shared", "-Xlinker", "-soname=libxlstm_b200.so", "-o", LIB, *objs])
+    tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    _run(["g++", "-shared", "-o", NATIVE, bobj, LIB, "-L", tlib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+          "-Wl,-rpath,$ORIGIN"])
     return LIB
 
 

@@ -92,7 +92,7 @@ typedef struct xl_mlstm_seq_params {
  * sequence kernel.  Returns XL_ERR_UNSUPPORTED for other shapes (use xl_mlstm_recurrent). */
 int xl_mlstm_chunkwise(const xl_mlstm_seq_params* p, void* cuda_stream);
 
-/* Token-by-token recurrence with the C state held on chip (exact fp32 arithmetic; the reference's
+/* fp32 arithmetic throughout, in chunks of 32 tokens with the C state held on chip (the reference's
  * `native_sequence__native` contract).  dtype XL_F32 or XL_BF16, any DHQK <= 512, any DHV. */
 int xl_mlstm_recurrent(const xl_mlstm_seq_params* p, void* cuda_stream);
 

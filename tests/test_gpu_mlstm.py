@@ -102,6 +102,20 @@ def test_recurrent_fp32_config1_shape():
     _check(h, st, h_ref, st_ref, TOL_F32)
 
 
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, TOL_F32), (torch.bfloat16, TOL_BF16)])
+@pytest.mark.parametrize("B,NH,S,DQ,DV,with_state", [
+    (1, 2, 1, 64, 128, True), (2, 1, 31, 36, 36, False), (1, 1, 32, 6, 33, True), (1, 2, 33, 100, 130, True),
+    (2, 3, 69, 64, 32, False), (1, 1, 97, 260, 64, True), (1, 1, 40, 512, 40, False), (1, 1, 64, 512, 31, True)])
+def test_recurrent_at_the_edges_of_its_tiles(dtype, tol, B, NH, S, DQ, DV, with_state):
+    """Chunks of 32 tokens, 32 columns per thread block, features in fours, one buffer instead of two beyond 256 features."""
+    import xlstm_b200
+    q, k, v, i, f = _inputs(51, B, NH, S, DQ, DV, dtype)
+    init = _state(52, B, NH, DQ, DV) if with_state else (None, None, None)
+    h_ref, st_ref = O.mlstm_sequence(q, k, v, i, f, *init)
+    h, st = xlstm_b200.mlstm_sequence(*_cuda(q, k, v, i, f), *_cuda(*init), kernel="recurrent")
+    _check(h, st, h_ref, st_ref, tol)
+
+
 # ------------------------------------------------------------------------------------------------ chunkwise (tcgen05)
 @pytest.mark.parametrize("B,NH,S,DQ,DV,with_state", [
     (2, 2, 256, 64, 128, False),

@@ -1,36 +1,71 @@
-// mLSTM token-by-token recurrence over a sequence, fp32 arithmetic throughout.
+// mLSTM over a sequence in fp32 arithmetic throughout (operands, products, accumulation, state).
 //
-// One CTA owns a REC_COLS-wide column slice of one document's C matrix and keeps it in shared memory for
-// the whole document: per token it applies  C' = f'C + i' k v^T,  accumulates q~^T C' for its columns,
-// updates n and writes h.  Only q,k,v,i,f are read from and h written to global memory per token; the
-// state touches HBM once at the start (initial state) and once at the end (final state).
 // It serves (a) fp32 models, where the tensor-core chunkwise kernel's bf16 operands would break the 1e-4
 // tolerance, (b) head sizes the chunkwise kernel does not cover, and it is the on-device cross-check for
 // the chunkwise kernel in the tests.
+//
+// One CTA owns a 32-column slice of one document's C matrix, keeps it transposed in shared memory for the whole document
+// and walks the document in chunks of 32 tokens -- one warp's width, so every warp forms the gate recurrence of a chunk with
+// shuffles, lane = token.  With b_j the in-chunk cumulative log forget gate, a_l = i_l - b_l, mu_j = max(m_prev, max_{l<=j} a_l):
+//   [S | QC] = Q [K ; C^T]^T      P_jl = S_jl / sqrt(d) exp(a_l - mu_j) (l <= j)      r_j = exp(m_prev - mu_j) / sqrt(d)
+//   h_j = (r_j QC_j + sum_l P_jl v_l) / (max(|r_j q_j.n + sum_l P_jl|, exp(-(b_j + mu_j))) + eps)
+//   C <- exp(m_prev - mu_31) C + sum_l w_l k_l v_l^T,  n likewise,  w_l = exp(a_l - mu_31),  m <- b_31 + mu_31
+// Token by token the kernel was a chain of two CTA barriers and a column reduction per token, 1.6 us each; a chunk
+// is two barriers for 32 tokens, and the products run from registers at 2 x 4 outputs per thread (six 16-byte
+// shared-memory loads per 32 FMAs).  Chunks of 64 would double the redundant part of the work (S, formed by every slice).
 #include "common.cuh"
 
 namespace xl {
 
 constexpr int REC_THREADS = 256;
-constexpr int REC_COLS = 64;                      // C columns per CTA
-constexpr int REC_RG = REC_THREADS / REC_COLS;    // row groups (4)
+constexpr int REC_L = 32;                         // tokens per chunk
+constexpr int REC_COLS = 32;                      // C columns per CTA
+constexpr int REC_LP = REC_L + 4;                 // padded row of the token-indexed tiles (floats)
+
+__device__ __forceinline__ void rec_cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void rec_cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
+  acc = fmaf(a.x, b.x, acc);
+  acc = fmaf(a.y, b.y, acc);
+  acc = fmaf(a.z, b.z, acc);
+  return fmaf(a.w, b.w, acc);
+}
+
+// shared memory (floats); rows of DP = DHQK rounded up to 4, plus 4: eight rows' 16-byte pieces then lie on distinct banks
+struct RecLayout {
+  int DQ4, DP, nbuf;
+  size_t q, k, vt, vw, c, pm, n, total;
+  __host__ __device__ explicit RecLayout(int DHQK) {
+    DQ4 = (DHQK + 3) / 4;
+    DP = 4 * DQ4 + 4;
+    nbuf = DHQK <= 256 ? 2 : 1;                   // two chunks in flight where they fit
+    q = 0;
+    k = q + (size_t)nbuf * REC_L * DP;
+    vt = k + (size_t)nbuf * REC_L * DP;           // v transposed [column][token]
+    vw = vt + (size_t)nbuf * REC_COLS * REC_LP;   // the same times w_l
+    c = vw + (size_t)REC_COLS * REC_LP;           // C^T [column][feature]
+    pm = c + (size_t)REC_COLS * DP;               // P [row][token]
+    n = pm + (size_t)REC_L * REC_LP;
+    total = n + (size_t)DP;
+  }
+};
 
 template <typename T>
-__global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_mlstm_seq_params p) {
+__global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_mlstm_seq_params p, int vec) {
   extern __shared__ __align__(16) float smem[];
-  const int DHQK = p.DHQK, DHV = p.DHV;
-  float* s_C = smem;                                 // DHQK x REC_COLS
-  float* s_n = s_C + (size_t)DHQK * REC_COLS;        // DHQK
-  float* s_q = s_n + DHQK;                           // 2 x DHQK (double buffered by token parity)
-  float* s_k = s_q + 2 * DHQK;                       // 2 x DHQK
-  float* s_part = s_k + 2 * DHQK;                    // REC_RG x REC_COLS
-  __shared__ float s_red[REC_THREADS / 32];
+  const RecLayout ly(p.DHQK);
+  const int DHQK = p.DHQK, DHV = p.DHV, DQ4 = ly.DQ4, DP = ly.DP;
+  float* s_c = smem + ly.c;
+  float* s_n = smem + ly.n;
+  float* s_p = smem + ly.pm;
+  float* s_vw = smem + ly.vw;
 
   const int doc = blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * REC_COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c = tid % REC_COLS, rg = tid / REC_COLS;
-  const int col = col0 + c;
-  const bool col_ok = col < DHV;
 
   // document -> (batch row, first token, length)
   int64_t tok0, len;
@@ -50,93 +85,216 @@ __global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_m
   const float* ig = p.igate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
   const float* fg = p.fgate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
   const int64_t sidx = (int64_t)doc * p.NH + head;
+  const float qscale = rsqrtf((float)DHQK);
+  const int nchunks = (int)((len + REC_L - 1) / REC_L);
+
+  // q, k, v of a chunk into buffer `buf`; rows past the document, features past DHQK and columns past DHV are zero.  The
+  // pieces a thread loads are the same for all tiles of a shape: 16-byte copies where rows are aligned (`vec`).
+  auto load_chunk = [&](int chunk, int buf) {
+    float* tq = smem + ly.q + (size_t)buf * REC_L * DP;
+    float* tk = smem + ly.k + (size_t)buf * REC_L * DP;
+    float* tv = smem + ly.vt + (size_t)buf * REC_COLS * REC_LP;
+    const int64_t t0 = (int64_t)chunk * REC_L;
+    const int rows = (int)(len - t0 < REC_L ? len - t0 : REC_L);
+    if (sizeof(T) == 4 && vec) {
+      for (int u = tid; u < REC_L * DQ4; u += REC_THREADS) {
+        const int r = u / DQ4, d = 4 * (u - r * DQ4);
+        if (r < rows) {
+          rec_cp_async16(smem_u32(tq + r * DP + d), q + (t0 + r) * p.q_st + d);
+          rec_cp_async16(smem_u32(tk + r * DP + d), k + (t0 + r) * p.k_st + d);
+        } else {
+          *reinterpret_cast<float4*>(tq + r * DP + d) = make_float4(0.f, 0.f, 0.f, 0.f);
+          *reinterpret_cast<float4*>(tk + r * DP + d) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+    } else {
+      const int D = 4 * DQ4;
+#pragma unroll 4
+      for (int u = tid; u < REC_L * D; u += REC_THREADS) {
+        const int r = u / D, d = u - r * D;
+        const bool in = r < rows && d < DHQK;
+        tq[r * DP + d] = in ? to_float(q[(t0 + r) * p.q_st + d]) : 0.f;
+        tk[r * DP + d] = in ? to_float(k[(t0 + r) * p.k_st + d]) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int u = tid; u < REC_L * REC_COLS; u += REC_THREADS) {   // a warp takes one token's columns
+      const int r = u / REC_COLS, c = u % REC_COLS;
+      const bool in = r < rows && col0 + c < DHV;
+      const T* src = v + (t0 + r) * p.v_st + col0 + c;
+      if (sizeof(T) == 4 && in) rec_cp_async4(smem_u32(tv + c * REC_LP + r), src);
+      else tv[c * REC_LP + r] = in ? to_float(*src) : 0.f;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
 
   // initial state
-  for (int r = rg; r < DHQK; r += REC_RG)
-    s_C[r * REC_COLS + c] = (p.c0 && col_ok) ? p.c0[(sidx * DHQK + r) * DHV + col] : 0.f;
-  for (int d = tid; d < DHQK; d += REC_THREADS) s_n[d] = p.n0 ? p.n0[sidx * DHQK + d] : 0.f;
-  float m = p.m0 ? p.m0[sidx] : 0.f;
-  const float qscale = rsqrtf((float)DHQK);
+  for (int u = tid; u < REC_COLS * 4 * DQ4; u += REC_THREADS) {
+    const int d = u / REC_COLS, c = u % REC_COLS;
+    s_c[c * DP + d] = (p.c0 && d < DHQK && col0 + c < DHV) ? p.c0[(sidx * DHQK + d) * DHV + col0 + c] : 0.f;
+  }
+  for (int d = tid; d < 4 * DQ4; d += REC_THREADS) s_n[d] = (p.n0 && d < DHQK) ? p.n0[sidx * DHQK + d] : 0.f;
+  float m_prev = p.m0 ? p.m0[sidx] : 0.f;
 
-  // prefetch token 0 into buffer 0
-  if (len > 0)
-    for (int d = tid; d < DHQK; d += REC_THREADS) {
-      s_q[d] = to_float(q[d]) * qscale;
-      s_k[d] = to_float(k[d]);
+  // output tile of a thread: rows j0, j0 + 16; S columns / value columns c0, c0 + 16
+  const int j0 = (warp & 3) * 4 + (lane >> 3), c0 = (warp >> 2) * 8 + (lane & 7);
+
+  if (nchunks > 0) load_chunk(0, 0);
+  float gi = lane < len ? ig[lane * p.g_st] : 0.f, gf = lane < len ? fg[lane * p.g_st] : 0.f;
+  for (int chunk = 0; chunk < nchunks; ++chunk) {
+    const int buf = chunk % ly.nbuf;
+    const float* tq = smem + ly.q + (size_t)buf * REC_L * DP;
+    const float* tk = smem + ly.k + (size_t)buf * REC_L * DP;
+    const float* tv = smem + ly.vt + (size_t)buf * REC_COLS * REC_LP;
+    const int64_t t0 = (int64_t)chunk * REC_L;
+    // ---- gate recurrence of the chunk, lane = token; every warp forms it for itself
+    const bool live = t0 + lane < len;
+    float bcum = live ? log_sigmoid(gf) : 0.f;
+    const float iv = gi;
+    {
+      const int64_t tn = t0 + REC_L + lane;   // the next chunk's gates
+      gi = tn < len ? ig[tn * p.g_st] : 0.f;
+      gf = tn < len ? fg[tn * p.g_st] : 0.f;
     }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_up_sync(0xffffffffu, bcum, o);
+      if (lane >= o) bcum += t;
+    }
+    const float al = live ? iv - bcum : -INFINITY;
+    float mu = fmaxf(al, m_prev);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_up_sync(0xffffffffu, mu, o);
+      if (lane >= o) mu = fmaxf(mu, t);
+    }
+    const float mu_last = __shfl_sync(0xffffffffu, mu, 31), b_last = __shfl_sync(0xffffffffu, bcum, 31);
+    const float r_tok = expf(m_prev - mu) * qscale, lower = expf(-(bcum + mu)), w_tok = expf(al - mu_last);
+    const float decay = expf(m_prev - mu_last);
+    m_prev = b_last + mu_last;
+
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();   // the chunk is in shared memory; C and n of the previous chunk are complete
+    if (ly.nbuf == 2 && chunk + 1 < nchunks) load_chunk(chunk + 1, buf ^ 1);
+
+    // ---- [S | QC] = Q [K ; C^T]^T, 2 x (2 + 2) outputs per thread
+    float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, qc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    {
+      const float *q0 = tq + j0 * DP, *q1 = q0 + 16 * DP, *k0 = tk + c0 * DP, *k1 = k0 + 16 * DP, *x0 = s_c + c0 * DP, *x1 = x0 + 16 * DP;
+#pragma unroll 4
+      for (int d = 0; d < 4 * DQ4; d += 4) {
+        const float4 a0 = *reinterpret_cast<const float4*>(q0 + d), a1 = *reinterpret_cast<const float4*>(q1 + d);
+        const float4 b0 = *reinterpret_cast<const float4*>(k0 + d), b1 = *reinterpret_cast<const float4*>(k1 + d);
+        const float4 e0 = *reinterpret_cast<const float4*>(x0 + d), e1 = *reinterpret_cast<const float4*>(x1 + d);
+        s[0][0] = dot4(a0, b0, s[0][0]); s[0][1] = dot4(a0, b1, s[0][1]);
+        s[1][0] = dot4(a1, b0, s[1][0]); s[1][1] = dot4(a1, b1, s[1][1]);
+        qc[0][0] = dot4(a0, e0, qc[0][0]); qc[0][1] = dot4(a0, e1, qc[0][1]);
+        qc[1][0] = dot4(a1, e0, qc[1][0]); qc[1][1] = dot4(a1, e1, qc[1][1]);
+      }
+    }
+    // ---- q_j . n of the four rows this warp's threads 8 i hold (rows 4 (warp % 4) + i and + 16): lane over features
+    float qn0 = 0.f, qn1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float x = 0.f, y = 0.f;
+      const float *ra = tq + ((warp & 3) * 4 + i) * DP, *rb = ra + 16 * DP;
+      for (int d = lane; d < DHQK; d += 32) {
+        x = fmaf(ra[d], s_n[d], x);
+        y = fmaf(rb[d], s_n[d], y);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        x += __shfl_xor_sync(0xffffffffu, x, o);
+        y += __shfl_xor_sync(0xffffffffu, y, o);
+      }
+      if ((lane >> 3) == i) { qn0 = x; qn1 = y; }
+    }
+    // ---- P and the w-scaled v
+    const float mu0 = __shfl_sync(0xffffffffu, mu, j0), mu1 = __shfl_sync(0xffffffffu, mu, j0 + 16);
+    const float al0 = __shfl_sync(0xffffffffu, al, c0), al1 = __shfl_sync(0xffffffffu, al, c0 + 16);
+    s_p[j0 * REC_LP + c0] = c0 <= j0 ? s[0][0] * qscale * expf(al0 - mu0) : 0.f;
+    s_p[j0 * REC_LP + c0 + 16] = 0.f;                                              // (c0 + 16 > j0)
+    s_p[(j0 + 16) * REC_LP + c0] = s[1][0] * qscale * expf(al0 - mu1);             // (c0 < j0 + 16)
+    s_p[(j0 + 16) * REC_LP + c0 + 16] = c0 <= j0 ? s[1][1] * qscale * expf(al1 - mu1) : 0.f;
+#pragma unroll
+    for (int i = 0; i < REC_COLS / 8; ++i) s_vw[(warp * (REC_COLS / 8) + i) * REC_LP + lane] = tv[(warp * (REC_COLS / 8) + i) * REC_LP + lane] * w_tok;
+    __syncthreads();   // P and the scaled v are complete, C and n are read
+
+    // ---- h = (r QC + P V) / den
+    {
+      float o[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, rs0 = 0.f, rs1 = 0.f;
+      const float *p0 = s_p + j0 * REC_LP, *p1 = p0 + 16 * REC_LP, *v0 = tv + c0 * REC_LP, *v1 = v0 + 16 * REC_LP;
+#pragma unroll
+      for (int l = 0; l < REC_L; l += 4) {
+        const float4 b0 = *reinterpret_cast<const float4*>(v0 + l), b1 = *reinterpret_cast<const float4*>(v1 + l);
+        const float4 a1 = *reinterpret_cast<const float4*>(p1 + l);
+        if (l < 16) {   // row j0 < 16 has no later tokens
+          const float4 a0 = *reinterpret_cast<const float4*>(p0 + l);
+          o[0][0] = dot4(a0, b0, o[0][0]); o[0][1] = dot4(a0, b1, o[0][1]);
+          rs0 += (a0.x + a0.y) + (a0.z + a0.w);
+        }
+        o[1][0] = dot4(a1, b0, o[1][0]); o[1][1] = dot4(a1, b1, o[1][1]);
+        rs1 += (a1.x + a1.y) + (a1.z + a1.w);
+      }
+      const float r0 = __shfl_sync(0xffffffffu, r_tok, j0), r1 = __shfl_sync(0xffffffffu, r_tok, j0 + 16);
+      const float lo0 = __shfl_sync(0xffffffffu, lower, j0), lo1 = __shfl_sync(0xffffffffu, lower, j0 + 16);
+      const float den0 = fmaxf(fabsf(fmaf(r0, qn0, rs0)), lo0) + p.eps, den1 = fmaxf(fabsf(fmaf(r1, qn1, rs1)), lo1) + p.eps;
+      T* h0 = h + (t0 + j0) * p.h_st + col0 + c0;
+      T* h1 = h0 + 16 * p.h_st;
+      const bool ok0 = col0 + c0 < DHV, ok1 = col0 + c0 + 16 < DHV;
+      if (t0 + j0 < len) {
+        if (ok0) h0[0] = from_float<T>(fmaf(r0, qc[0][0], o[0][0]) / den0);
+        if (ok1) h0[16] = from_float<T>(fmaf(r0, qc[0][1], o[0][1]) / den0);
+      }
+      if (t0 + j0 + 16 < len) {
+        if (ok0) h1[0] = from_float<T>(fmaf(r1, qc[1][0], o[1][0]) / den1);
+        if (ok1) h1[16] = from_float<T>(fmaf(r1, qc[1][1], o[1][1]) / den1);
+      }
+    }
+    // ---- C^T <- decay C^T + (w v)^T K: units of two columns x four features
+    for (int u = tid; u < (REC_COLS / 2) * DQ4; u += REC_THREADS) {
+      const int cp = u / DQ4, d = 4 * (u - cp * DQ4);
+      float4* x0 = reinterpret_cast<float4*>(s_c + cp * DP + d);
+      float4* x1 = reinterpret_cast<float4*>(s_c + (cp + 16) * DP + d);
+      float4 a = *x0, e = *x1;
+      a.x *= decay; a.y *= decay; a.z *= decay; a.w *= decay;
+      e.x *= decay; e.y *= decay; e.z *= decay; e.w *= decay;
+#pragma unroll
+      for (int l = 0; l < REC_L; l += 4) {
+        const float4 wa = *reinterpret_cast<const float4*>(s_vw + cp * REC_LP + l), we = *reinterpret_cast<const float4*>(s_vw + (cp + 16) * REC_LP + l);
+        const float ca[4] = {wa.x, wa.y, wa.z, wa.w}, ce[4] = {we.x, we.y, we.z, we.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 kk = *reinterpret_cast<const float4*>(tk + (l + i) * DP + d);
+          a.x = fmaf(ca[i], kk.x, a.x); a.y = fmaf(ca[i], kk.y, a.y); a.z = fmaf(ca[i], kk.z, a.z); a.w = fmaf(ca[i], kk.w, a.w);
+          e.x = fmaf(ce[i], kk.x, e.x); e.y = fmaf(ce[i], kk.y, e.y); e.z = fmaf(ce[i], kk.z, e.z); e.w = fmaf(ce[i], kk.w, e.w);
+        }
+      }
+      *x0 = a;
+      *x1 = e;
+    }
+    // ---- n <- decay n + sum_l w_l k_l: warp i takes features i, i + 8, ...; lane = token
+    for (int d = warp; d < DHQK; d += REC_THREADS / 32) {
+      float x = tk[lane * DP + d] * w_tok;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      if (lane == 0) s_n[d] = fmaf(decay, s_n[d], x);
+    }
+    if (ly.nbuf == 1 && chunk + 1 < nchunks) {
+      __syncthreads();   // the only buffer is free
+      load_chunk(chunk + 1, 0);
+    }
+  }
   __syncthreads();
 
-  for (int64_t t = 0; t < len; ++t) {
-    const int cur = (int)(t & 1), nxt = cur ^ 1;
-    const float* sq = s_q + cur * DHQK;
-    const float* sk = s_k + cur * DHQK;
-    // issue next token's loads early (registers), store them to the other buffer after the math
-    float qn_[2], kn_[2];  // up to 2 elements per thread (DHQK <= 512)
-    const bool more = t + 1 < len;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int d = tid + u * REC_THREADS;
-      if (more && d < DHQK) {
-        qn_[u] = to_float(q[(t + 1) * p.q_st + d]) * qscale;
-        kn_[u] = to_float(k[(t + 1) * p.k_st + d]);
-      }
-    }
-    const float vv = col_ok ? to_float(v[t * p.v_st + col]) : 0.f;
-    const float logf = log_sigmoid(fg[t * p.g_st]);
-    const float iv = ig[t * p.g_st];
-    const float m_new = fmaxf(logf + m, iv);
-    const float f_act = expf(logf + m - m_new);
-    const float i_act = expf(iv - m_new);
-
-    // column slice update + partial q~^T C'
-    float acc = 0.f;
-    const float iv_v = i_act * vv;
-#pragma unroll 8
-    for (int r = rg; r < DHQK; r += REC_RG) {
-      const float cn = fmaf(f_act, s_C[r * REC_COLS + c], sk[r] * iv_v);
-      s_C[r * REC_COLS + c] = cn;
-      acc = fmaf(sq[r], cn, acc);
-    }
-    s_part[rg * REC_COLS + c] = acc;
-    // n update and q~ . n'
-    float qn = 0.f;
-    for (int d = tid; d < DHQK; d += REC_THREADS) {
-      const float nn = fmaf(f_act, s_n[d], i_act * sk[d]);
-      s_n[d] = nn;
-      qn = fmaf(sq[d], nn, qn);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) qn += __shfl_xor_sync(0xffffffffu, qn, o);
-    if (lane == 0) s_red[warp] = qn;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int d = tid + u * REC_THREADS;
-      if (more && d < DHQK) {
-        s_q[nxt * DHQK + d] = qn_[u];
-        s_k[nxt * DHQK + d] = kn_[u];
-      }
-    }
-    __syncthreads();
-    if (tid < REC_COLS && col0 + tid < DHV) {
-      float tot = 0.f;
-#pragma unroll
-      for (int w = 0; w < REC_THREADS / 32; ++w) tot += s_red[w];
-      float num = 0.f;
-#pragma unroll
-      for (int g = 0; g < REC_RG; ++g) num += s_part[g * REC_COLS + tid];
-      const float den = fmaxf(fabsf(tot), expf(-m_new)) + p.eps;
-      h[t * p.h_st + col0 + tid] = from_float<T>(num / den);
-    }
-    m = m_new;
-    __syncthreads();
-  }
-
   // final state
-  for (int r = rg; r < DHQK; r += REC_RG)
-    if (col_ok) p.c_out[(sidx * DHQK + r) * DHV + col] = s_C[r * REC_COLS + c];
+  for (int u = tid; u < REC_COLS * DHQK; u += REC_THREADS) {
+    const int d = u / REC_COLS, c = u % REC_COLS;
+    if (col0 + c < DHV) p.c_out[(sidx * DHQK + d) * DHV + col0 + c] = s_c[c * DP + d];
+  }
   if (blockIdx.x == 0) {
     for (int d = tid; d < DHQK; d += REC_THREADS) p.n_out[sidx * DHQK + d] = s_n[d];
-    if (tid == 0) p.m_out[sidx] = m;
+    if (tid == 0) p.m_out[sidx] = m_prev;
   }
 }
 
@@ -155,24 +313,26 @@ int validate_seq_common(const xl_mlstm_seq_params* p) {
   return XL_OK;
 }
 
+template <typename T>
+static int launch_recurrent(const xl_mlstm_seq_params* p, size_t smem, cudaStream_t st) {
+  auto kern = mlstm_recurrent_kernel<T>;
+  XL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int nd = p->cu_seqlens ? p->num_docs : p->B;
+  // 16-byte copies of q and k rows (fp32): every row starts on a 16-byte boundary and is a whole number of pieces
+  const bool vec = aligned16(p->q) && aligned16(p->k) && p->DHQK % 4 == 0 &&
+                   !((p->q_sb | p->q_sh | p->q_st | p->k_sb | p->k_sh | p->k_st) & 3);
+  kern<<<dim3((p->DHV + REC_COLS - 1) / REC_COLS, p->NH, nd), REC_THREADS, smem, st>>>(*p, vec ? 1 : 0);
+  return check_launch("xl_mlstm_recurrent");
+}
+
 }  // namespace xl
 
 extern "C" int xl_mlstm_recurrent(const xl_mlstm_seq_params* p, void* cuda_stream) {
   using namespace xl;
   int rc = validate_seq_common(p);
   if (rc != XL_OK) return rc;
-  if (p->DHQK > 2 * REC_THREADS) return XL_ERR_BAD_SHAPE;
-  const int nd = p->cu_seqlens ? p->num_docs : p->B;
-  const size_t smem = ((size_t)p->DHQK * REC_COLS + 5 * (size_t)p->DHQK + REC_RG * REC_COLS) * sizeof(float);
-  if (smem > 200 * 1024) return XL_ERR_BAD_SHAPE;
-  dim3 grid((p->DHV + REC_COLS - 1) / REC_COLS, p->NH, nd), block(REC_THREADS);
+  if (p->DHQK > 512) return XL_ERR_BAD_SHAPE;
+  const size_t smem = RecLayout(p->DHQK).total * sizeof(float);
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
-  if (p->dtype == XL_F32) {
-    XL_CUDA_TRY(cudaFuncSetAttribute(mlstm_recurrent_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    mlstm_recurrent_kernel<float><<<grid, block, smem, st>>>(*p);
-  } else {
-    XL_CUDA_TRY(cudaFuncSetAttribute(mlstm_recurrent_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    mlstm_recurrent_kernel<__nv_bfloat16><<<grid, block, smem, st>>>(*p);
-  }
-  return check_launch("xl_mlstm_recurrent");
+  return p->dtype == XL_F32 ? launch_recurrent<float>(p, smem, st) : launch_recurrent<__nv_bfloat16>(p, smem, st);
 }

@@ -92,6 +92,14 @@ typedef struct xl_mlstm_seq_params {
  * sequence kernel.  Returns XL_ERR_UNSUPPORTED for other shapes (use xl_mlstm_recurrent). */
 int xl_mlstm_chunkwise(const xl_mlstm_seq_params* p, void* cuda_stream);
 
+/* The same computation for callers that lend scratch memory: documents too long for the number of (document, head,
+ * 128-column) chains are cut into parts that run side by side, and packed documents are taken longest first.  `scratch`
+ * (device, 16-byte aligned) needs xl_mlstm_chunkwise_scratch_bytes(p) bytes -- a host-only computation from the sizes in
+ * `p`, 0 where the split would not pay; contents need not be initialised and are free again when the call's kernels have
+ * run.  With scratch == NULL, or where the split would not pay, this is xl_mlstm_chunkwise. */
+int64_t xl_mlstm_chunkwise_scratch_bytes(const xl_mlstm_seq_params* p);
+int xl_mlstm_chunkwise_parts(const xl_mlstm_seq_params* p, void* scratch, int64_t scratch_bytes, void* cuda_stream);
+
 /* fp32 arithmetic throughout, in chunks of 32 tokens with the C state held on chip (the reference's
  * `native_sequence__native` contract).  dtype XL_F32 or XL_BF16, any DHQK <= 512, any DHV. */
 int xl_mlstm_recurrent(const xl_mlstm_seq_params* p, void* cuda_stream);

@@ -161,6 +161,44 @@ def test_chunkwise_cluster_shared_normaliser_opt_in(cluster, DQ, DV):
     assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-2000:]
 
 
+@pytest.mark.parametrize("B,NH,S,DQ,DV,with_state,f_mean", [
+    (1, 1, 2496, 64, 128, False, 3.0),    # 39 chunks: parts of unequal length
+    (1, 2, 2000, 256, 512, True, 3.0),    # initial state, a tail chunk in the last part
+    (1, 1, 4096, 128, 256, True, -2.0),   # strong decay: the states of early parts vanish
+    (1, 1, 2048, 256, 128, False, 3.0),   # one value slice forms every feature block of n
+    (4, 2, 3000, 64, 256, False, 3.0),    # several rows, a short tail
+])
+def test_chunkwise_split_into_parts_matches_oracle(B, NH, S, DQ, DV, with_state, f_mean):
+    """Sizes whose documents are cut into parts: the C entry says so through the scratch it asks for."""
+    import ctypes
+    import xlstm_b200
+    from xlstm_b200 import _lib
+    p = _lib.MlstmSeqParams()
+    p.B, p.NH, p.S, p.DHQK, p.DHV = B, NH, S, DQ, DV
+    assert _lib.lib().xl_mlstm_chunkwise_scratch_bytes(ctypes.byref(p)) > 0
+    q, k, v, i, f = _inputs(61, B, NH, S, DQ, DV, torch.bfloat16, f_mean=f_mean)
+    if f_mean < 0:
+        i[:, :, S // 2:] += 25.0          # the stabiliser jumps between parts
+    init = _state(62, B, NH, DQ, DV) if with_state else (None, None, None)
+    h_ref, st_ref = O.mlstm_inference(q, k, v, i, f, *init)
+    h, st = xlstm_b200.mlstm_sequence(*_cuda(q, k, v, i, f), *_cuda(*init), kernel="chunkwise")
+    xlstm_b200.check_device_status()
+    _check(h, st, h_ref, st_ref, TOL_BF16)
+
+
+def test_chunkwise_packed_documents_longer_than_a_part():
+    """Packed rows with documents far above and far below the length of a part, empty ones among them."""
+    import xlstm_b200
+    B, NH, S, DQ, DV = 2, 1, 4096, 64, 128
+    cu = [0, 1, 1, 3000, 3064, 4095, 4096, 4096 + 4096, 8192]
+    q, k, v, i, f = _inputs(63, B, NH, S, DQ, DV, torch.bfloat16)
+    flat = lambda t: t.transpose(0, 1).reshape(NH, B * S, *t.shape[3:])
+    h_ref, st_ref = O.mlstm_packed(flat(q), flat(k), flat(v), flat(i), flat(f), cu)
+    h, st = xlstm_b200.mlstm_sequence(*_cuda(q, k, v, i, f), cu_seqlens=cu, kernel="chunkwise")
+    xlstm_b200.check_device_status()
+    _check(flat(h.cpu()), st, h_ref, st_ref, TOL_BF16)
+
+
 def test_chunkwise_harsh_gates_stay_finite_and_match():
     """Forget gates around -6 (strong decay) and input gates with a wide spread exercise the stabilisers."""
     import xlstm_b200

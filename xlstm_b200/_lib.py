@@ -17,7 +17,7 @@ XL_F32, XL_BF16 = 0, 1
 
 EXPORTS = (
     "xl_strerror", "xl_last_cuda_error", "xl_abi_version",
-    "xl_mlstm_chunkwise", "xl_mlstm_recurrent", "xl_mlstm_step", "xl_slstm_forward",
+    "xl_mlstm_chunkwise", "xl_mlstm_chunkwise_parts", "xl_mlstm_chunkwise_scratch_bytes", "xl_mlstm_recurrent", "xl_mlstm_step", "xl_slstm_forward",
     "xl_add_rmsnorm", "xl_headnorm_gate", "xl_soft_cap", "xl_causal_conv1d",
     "xl_softcap_argmax", "xl_softcap_argmax_scratch_bytes", "xl_swiglu",
     "xl_softcap_argmax_noalloc", "xl_softcap_argmax_noalloc_max_rows", "xl_peer_reduce_add_rmsnorm", "xl_headwise_proj", "xl_mlstm_decode_cell",
@@ -191,6 +191,10 @@ def lib() -> C.CDLL:
             fn = getattr(l, name)
             fn.restype = C.c_int
             fn.argtypes = [C.POINTER(ptype), C.c_void_p]
+        l.xl_mlstm_chunkwise_parts.restype = C.c_int
+        l.xl_mlstm_chunkwise_parts.argtypes = [C.POINTER(MlstmSeqParams), C.c_void_p, C.c_int64, C.c_void_p]
+        l.xl_mlstm_chunkwise_scratch_bytes.restype = C.c_int64
+        l.xl_mlstm_chunkwise_scratch_bytes.argtypes = [C.POINTER(MlstmSeqParams)]
         l.xl_softcap_argmax_scratch_bytes.restype = C.c_int64
         l.xl_softcap_argmax_scratch_bytes.argtypes = [C.c_int32]
         l.xl_softcap_argmax_noalloc_max_rows.restype = C.c_int32

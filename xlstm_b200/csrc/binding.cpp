@@ -158,7 +158,11 @@ PyObject* mlstm_sequence(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.h_sb = h.stride(0); p.h_sh = h.stride(1); p.h_st = h.stride(2);
   p.g_sb = i.stride(0); p.g_sh = i.stride(1); p.g_st = i.stride(2);
   p.eps = (float)double_arg(a[10]); p.dtype = dtype_code(q);
-  if (kernel == 1) check(xl_mlstm_chunkwise(&p, stream_of(q)), "xl_mlstm_chunkwise");
+  if (kernel == 1) {
+    const int64_t bytes = xl_mlstm_chunkwise_scratch_bytes(&p);
+    const Tensor scratch = bytes ? empty_on({bytes}, at::kByte, q) : Tensor();   // (stream-ordered: free for the allocator at return)
+    check(xl_mlstm_chunkwise_parts(&p, bytes ? scratch.data_ptr() : nullptr, bytes, stream_of(q)), "xl_mlstm_chunkwise");
+  }
   else check(xl_mlstm_recurrent(&p, stream_of(q)), "xl_mlstm_recurrent");
   return pack_pair(THPVariable_Wrap(h), pack({c, n, m}));
   END_HANDLE_TH_ERRORS

@@ -25,6 +25,27 @@ int check_launch(const char* where);  // cudaPeekAtLastError -> XL_OK / XL_ERR_C
     }                                                       \
   } while (0)
 
+// Launch with programmatic dependence: the grid may be scheduled while the kernel in front of it in the stream still runs,
+// once all blocks of that one have called grid_dependents_launch() or ended.  Every kernel launched this way calls
+// grid_dependency_wait() before it touches global memory; what it does before that (barriers, tensor memory, constants)
+// hides behind the predecessor's tail, and a back-to-back launch costs ~1 us less.
+template <typename... P, typename... A>
+static inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---------------------------------------------------------------------------------------------

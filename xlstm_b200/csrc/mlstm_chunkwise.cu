@@ -50,17 +50,12 @@
 // q, k, v tiles arrive by TMA (128-byte swizzle) straight from the caller's strided (B, NH, S, D) views;
 // documents are chunked from their own first token, so a chunk never straddles a document boundary and the
 // tail chunk is masked (i = -inf, log f = 0) instead of padded.
-#include <cuda.h>
-
-#include "common.cuh"
+#include "mlstm_chunkwise.cuh"
 
 namespace xl {
 
-constexpr int CW_L = 64;         // tokens per chunk
-constexpr int CW_DV = 128;       // value columns per CTA (UMMA M)
 constexpr int CW_THREADS = 480;  // 15 warps, see roles above
 constexpr int CW_STAGES = 2;
-constexpr int CW_BOX_BYTES = 64 * 128;  // one TMA box: 64 rows x 64 bf16
 constexpr uint32_t CW_TMEM_COLS = 512;
 constexpr float CW_RESCALE_BELOW = -30.f;  // lazy-decay frame limit (natural log)
 constexpr float CW_LOG2E = 1.4426950408889634f;
@@ -108,7 +103,6 @@ enum CwBar {  // mbarrier indices.  Barriers whose producer may run two chunks a
   BAR_INV,   // gate group -> epilogue group: 1/denominator published
   BAR_EGDONE,  // epilogue group -> gate group: 1/denominator consumed
   BAR_QNREAD,  // gate group -> epilogue group: q.n of a chunk is in registers (its columns may take the bf16 copy again)
-  BAR_TINIT,   // state group -> epilogue group: the initial state is in tensor memory
   BAR_COUNT
 };
 
@@ -150,31 +144,13 @@ struct CwLayout {
   static constexpr bool TAIL_SHARED = (T_CB + DHQK / 2 > T_SX);
 };
 
-struct CwMaps {
-  CUtensorMap q, k, v;
-  // position (1..3) of the token / head / batch coordinate in each map; the outer dimensions are ordered by
-  // ascending stride, which differs between a contiguous (B,NH,S,D) tensor and a transposed (B,S,NH,D) view
-  int pos[3][3];  // [q|k|v][token|head|batch]
-};
-
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float fast_log_sigmoid(float x) { return fminf(x, 0.f) - __logf(1.f + __expf(-fabsf(x))); }
 __device__ __forceinline__ void gate_group_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ void epilogue_group_sync() { asm volatile("bar.sync 2, 128;" ::: "memory"); }
-
-// 16 bytes of bf16 times a bf16x2 splat, rounded once per product
-__device__ __forceinline__ uint4 scale_bf16x8(uint4 raw, __nv_bfloat162 s) {
-  __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&raw);
-  p[0] = __hmul2(p[0], s);
-  p[1] = __hmul2(p[1], s);
-  p[2] = __hmul2(p[2], s);
-  p[3] = __hmul2(p[3], s);
-  return raw;
-}
 
 // byte offset of element (row, col) in an [rows x 64] bf16 box with 128-byte swizzle
 __device__ __forceinline__ uint32_t sw128_off(int row, int col) {
@@ -231,14 +207,67 @@ static __device__ __noinline__ void cw_convert_T(uint32_t tC, uint32_t tCb, int 
   tc_wait_st();
 }
 
+// T <- the state a part starts from, in blocks of 32 columns that three groups share (group index 0, 1, 2; one group alone
+// spent 0.7 us of load latency per block and folded part).  Not inlined, like the conversion: code that runs once must not
+// take registers from the loops.
+template <int DHQK>
+static __device__ __noinline__ void cw_init_state(const float* c0, int DHV, const float4* cl0, long long part_stride, int parts_before, const float* coef,
+                                                  int group, uint32_t tC) {
+#pragma unroll 1
+  for (int cb = group; cb < DHQK / 32; cb += 3) {
+    uint32_t r[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = c0 ? __float_as_uint(__ldcg(c0 + (long long)(cb * 32 + i) * DHV)) : 0u;
+    if (parts_before > 0) {
+      const float cf = coef[CW_MAX_PARTS];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * cf);
+      const float4* cl = cl0 + (cb * 8) * CW_DV;
+#pragma unroll 2
+      for (int j = 0; j < parts_before; ++j) {
+        const float cj = coef[j];
+        float4 x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = __ldcg(cl + j * part_stride + i * CW_DV);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          r[4 * i + 0] = __float_as_uint(fmaf(cj, x[i].x, __uint_as_float(r[4 * i + 0])));
+          r[4 * i + 1] = __float_as_uint(fmaf(cj, x[i].y, __uint_as_float(r[4 * i + 1])));
+          r[4 * i + 2] = __float_as_uint(fmaf(cj, x[i].z, __uint_as_float(r[4 * i + 2])));
+          r[4 * i + 3] = __float_as_uint(fmaf(cj, x[i].w, __uint_as_float(r[4 * i + 3])));
+        }
+      }
+    }
+    tmem_st_x32(tC + cb * 32, r);
+  }
+  tc_wait_st();
+  tc_fence_before();
+  asm volatile("bar.sync 3, 384;" ::: "memory");   // gate, state and epilogue group
+  tc_fence_after();
+}
+
+// Final C = exp(rho) T, in blocks of 32 columns that the state and the gate group share (group index 0, 1)
+template <int DHQK>
+static __device__ __noinline__ void cw_store_state(float* c_out, int DHV, int group, uint32_t tC, float back) {
+#pragma unroll 1
+  for (int cb = group; cb < DHQK / 32; cb += 2) {
+    uint32_t r[32];
+    tmem_ld_x32(tC + cb * 32, r);
+    tc_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) c_out[(long long)(cb * 32 + i) * DHV] = __uint_as_float(r[i]) * back;
+  }
+}
+
 template <int DHQK>
 __global__ void __launch_bounds__(CW_THREADS, 1)
-mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_params p) {
+mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_params p, const CwSplit split) {
   using LY = CwLayout<DHQK>;
   constexpr int NKB = LY::NKB;
   constexpr int NB = NKB;  // 64-feature blocks of the normaliser state n
   static_assert(NB == 1 || NB == 2 || NB == 4, "feature blocks");
   extern __shared__ unsigned char cw_smem_raw[];
+  __shared__ float s_coef[CW_MAX_PARTS + 2];
   // 128-byte-swizzled tiles need 1024-byte aligned bases
   // (pointer arithmetic on the __shared__ array, not an integer round trip, so that every access below is
   // compiled as a shared-memory instruction rather than a generic one)
@@ -258,24 +287,40 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
   // plain `threadIdx.x >> 5` every UMMA becomes a ~35-instruction sequence and the issuing warp, not the tensor
   // pipe, sets the pace.
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int slice = blockIdx.x, head = blockIdx.y, doc = blockIdx.z;
+  const int slice = blockIdx.x, head = blockIdx.y;
   const int col0 = slice * CW_DV;
   const int DHV = p.DHV;
 
-  // ---- document -> (batch row, first token, length)
+  // Behind mlstm_part_state_kernel a document's first part does not wait for it, so all it reads through this path was
+  // complete when that kernel passed its own wait, and is read from L2 (__ldcg, TMA).
+  if (!split.after_states) grid_dependency_wait();
+
+  // ---- this block's part of a document
+  CwItem it;
+  if (split.counts) {
+    if ((int)blockIdx.z >= __ldcg(split.counts)) { grid_dependency_wait(); return; }
+    it = cw_load_item(split.items + blockIdx.z);
+  } else {
+    it.parts = split.parts;
+    it.doc = (int)blockIdx.z / it.parts;
+    it.part = (int)blockIdx.z - it.doc * it.parts;
+    it.first_chunk = it.part * split.part_chunks;
+    it.chunks = split.part_chunks;
+    it.slot0 = it.doc * (it.parts - 1);
+  }
+  const int doc = it.doc;
+  const bool last_part = it.part + 1 == it.parts;
   long long tok0, len;
   int b;
-  if (p.cu_seqlens) {
-    const long long s = p.cu_seqlens[doc], e = p.cu_seqlens[doc + 1];
-    b = (int)(s / p.S);
-    tok0 = s - (long long)b * p.S;
-    len = e - s;
-  } else {
-    b = doc; tok0 = 0; len = p.S;
-  }
+  cw_document(p, doc, b, tok0, len);
+  tok0 += (long long)it.first_chunk * CW_L;
+  len = last_part ? len - (long long)it.first_chunk * CW_L : (long long)it.chunks * CW_L;
   const long long sidx = (long long)doc * p.NH + head;
+  // From the zero state chunk 0 has no inter-chunk product: nothing is converted for it, T and H^T are zeroed and added to.
+  const bool zero_start = it.part == 0 && !p.c0;
 
   if (len <= 0) {  // empty document: the state passes through unchanged
+    grid_dependency_wait();
     if (tid < CW_DV) {
       const float* c0 = p.c0 ? p.c0 + (sidx * DHQK) * DHV + col0 + tid : nullptr;
       float* c_out = p.c_out + (sidx * DHQK) * DHV + col0 + tid;
@@ -302,9 +347,6 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       mbar_init(bar0 + 8u * i, cnt);
     }
     fence_barrier_init();
-    tma_prefetch_desc(&maps.q);
-    tma_prefetch_desc(&maps.k);
-    tma_prefetch_desc(&maps.v);
   }
   // OFF_P .. OFF_HST: the P tile (its blocks right of the diagonal stay zero for ever) and the w operand of nu
   for (int i = tid; i < (LY::OFF_HST - LY::OFF_P) / 16; i += CW_THREADS)
@@ -320,10 +362,34 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
     tmem_alloc(smem_u32(s_tmem), CW_TMEM_COLS);
     tmem_relinquish();
   }
+  // ---- the state this part starts from: the initial state and the parts in front of it, each decayed to here.  With G_j
+  // the sum of log f of the parts behind j: m = max_j(m_j + G_j), C = sum_j exp(m_j + G_j - m) C_loc,j (lane j = part j; the
+  // initial state joins as m0 + the sum over all parts).  s_coef holds the factors, the initial state's, and m.
+  if (it.part > 0) {
+    grid_dependency_wait();   // (the first part of a document needs nothing of the launch in front)
+    if (warp == 0) {
+      const float2 v = lane < it.part ? split.gm[(long long)(it.slot0 + lane) * p.NH + head] : make_float2(0.f, -INFINITY);
+      float g = v.x;   // inclusive sum over the lanes from here on
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_down_sync(0xffffffffu, g, o);
+        if (lane + o < 32) g += t;
+      }
+      const float mine = v.y + (g - v.x), first = (p.m0 ? p.m0[sidx] : 0.f) + __shfl_sync(0xffffffffu, g, 0);
+      float m = mine;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      m = fmaxf(m, first);
+      s_coef[lane] = expf(mine - m);
+      if (lane == 0) { s_coef[CW_MAX_PARTS] = expf(first - m); s_coef[CW_MAX_PARTS + 1] = m; }
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
+  // (No early launch of the kernel behind: its blocks waiting on the idle SMs cost this one 12 % at 128 blocks, 250 -> 285 us.)
+  const float m_start = it.part > 0 ? s_coef[CW_MAX_PARTS + 1] : (p.m0 ? __ldcg(p.m0 + sidx) : 0.f);
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;  // tcgen05.ld/st: a warp reaches lanes 32*(warp%4)..+31
   const uint32_t tC = tmem + LY::T_C + lane_base, tCb = tmem + LY::T_CB + lane_base;
   const uint32_t tH = tmem + LY::T_H + lane_base, tS = tmem + LY::T_S + lane_base;
@@ -334,20 +400,31 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
   // group, whose P pass gates phase B, converts nothing).
   constexpr int CB_SPLIT = DHQK / 64 >= 2 ? DHQK / 64 - 1 : 1;
 
+  auto init_state = [&](int group) {
+    const int dv = (warp & 3) * 32 + lane;
+    cw_init_state<DHQK>(p.c0 ? p.c0 + (sidx * DHQK) * DHV + col0 + dv : nullptr, DHV,
+                        reinterpret_cast<const float4*>(split.c_loc) + cw_c_loc_offset<DHQK>(p, it.slot0, head, slice) + dv,
+                        (long long)p.NH * DHQK * DHV / 4, it.part, s_coef, group, tC);
+  };
+  auto store_C = [&](int group, float back) {
+    tc_fence_after();
+    cw_store_state<DHQK>(p.c_out + (sidx * DHQK) * DHV + col0 + (warp & 3) * 32 + lane, DHV, group, tC, back);
+  };
+
   if (warp == W_SCAN) {
     // =========================================================================================== scan warp
     // Carries the gate recurrence one or two chunks ahead of everybody else: lane L owns tokens 2L and 2L+1.
     const float* ig = p.igate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
     const float* fg = p.fgate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
-    float m_prev = p.m0 ? p.m0[sidx] : 0.f;
+    float m_prev = m_start;
     float rho = 0.f;
     // Gate loads are issued one chunk ahead, unconditionally and from clamped addresses; the tail mask is applied
     // when the values are used.
     float gi0, gi1, gf0, gf1;
     {
       const long long t0 = 2 * lane, ta = t0 < len ? t0 : len - 1, tb = t0 + 1 < len ? t0 + 1 : len - 1;
-      gi0 = ig[ta * p.g_st]; gf0 = fg[ta * p.g_st];
-      gi1 = ig[tb * p.g_st]; gf1 = fg[tb * p.g_st];
+      gi0 = __ldcg(ig + ta * p.g_st); gf0 = __ldcg(fg + ta * p.g_st);
+      gi1 = __ldcg(ig + tb * p.g_st); gf1 = __ldcg(fg + tb * p.g_st);
     }
 #pragma unroll 1
     for (int chunk = 0; chunk < nchunks; ++chunk) {
@@ -360,8 +437,8 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       {
         const long long tn = (long long)(chunk + 1) * CW_L + 2 * lane;
         const long long ta = tn < len ? tn : len - 1, tb = tn + 1 < len ? tn + 1 : len - 1;
-        gi0 = ig[ta * p.g_st]; gf0 = fg[ta * p.g_st];
-        gi1 = ig[tb * p.g_st]; gf1 = fg[tb * p.g_st];
+        gi0 = __ldcg(ig + ta * p.g_st); gf0 = __ldcg(fg + ta * p.g_st);
+        gi1 = __ldcg(ig + tb * p.g_st); gf1 = __ldcg(fg + tb * p.g_st);
       }
       const int t0 = 2 * lane, t1 = t0 + 1;
       const float lf0 = (t0 < len_c) ? fast_log_sigmoid(cf0) : 0.f;
@@ -436,13 +513,20 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       fence_proxy_async_smem();
       mbar_arrive(bar0 + 8u * (BAR_GFULL0 + buf));
     }
-    if (ok && slice == 0 && lane == 0) p.m_out[sidx] = m_prev;
+    if (ok && last_part && slice == 0 && lane == 0) p.m_out[sidx] = m_prev;
   } else if (warp < W_STATE_GROUP) {
     // =========================================================================================== gate group
     // Iteration j: q.n(j) and S(j) out of tensor memory, P(j); then, with nu(j) (issued one chunk ahead, behind S(j)):
     // n(j) and its hi/lo rows for the S product of chunk j+1, and the denominators of chunk j.
     const int g = tid;  // 0..127
-    for (int d = g; d < DHQK; d += 128) s_n[d] = p.n0 ? p.n0[sidx * DHQK + d] : 0.f;
+    for (int d = g; d < DHQK; d += 128) {
+      float nv = p.n0 ? __ldcg(p.n0 + sidx * DHQK + d) : 0.f;
+      if (it.part > 0) {
+        nv *= s_coef[CW_MAX_PARTS];
+        for (int j = 0; j < it.part; ++j) nv = fmaf(s_coef[j], split.n_loc[((long long)(it.slot0 + j) * p.NH + head) * DHQK + d], nv);
+      }
+      s_n[d] = nv;
+    }
     // hi/lo bf16 split of n[d] into rows 0/1 in front of the k box of feature block d/64 in stage `nbuf`, where the S
     // product of that stage's chunk picks them up as eight more B rows
     auto publish_n = [&](int nbuf, int d, float nv) {
@@ -456,6 +540,7 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
     fence_proxy_async_smem();
     if (mbar_wait(bar0 + 8u * BAR_GFULL0, 0u)) mbar_arrive(bar0 + 8u * BAR_C2);  // n rows and gate data of chunk 0
     else ok = false;
+    init_state(0);
     // S fragment of this thread: rows j0 and j0 + 8, column pair cq of every 8-column group (q.n is the group in front
     // of S: the threads with cq == 0 hold its hi and lo part); the nu products sit on lanes 16..31 of the plain
     // (lane = thread) view
@@ -573,8 +658,12 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       if ((lane & 2) == 0) s_inv[jd] = __fdividef(1.f, fmaxf(fabsf(fmaf(dot, qn_scale, (lane & 1) ? rs1 : rs0)), lower) + eps_j);
       mbar_arrive(bar0 + 8u * BAR_INV);
     }
+    if (ok && last_part) {
+      if (mbar_wait(bar0 + 8u * BAR_HC, (uint32_t)(nchunks - 1) & 1u)) store_C(1, back_last);
+      else ok = false;
+    }
     // ---- final n (back in the true frame)
-    if (ok && slice == 0 && lane >= 16) {  // the first slice of the head writes n
+    if (ok && last_part && slice == 0 && lane >= 16) {  // the first slice of the head writes n
 #pragma unroll
       for (int gq = 0; gq < NB; ++gq) {
         const int d = 64 * gq + 16 * warp + (lane - 16);
@@ -584,19 +673,7 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
   } else if (warp < W_EPI_GROUP) {
     // =========================================================================================== state group
     const int t = tid - 128;
-    const int dv = (warp & 3) * 32 + lane;  // tensor-memory lane = value column within the slice
-    const float* c0 = p.c0 ? p.c0 + (sidx * DHQK) * DHV + col0 + dv : nullptr;
-    float* c_out = p.c_out + (sidx * DHQK) * DHV + col0 + dv;
-#pragma unroll 1
-    for (int cb = 0; cb < DHQK / 32; ++cb) {
-      uint32_t r[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) r[i] = c0 ? __float_as_uint(c0[(long long)(cb * 32 + i) * DHV]) : 0u;
-      tmem_st_x32(tC + cb * 32, r);
-    }
-    tc_wait_st();
-    tc_fence_before();
-    mbar_arrive(bar0 + 8u * BAR_TINIT);  // the epilogue group converts its block of the initial state
+    init_state(1);
     float rho_last = 0.f;
 #pragma unroll 1
     for (int chunk = 0; chunk < nchunks; ++chunk) {
@@ -612,7 +689,7 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       if (chunk >= 1) CW_WAIT(BAR_HC, par ^ 1u);  // T holds chunk-1; its UMMAs no longer read Tb or the scaled-v tile
       tc_fence_after();
       // ---- T -> bf16 copy, this group's blocks
-      convert_T(0, CB_SPLIT, cb_scale, mult);
+      if (chunk > 0 || !zero_start) convert_T(0, CB_SPLIT, cb_scale, mult);
       tc_fence_before();
       mbar_arrive(bar0 + 8u * BAR_A);
       if (!exact) mbar_arrive(bar0 + 8u * BAR_A);  // common frame: q is used as loaded
@@ -663,21 +740,9 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       mbar_arrive(bar0 + 8u * (BAR_EMPTY0 + st));
       mbar_arrive(bar0 + 8u * (BAR_GEMPTY0 + buf));
     }
-    // ---- final C = exp(rho) T
-    if (ok) {
-      do {
-        CW_WAIT(BAR_HC, (uint32_t)(nchunks - 1) & 1u);
-        tc_fence_after();
-        const float back = expf(rho_last);
-#pragma unroll 1
-        for (int cb = 0; cb < DHQK / 32; ++cb) {
-          uint32_t r[32];
-          tmem_ld_x32(tC + cb * 32, r);
-          tc_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) c_out[(long long)(cb * 32 + i) * DHV] = __uint_as_float(r[i]) * back;
-        }
-      } while (false);
+    if (ok && last_part) {
+      if (mbar_wait(bar0 + 8u * BAR_HC, (uint32_t)(nchunks - 1) & 1u)) store_C(0, expf(rho_last));
+      else ok = false;
     }
   } else if (warp < W_UMMA) {
     // =========================================================================================== epilogue group
@@ -744,13 +809,15 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       mbar_arrive(bar0 + 8u * BAR_A);  // this group's share of the bf16 copy for chunk `next`
       return true;
     };
-    if constexpr (EG_CONVERTS) {
-      if (!mbar_wait(bar0 + 8u * BAR_TINIT, 0u)) ok = false;
-      tc_fence_after();
+    if (zero_start) {
+      const uint32_t z[32] = {};
+      tmem_st_x32(tH, z);
+      tmem_st_x32(tH + 32, z);
     }
-    if (ok && !convert_block(0)) ok = false;
+    init_state(2);
     mbar_arrive(bar0 + 8u * BAR_A);  // the accumulator is free for chunk 0
-    if (ok && !finish_block(0)) ok = false;
+    if (zero_start) mbar_arrive(bar0 + 8u * BAR_A);
+    else if (!convert_block(0) || !finish_block(0)) ok = false;
     // Denominators of chunk c: ready long before H^T(c) is (they depend on the previous phase of UMMAs only).
     auto denominators_ready = [&](int c) -> bool {
       if (!mbar_wait(bar0 + 8u * BAR_INV, (uint32_t)c & 1u)) return false;
@@ -828,6 +895,9 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0), sbase_u = __shfl_sync(0xffffffffu, sbase, 0) & 0x3FFFFu;
     const uint32_t bar_u = __shfl_sync(0xffffffffu, bar0, 0);
     const int nchunks_u = __shfl_sync(0xffffffffu, nchunks, 0);
+    // k boxes of the inter-chunk product: none in chunk 0 of a zero start.  (A uniform loop bound, not a branch around the
+    // issue loop: see above.)
+    int nkb_u = __shfl_sync(0xffffffffu, zero_start ? 0 : NKB, 0);
     const uint32_t t_odd = tmem_u + LY::T_S + (16u << 16);  // odd 16-lane halves of the S columns
     // lower descriptor words (start address >> 4 | leading offset); K-major tiles use leading offset 16 B, MN-major
     // tiles the distance between their 64-wide boxes (8 KiB; 9 KiB for k, whose boxes have the n rows in front)
@@ -869,7 +939,7 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       okm &= MMA_WAIT_U(BAR_A, par);
       tc_fence_after();
 #pragma unroll 1
-      for (int kb = 0; kb < NKB; ++kb)
+      for (int kb = 0; kb < nkb_u; ++kb)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           umma_ts_lo(tmem_u + LY::T_H, tmem_u + LY::T_CB + (4 * kb + kk) * 8,
@@ -886,6 +956,7 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
                      (LBO_MN_K + ((s_k >> 4) + ((kk * 2048) >> 4))), IDESC_C, 1);
         }
       }
+      nkb_u = NKB;
       umma_commit_elect(bar_u + 8u * BAR_HC);
       umma_commit_elect(bar_u + 8u * (BAR_EMPTY0 + (chunk & 1)));  // the stage of this chunk is consumed
       // ---- phase C for the next chunk (one branch around the whole phase, none inside the issue loops)
@@ -904,24 +975,23 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
         const uint32_t dst = sbase + LY::OFF_STAGE + st * LY::STAGE_BYTES;
         const int tk = (int)(tok0 + (long long)chunk * CW_L);
         mbar_expect_tx(bar, LY::TX_BYTES);
-        int cq[4], ck[4], cv[4];
-        cq[maps.pos[0][0]] = tk; cq[maps.pos[0][1]] = head; cq[maps.pos[0][2]] = b;
-        ck[maps.pos[1][0]] = tk; ck[maps.pos[1][1]] = head; ck[maps.pos[1][2]] = b;
-        cv[maps.pos[2][0]] = tk; cv[maps.pos[2][1]] = head; cv[maps.pos[2][2]] = b;
+        auto at = [&](int t, int i) { return cw_coord(maps, t, i, tk, head, b); };
 #pragma unroll
         for (int kb = 0; kb < NKB; ++kb) {
-          tma_load_4d(dst + kb * CW_BOX_BYTES, &maps.q, bar, kb * 64, cq[1], cq[2], cq[3]);
-          tma_load_4d(dst + LY::OFF_K + kb * LY::K_STRIDE + 1024, &maps.k, bar, kb * 64, ck[1], ck[2], ck[3]);
+          tma_load_4d(dst + kb * CW_BOX_BYTES, &maps.q, bar, kb * 64, at(0, 1), at(0, 2), at(0, 3));
+          tma_load_4d(dst + LY::OFF_K + kb * LY::K_STRIDE + 1024, &maps.k, bar, kb * 64, at(1, 1), at(1, 2), at(1, 3));
         }
 #pragma unroll
         for (int vb = 0; vb < 2; ++vb)
-          tma_load_4d(dst + LY::OFF_V + vb * CW_BOX_BYTES, &maps.v, bar, col0 + vb * 64, cv[1], cv[2], cv[3]);
+          tma_load_4d(dst + LY::OFF_V + vb * CW_BOX_BYTES, &maps.v, bar, col0 + vb * 64, at(2, 1), at(2, 2), at(2, 3));
       }
     }
     __syncwarp();
   }
 
   if (!ok && p.status) atomicExch(p.status, 1);
+  // (a first part has not waited yet: the end of this kernel means the end of the one in front, too)
+  if (split.after_states && it.part == 0) grid_dependency_wait();
   tc_fence_before();
   __syncthreads();
   if (warp == W_UMMA) tmem_dealloc(tmem, CW_TMEM_COLS);
@@ -993,20 +1063,22 @@ static int make_map(CUtensorMap* m, int pos[3], const void* base, int D, int S, 
 int validate_seq_common(const xl_mlstm_seq_params* p);
 
 template <int DHQK>
-static int launch_chunkwise(const CwMaps& maps, const xl_mlstm_seq_params* p, cudaStream_t st) {
+static int launch_chunkwise(const CwMaps& maps, const xl_mlstm_seq_params* p, const CwSplit& split, unsigned grid_z, cudaStream_t st) {
   using LY = CwLayout<DHQK>;
   static_assert(LY::DYN_SMEM <= 227 * 1024, "shared memory budget");
-  const int nd = p->cu_seqlens ? p->num_docs : p->B;
-  dim3 grid(p->DHV / CW_DV, p->NH, nd);
   auto kern = mlstm_chunkwise_kernel<DHQK>;
   XL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::DYN_SMEM));
-  kern<<<grid, CW_THREADS, LY::DYN_SMEM, st>>>(maps, *p);
+  XL_CUDA_TRY(launch_dependent(kern, dim3(p->DHV / CW_DV, p->NH, grid_z), dim3(CW_THREADS), LY::DYN_SMEM, st, maps, *p, split));
   return check_launch("xl_mlstm_chunkwise");
 }
 
 }  // namespace xl
 
-extern "C" int xl_mlstm_chunkwise(const xl_mlstm_seq_params* p, void* cuda_stream) {
+extern "C" int64_t xl_mlstm_chunkwise_scratch_bytes(const xl_mlstm_seq_params* p) { return p ? xl::cw_split_scratch_bytes(p) : 0; }
+
+extern "C" int xl_mlstm_chunkwise(const xl_mlstm_seq_params* p, void* cuda_stream) { return xl_mlstm_chunkwise_parts(p, nullptr, 0, cuda_stream); }
+
+extern "C" int xl_mlstm_chunkwise_parts(const xl_mlstm_seq_params* p, void* scratch, int64_t scratch_bytes, void* cuda_stream) {
   using namespace xl;
   int rc = validate_seq_common(p);
   if (rc != XL_OK) return rc;
@@ -1023,9 +1095,20 @@ extern "C" int xl_mlstm_chunkwise(const xl_mlstm_seq_params* p, void* cuda_strea
   if ((rc = make_map(&maps.k, maps.pos[1], p->k, p->DHQK, p->S, p->NH, p->B, p->k_sb, p->k_sh, p->k_st)) != XL_OK) return rc;
   if ((rc = make_map(&maps.v, maps.pos[2], p->v, p->DHV, p->S, p->NH, p->B, p->v_sb, p->v_sh, p->v_st)) != XL_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
+  CwSplit split = {};
+  split.parts = 1;
+  split.part_chunks = (p->S + CW_L - 1) / CW_L;
+  unsigned grid_z = p->cu_seqlens ? p->num_docs : p->B;
+  if (scratch) {
+    if (scratch_bytes < cw_split_scratch_bytes(p)) return XL_ERR_TOO_LARGE;
+    if (!aligned16(scratch)) return XL_ERR_BAD_ALIGNMENT;
+    if (cw_split_scratch_bytes(p) > 0) {
+      if ((rc = cw_prepare_split(maps, p, scratch, scratch_bytes, &split, &grid_z, st)) != XL_OK) return rc;
+    }
+  }
   switch (p->DHQK) {
-    case 64: return launch_chunkwise<64>(maps, p, st);
-    case 128: return launch_chunkwise<128>(maps, p, st);
-    default: return launch_chunkwise<256>(maps, p, st);
+    case 64: return launch_chunkwise<64>(maps, p, split, grid_z, st);
+    case 128: return launch_chunkwise<128>(maps, p, split, grid_z, st);
+    default: return launch_chunkwise<256>(maps, p, split, grid_z, st);
   }
 }

@@ -42,6 +42,32 @@ def test_matches_oracle(B, S, NH, DH, with_state):
         assert rel_l2(last[idx], last_ref[idx]) < TOL, (idx, rel_l2(last[idx], last_ref[idx]))
 
 
+@pytest.mark.parametrize("B,S,NH,DH,with_state", [
+    (7, 9, 4, 256, True), (8, 17, 2, 128, True), (9, 3, 1, 256, False), (32, 5, 4, 256, True),   # clusters of eight batch rows
+    (72, 6, 4, 256, True), (200, 4, 4, 128, False), (523, 3, 4, 64, True)])                       # too many of them: sixteen rows
+def test_matches_oracle_on_both_sides_of_the_row_split(B, S, NH, DH, with_state):
+    wx, R, bias, st = _case(B * 7 + S, B, S, NH, DH, with_state)
+    out_ref, last_ref = O.slstm_forward(wx, R, bias, st)
+    out, last = _run(wx, R, bias, st)
+    assert rel_l2(out, out_ref) < TOL and all(rel_l2(last[i], last_ref[i]) < TOL for i in range(4))
+
+
+def test_document_boundaries_in_several_row_groups():
+    """Boundaries in both rows of a thread's pair, in neighbouring steps and in the second group of eight rows."""
+    B, S, NH, DH = 11, 24, 2, 256
+    wx, R, bias, _ = _case(15, B, S, NH, DH)
+    starts = {0: [7], 1: [7, 8], 2: [1], 3: [23], 9: [11, 12, 13], 10: [5]}
+    cu, reset = [0], torch.zeros(B, S, dtype=torch.bool)
+    for b in range(B):
+        for t in starts.get(b, []):
+            cu.append(b * S + t)
+            reset[b, t] = True
+        cu.append((b + 1) * S)
+    out_ref, last_ref = O.slstm_forward(wx, R, bias, reset=reset)
+    out, last = _run(wx, R, bias, cu=cu)
+    assert rel_l2(out, out_ref) < TOL and rel_l2(last, last_ref) < TOL
+
+
 def test_matches_reference_vanilla_fixture():
     g = load_golden("slstm_bf16")  # produced by the reference's vanilla cell in bf16
     out, last = _run(g["wx"].bfloat16(), g["R"].bfloat16(), g["bias"])
@@ -107,6 +133,7 @@ def _grads_kernel(wx, R, bias, st, gh, gl):
 @pytest.mark.parametrize("B,S,NH,DH,with_state,state_loss", [
     (2, 1, 1, 64, True, False), (2, 2, 2, 64, False, False), (1, 9, 1, 128, True, True),
     (3, 5, 1, 64, False, False), (3, 37, 2, 64, True, False), (16, 64, 4, 256, True, False),
+    (9, 11, 2, 256, True, True), (8, 3, 1, 128, False, True), (72, 4, 4, 256, True, True), (300, 3, 4, 64, False, False),
     (20, 33, 1, 128, True, True), (16, 200, 2, 256, False, True)])
 def test_backward_matches_autograd_of_the_oracle(B, S, NH, DH, with_state, state_loss):
     """dWx, dR, dbias and the gradient of the initial state from the backward kernel against autograd over the CPU

@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(SLB_THREADS, 1) slstm_backward_kernel(const xl
   const bool ok_r = gb < B;
   const size_t st_off = (size_t)(ok_r ? gb : 0) * H + (size_t)head * DH + unit_h;   // this thread's pair in a (4,B,H) state
 
+  grid_dependency_wait();
   // ---- the CTA's slice of R as B fragments of dh[b,k] = sum_{(g,u)} dg[b,(g,u)] R[k,g,u]:  n = k, contraction index
   // kk = 32 g + (u - 32 rank); a fragment register holds two adjacent u of one (k, g)
   uint32_t bfrag[NTW][KS][2];
@@ -301,27 +302,261 @@ __global__ void __launch_bounds__(SLB_THREADS, 1) slstm_backward_kernel(const xl
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Clusters of EIGHT batch rows (the counterpart of slstm_forward_rows8_kernel): the rows are the N = 8 side of the products
+// and R the A operand, dh_{t-1}^T [DH x 8] = R [DH x 128] dg^T [128 x 8], so a step costs 16 products per warp instead of 32,
+// half the exchange and one (row, unit) pair of gate arithmetic per thread, on twice the SMs: 2.79 -> SL8_BWD_MS ms at B = 16,
+// S = 2048, 4 x 256.
+//
+// Eight warps: warps 2w and 2w+1 share the pairs of forward warp w -- thread (w, lane) of the forward owns unit 8w + lane/4 and
+// rows 2 (lane%4), + 1; the first warp takes the even row, the second the odd one.  The dg tile is [gate x unit][row]: a B
+// fragment is one transposing ldmatrix without bank conflicts, and the same fragment is dWx_t in (row, two units) words for the
+// store.  Warp w forms the 32 columns of dh_{t-1} that CTA w of the cluster owns (DH = 256), and a lane's accumulators are
+// four units x two rows: packed over the rows they ARE the lane's 16-byte granule, one asynchronous store per thread and step
+// with nothing regrouped.  The receiver reads word `unit/8` of granule (unit%8, row/2) from every source; granules rotate
+// their words by lane/8, which puts the four lanes that would share a bank on four.
+constexpr int SLB8_BLOCK = SL8_ROWS * SL_UNITS * 2;        // bytes of one (source, destination) block of partial sums
+
+template <int DH>
+struct Slb8Layout {
+  static constexpr int NCTA = DH / SL_UNITS;
+  static constexpr int DG = 4 * SL_UNITS * SL8_ROWS * 2;               // dg tile, bytes
+  static constexpr int OFF_RB = 2 * DG;                                // received: [2][source CTA][SLB8_BLOCK]
+  static constexpr int OFF_REC = OFF_RB + 2 * NCTA * SLB8_BLOCK;       // [SL_RING][SL8_REC_STEP]
+  static constexpr int OFF_BAR = OFF_REC + SL_RING * SL8_REC_STEP;     // 2 mbarriers: partials landed
+  static constexpr int TOTAL = OFF_BAR + 16;
+};
+
+template <int DH>
+__global__ void __launch_bounds__(SLB_THREADS, 1) slstm_backward_rows8_kernel(const xl_slstm_bwd_params p) {
+  using LY = Slb8Layout<DH>;
+  constexpr int NCTA = LY::NCTA;
+  constexpr int MT = DH / 16;                               // 16-column tiles of dh_{t-1}, two per destination CTA
+  constexpr int KS = 4 * SL_UNITS / 16;                     // k-steps over the CTA's 128 gate gradients
+  constexpr uint32_t RB_BYTES = NCTA * SLB8_BLOCK;          // what one step delivers to a CTA
+  static_assert(SLB_THREADS / 32 >= NCTA, "one warp per destination");
+  extern __shared__ __align__(16) unsigned char slb_smem[];
+  unsigned char* s_dg = slb_smem;
+  unsigned char* s_rb = slb_smem + LY::OFF_RB;
+  unsigned char* s_rec = slb_smem + LY::OFF_REC;
+  const uint32_t s_bar = smem_u32(slb_smem + LY::OFF_BAR);
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t rank = cluster_ctarank();
+  const int head = blockIdx.y, bgroup = blockIdx.z;
+  const int B = p.B, S = p.S, NH = p.NH, H = NH * DH;
+  const int fwarp = warp >> 1, half = warp & 1;             // the forward thread whose record this thread shares, and which row of it
+  const int ftid = fwarp * 32 + lane;
+  const int unit_l = fwarp * 8 + (lane >> 2), row = 2 * (lane & 3) + half;
+  const int unit_h = (int)rank * SL_UNITS + unit_l;
+  const int gb = bgroup * SL8_ROWS + row;
+  const bool ok_r = gb < B;
+  const size_t st_off = (size_t)(ok_r ? gb : 0) * H + (size_t)head * DH + unit_h;
+
+  if (tid == 0) {
+    mbar_init(s_bar, 1);      // one arrival per phase: the local expect_tx
+    mbar_init(s_bar + 8, 1);
+    fence_barrier_init();
+  }
+  grid_dependency_wait();
+
+  // ---- cache ring: the records of one step and CTA are 6 KB of contiguous global memory, fetched SL_RING - 1 steps ahead
+  const unsigned char* cache = reinterpret_cast<const unsigned char*>(p.cache) + (((size_t)bgroup * NH + head) * NCTA + rank) * (size_t)S * SL8_REC_STEP;
+  const uint32_t s_rec_u32 = smem_u32(s_rec);
+  constexpr int GRAN = SL8_REC_STEP / 16;                   // 384: one granule per thread, a second one for the first half
+  auto issue = [&](int t) {
+    if (t >= 0) {
+      const unsigned char* src = cache + (size_t)t * SL8_REC_STEP + tid * 16;
+      const uint32_t dst = s_rec_u32 + (uint32_t)(t % SL_RING) * SL8_REC_STEP + tid * 16;
+      cp_async16(dst, src);
+      if (tid < GRAN - SLB_THREADS) cp_async16(dst + SLB_THREADS * 16, src + SLB_THREADS * 16);
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int j = 0; j < SL_RING - 1; ++j) issue(S - 1 - j);
+
+  // ---- the CTA's slice of R as A fragments: rows k = 16 mt + lane/4 (+ 8), contraction index 32 g + (u - 32 rank)
+  uint32_t afrag[2][KS][4];
+  {
+    const __nv_bfloat16* R = reinterpret_cast<const __nv_bfloat16*>(p.R) + (size_t)head * DH * 4 * DH;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int k_in = (2 * warp + j) * 16 + (lane >> 2);
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) {
+        const __nv_bfloat16* base = R + ((size_t)(2 * warp + j < MT ? k_in : 0) * 4 + (ks >> 1)) * DH + rank * SL_UNITS + (ks & 1) * 16 + (lane & 3) * 2;
+        afrag[j][ks][0] = *reinterpret_cast<const uint32_t*>(base);
+        afrag[j][ks][1] = *reinterpret_cast<const uint32_t*>(base + (size_t)8 * 4 * DH);
+        afrag[j][ks][2] = *reinterpret_cast<const uint32_t*>(base + 8);
+        afrag[j][ks][3] = *reinterpret_cast<const uint32_t*>(base + (size_t)8 * 4 * DH + 8);
+      }
+    }
+  }
+
+  float dc_, dn_, dhrec;
+  {
+    const bool have = p.dstate_out != nullptr && ok_r;
+    dhrec = have ? p.dstate_out[0 * (size_t)B * H + st_off] : 0.f;
+    dc_ = have ? p.dstate_out[1 * (size_t)B * H + st_off] : 0.f;
+    dn_ = have ? p.dstate_out[2 * (size_t)B * H + st_off] : 0.f;
+  }
+  // the gradient from above, (B, NH, S, DH), loaded one step ahead
+  const __nv_bfloat16* dh = reinterpret_cast<const __nv_bfloat16*>(p.dh) + ((size_t)(ok_r ? gb : B - 1) * NH + head) * (size_t)S * DH + unit_h;
+  auto load_dh = [&](int t) {
+    unsigned short v;
+    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(dh + (size_t)t * DH));
+    return v;
+  };
+  cp_async_wait<SL_RING - 4>();   // this thread's granules of the last three steps' records; everybody's behind the barrier
+  cluster_barrier();  // every CTA's barriers exist before anything crosses over; also a CTA-wide barrier
+
+  const uint32_t s_dg_u32 = smem_u32(s_dg), s_rb_u32 = smem_u32(s_rb);
+  // dWx: warps 0-3 store gate `warp`, lane (row lane/4; units 8 j + 2 (lane%4), + 1)
+  const int wrow = bgroup * SL8_ROWS + (lane >> 2);
+  uint32_t* dwx = reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.dwx) +
+                                              ((size_t)(wrow < B ? wrow : 0) * S * 4 + (warp & 3)) * H + (size_t)head * DH + rank * SL_UNITS + 2 * (lane & 3));
+  const bool stores_dwx = warp < 4 && wrow < B;
+  const uint32_t push_off = rank * SLB8_BLOCK + (uint32_t)lane * 16;
+  const int rot = lane >> 3;
+  const uint32_t recv_off = (uint32_t)lane * 16 + (uint32_t)((fwarp + rot) & 3) * 4;   // (lane/4, lane%4) = (unit % 8, row / 2)
+
+  // everything of a step that does not depend on the incoming gradient, formed one step ahead (names as above)
+  float pa, pb, pig, pzt, pfg, pff, pcp, pnp, pz2, po2;
+  auto pick = [&](uint32_t w) { return half ? __uint_as_float(w & 0xffff0000u) : __uint_as_float(w << 16); };   // this thread's row of a pair
+  auto precompute = [&](int t) {
+    const unsigned char* rt = s_rec + (t % SL_RING) * SL8_REC_STEP + ftid * SL8_REC_BYTES;
+    const uint4 gw = *reinterpret_cast<const uint4*>(rt);
+    const float yn = pick(*reinterpret_cast<const uint32_t*>(rt + 16));
+    const float nn = *reinterpret_cast<const float*>(rt + 32 + 4 * half), mn = *reinterpret_cast<const float*>(rt + 40 + 4 * half);
+    float cp, np, mp;
+    if (t > 0) {
+      const unsigned char* rp = s_rec + ((t - 1) % SL_RING) * SL8_REC_STEP + ftid * SL8_REC_BYTES;
+      cp = *reinterpret_cast<const float*>(rp + 24 + 4 * half);
+      np = *reinterpret_cast<const float*>(rp + 32 + 4 * half);
+      mp = *reinterpret_cast<const float*>(rp + 40 + 4 * half);
+    } else {
+      const bool have = p.state0 != nullptr && ok_r;
+      cp = have ? p.state0[1 * (size_t)B * H + st_off] : 0.f;
+      np = have ? p.state0[2 * (size_t)B * H + st_off] : 0.f;
+      mp = have ? p.state0[3 * (size_t)B * H + st_off] : 0.f;
+    }
+    const float ig = pick(gw.x), fr = pick(gw.y), zt = pick(gw.z), os = pick(gw.w);
+    const float rn = __fdividef(1.f, nn);
+    const float fg = fminf(1.f, __expf(fast_logsigmoid(fr) + mp - mn));
+    const float fsig = __fdividef(1.f, 1.f + __expf(-fr));
+    pa = os * rn;
+    pb = yn * rn;
+    pig = ig;
+    pzt = zt;
+    pfg = fg;
+    pff = fg * (1.f - fsig);
+    pcp = cp;
+    pnp = np;
+    pz2 = ig * (1.f - zt * zt);
+    po2 = (1.f - os) * yn;
+  };
+  bool ok = true;
+  precompute(S - 1);
+  unsigned short dh_w = load_dh(S - 1);
+
+  for (int it = 0; it < S; ++it) {
+    const int t = S - 1 - it;
+    const int buf = it & 1;
+    {
+      const float dy = (ok_r ? __uint_as_float((uint32_t)dh_w << 16) : 0.f) + dhrec;
+      const float dc = fmaf(dy, pa, dc_);
+      const float dn = fmaf(-dy, pb, dn_);
+      const float dg[4] = {pig * fmaf(pzt, dc, dn), pff * fmaf(dc, pcp, dn * pnp), dc * pz2, po2 * dy};
+      dc_ = pfg * dc;
+      dn_ = pfg * dn;
+      __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(s_dg + buf * LY::DG) + unit_l * SL8_ROWS + row;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) w[g * SL_UNITS * SL8_ROWS] = __float2bfloat16_rn(dg[g]);
+    }
+    // the one CTA-wide barrier of a step (what it orders: see the sixteen-row kernel)
+    if (__syncthreads_or(ok ? 0 : 1)) { ok = false; break; }
+    uint32_t bf[KS][2];
+#pragma unroll
+    for (int kp = 0; kp < KS / 2; ++kp)
+      ldmatrix_x4_trans(s_dg_u32 + buf * LY::DG + kp * 512 + lane * 16, bf[2 * kp][0], bf[2 * kp][1], bf[2 * kp + 1][0], bf[2 * kp + 1][1]);
+    if (tid == 0) mbar_expect_tx(s_bar + 8u * buf, RB_BYTES);   // what this step delivers to this CTA
+    issue(t - (SL_RING - 1));
+    if (t >= 1) dh_w = load_dh(t - 1);
+    if (stores_dwx) {   // dWx_t = dg_t, (B, S, 4, NH, DH)
+      uint32_t* o = dwx + (size_t)t * 2 * H;
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        if (g == warp) { o[0] = bf[2 * g][0]; o[4] = bf[2 * g][1]; o[8] = bf[2 * g + 1][0]; o[12] = bf[2 * g + 1][1]; }
+    }
+    // partial dh_{t-1} of the destination CTA's 32 columns; even and odd k-steps apart (dependent products run at their latency)
+    if (warp < NCTA) {
+      float acc[2][2][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][0][i] = acc[j][1][i] = 0.f;
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          mma_bf16_16816(acc[j][ks & 1], afrag[j][ks][0], afrag[j][ks][1], afrag[j][ks][2], afrag[j][ks][3], bf[ks][0], bf[ks][1]);
+      // word i: units lane/4 + 8 i, rows 2 (lane%4) and + 1; rotated by lane/8
+      uint32_t v[4], r1[4], r2[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[i] = pack_bf16x2(acc[i >> 1][0][2 * (i & 1)] + acc[i >> 1][1][2 * (i & 1)], acc[i >> 1][0][2 * (i & 1) + 1] + acc[i >> 1][1][2 * (i & 1) + 1]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r1[i] = (rot & 1) ? v[(i + 3) & 3] : v[i];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r2[i] = (rot & 2) ? r1[(i + 2) & 3] : r1[i];
+      st_async_v4(map_to_cta(s_rb_u32 + (uint32_t)buf * RB_BYTES + push_off, (uint32_t)warp), r2, map_to_cta(s_bar + 8u * buf, (uint32_t)warp));
+    }
+    // while the partials are in flight: the gradient-independent part of the next step (t - 1)
+    if (t >= 1) precompute(t - 1);   // records t-1, t-2: waited for a step ago, published by this step's barrier
+    cp_async_wait<SL_RING - 4>();    // this thread's granules of records t-2 and t-3, which the next step reads
+    if (!sl_wait(s_bar + 8u * buf, (uint32_t)(it >> 1) & 1u)) ok = false;
+    {
+      const unsigned char* rb = s_rb + buf * RB_BYTES + recv_off;
+      float sum = 0.f;
+#pragma unroll
+      for (int s = 0; s < NCTA; ++s) sum += pick(*reinterpret_cast<const uint32_t*>(rb + s * SLB8_BLOCK));
+      dhrec = sum;
+    }
+  }
+  if (!ok && p.status) atomicExch(p.status, 1);
+  cluster_barrier();  // nobody leaves while a peer may still push into its buffers
+
+  // gradient of the initial state (4, B, H): dh, dc, dn, 0
+  if (ok_r) {
+    p.dstate0[0 * (size_t)B * H + st_off] = dhrec;
+    p.dstate0[1 * (size_t)B * H + st_off] = dc_;
+    p.dstate0[2 * (size_t)B * H + st_off] = dn_;
+    p.dstate0[3 * (size_t)B * H + st_off] = 0.f;
+  }
+}
+
 template <int DH>
 static int launch_slstm_bwd(const xl_slstm_bwd_params* p, cudaStream_t st) {
   constexpr int NCTA = DH / SL_UNITS;
-  const size_t smem = 2 * (size_t)SL_ROWS * SLB_DG_STRIDE * 2 + 2 * (size_t)NCTA * SLB_PBLOCK + (size_t)SL_ROWS * DH * 2 +
-                      (size_t)SL_RING * SLB_REC_STEP + 16 + 8 * SL_RING;
-  XL_CUDA_TRY(cudaFuncSetAttribute(slstm_backward_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(NCTA, p->NH, (p->B + SL_ROWS - 1) / SL_ROWS);
-  cfg.blockDim = dim3(SLB_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = NCTA;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  XL_CUDA_TRY(cudaLaunchKernelEx(&cfg, slstm_backward_kernel<DH>, *p));
+  if (slstm_rows8(p->B, p->NH, DH, true)) {
+    constexpr size_t smem = Slb8Layout<DH>::TOTAL;
+    auto kern = slstm_backward_rows8_kernel<DH>;
+    XL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    XL_CUDA_TRY(slstm_launch(kern, *p, NCTA, (p->B + SL8_ROWS - 1) / SL8_ROWS, SLB_THREADS, smem, st));
+  } else {
+    const size_t smem = 2 * (size_t)SL_ROWS * SLB_DG_STRIDE * 2 + 2 * (size_t)NCTA * SLB_PBLOCK + (size_t)SL_ROWS * DH * 2 +
+                        (size_t)SL_RING * SLB_REC_STEP + 16 + 8 * SL_RING;
+    auto kern = slstm_backward_kernel<DH>;
+    XL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    XL_CUDA_TRY(slstm_launch(kern, *p, NCTA, (p->B + SL_ROWS - 1) / SL_ROWS, SLB_THREADS, smem, st));
+  }
   return check_launch("xl_slstm_backward");
 }
+
+template <int DH>
+static int max_clusters_bwd8() { return slstm_resident_clusters(slstm_backward_rows8_kernel<DH>, DH / SL_UNITS, SLB_THREADS, Slb8Layout<DH>::TOTAL); }
+int slstm_max_clusters_bwd8(int DH) { return DH == 64 ? max_clusters_bwd8<64>() : DH == 128 ? max_clusters_bwd8<128>() : max_clusters_bwd8<256>(); }
 
 }  // namespace xl
 

@@ -16,6 +16,21 @@ constexpr int SL_WX_STEP_BYTES = SL_ROWS * SL_WX_ROW_BYTES;
 // (row, unit) pairs.  Records of a CTA are contiguous: [cluster][CTA][step][thread].
 constexpr int SL_REC_BYTES = 96;
 
+// The eight-row kernels (the batch rows are the N = 8 side of the products, see slstm_fwd.cu): one cluster per (head, 8
+// batch rows).  A thread owns one unit and two adjacent rows; its record is 48 bytes: i', raw f, tanh z, sigmoid o and h' as
+// bf16 pairs over the rows, 4 B pad, then c', n', m' in fp32, two each.
+constexpr int SL8_ROWS = 8;
+constexpr int SL8_REC_BYTES = 48;
+constexpr int SL8_REC_STEP = SL_THREADS * SL8_REC_BYTES;
+
+// Whether a batch of B rows runs on the eight-row kernels: where all their clusters are resident at once.  Eight rows take
+// half the products, half the gate arithmetic and half the exchange of a sixteen-row step, on twice the SMs; with more
+// clusters than fit, a second round would cost more than that saves.  The training forward and the backward share the
+// answer, because it decides the layout of the cache between them.
+bool slstm_rows8(int B, int NH, int DH, bool train);
+int slstm_max_clusters_fwd8(int DH, bool train);
+int slstm_max_clusters_bwd8(int DH);
+
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -52,6 +67,18 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t& r0, uint32_
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
                : "r"(addr));
 }
+// ... each 8 x 8 matrix transposed: thread t receives elements (rows 2 (t%4) and + 1, column t/4)
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+               : "r"(addr));
+}
+// transposes an 8 x 8 matrix of 16-bit elements held as an accumulator-like fragment (row t/4, columns 2 (t%4) and + 1)
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
+}
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                                uint32_t b1) {
   asm volatile(
@@ -60,11 +87,6 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ float fast_tanh(float x) {
-  // 1 - 2/(1+e^{2x}); saturates cleanly for large |x|
-  const float e = __expf(2.f * x);
-  return 1.f - __fdividef(2.f, 1.f + e);
-}
 __device__ __forceinline__ float tanh_approx(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -72,5 +94,45 @@ __device__ __forceinline__ float tanh_approx(float x) {
 }
 __device__ __forceinline__ float fast_logsigmoid(float x) { return fminf(x, 0.f) - __logf(1.f + __expf(-fabsf(x))); }
 
+
+// Number of clusters of DH/32 blocks of `kern` that can be resident at once (0 if that cannot be found out).
+template <typename K>
+static int slstm_resident_clusters(K kern, int ncta, int threads, size_t smem) {
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ncta);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ncta;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+  return n;
+}
+
+// One cluster of `ncta` blocks per (head, batch group); the launch may overlap the tail of the kernel in front of it.
+template <typename K, typename P>
+static cudaError_t slstm_launch(K kern, const P& p, int ncta, int groups, int threads, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ncta, p.NH, groups);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ncta;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kern, p);
+}
 
 }  // namespace xl

@@ -30,6 +30,8 @@
 // (i', raw f, tanh z, sigmoid o as bf16 pairs), its h' and its c', n', m' in fp32 -- into a cache that the backward
 // kernel (slstm_bwd.cu) reads back by the same (warp, lane) index (the counterpart of the reference's `states` and
 // gate caches, slstm.cc:88-101).  The 12 KB of a step are staged in shared memory and leave as one bulk copy.
+#include <atomic>
+
 #include "common.cuh"
 #include "slstm_common.cuh"
 
@@ -54,6 +56,17 @@ __device__ __forceinline__ int next_boundary(const xl_slstm_params& p, int gb, i
   if (idx > p.num_docs) return 0x7fffffff;
   const long long pos = p.cu_seqlens[idx];
   return pos < row0 + p.S ? (int)(pos - row0) : 0x7fffffff;
+}
+
+// index of the first offset beyond the start of batch row gb
+__device__ __forceinline__ int first_boundary_after(const xl_slstm_params& p, int gb) {
+  const long long row0 = (long long)gb * p.S;
+  int lo = 0, hi = p.num_docs + 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if ((long long)p.cu_seqlens[mid] > row0) hi = mid; else lo = mid + 1;
+  }
+  return lo;
 }
 
 template <int DH, bool TRAIN>
@@ -86,6 +99,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) slstm_forward_kernel(const xl_s
   const int gb_a = bgroup * SL_ROWS + row_a, gb_b = bgroup * SL_ROWS + row_b;  // global batch rows
   const bool ok_a = gb_a < B, ok_b = gb_b < B;
 
+  grid_dependency_wait();
   // ---- recurrent matrix slice -> registers (B fragments).  R is (NH, DH_in, 4, DH_out).
   uint32_t rfrag[KSTEPS][4][2];
   {
@@ -136,14 +150,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) slstm_forward_kernel(const xl_s
       const int gb = r == 0 ? gb_a : gb_b;
       const bool ok = r == 0 ? ok_a : ok_b;
       if (!ok) continue;
-      // binary search for the first boundary beyond the start of row gb, then the shared helper
-      const long long row0 = (long long)gb * S;
-      int lo = 0, hi = p.num_docs + 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if ((long long)p.cu_seqlens[mid] > row0) hi = mid; else lo = mid + 1;
-      }
-      nxt_idx[r] = lo;
+      nxt_idx[r] = first_boundary_after(p, gb);
       nxt_t[r] = next_boundary(p, gb, 0, nxt_idx[r]);
     }
   }
@@ -351,26 +358,310 @@ __global__ void __launch_bounds__(SL_THREADS, 1) slstm_forward_kernel(const xl_s
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same recurrence for clusters of EIGHT batch rows: the rows are the N = 8 side of m16n8k16 and the recurrent matrix the
+// A operand, so that a step costs 32 products per warp instead of 64, two (row, unit) pairs of gate arithmetic per thread
+// instead of four, and 4 KB of h per CTA instead of 8.  The step chain is what the kernel is bound by, and a batch of 16 rows
+// now uses 64 SMs where it used 32: 1.90 -> SL8_FWD_MS ms at B = 16, S = 2048, 4 x 256.
+//
+// Rows of an A tile are (gate, unit): tile 0 = input gate of the warp's eight units, then their forget gate; tile 1 = z, o.
+// A thread's accumulators are then all four gates of unit lane/4 for batch rows 2 (lane%4) and + 1.  Tiles in shared memory
+// are 16-byte granules chosen so that every access is one conflict-free ldmatrix:
+//   h   [unit group][row]                 granule = eight units of one row: B operand as it lies; a push fills whole sectors
+//   Wx  [gate][unit group][row]           transposed by the load into the accumulators' layout
+//   R   [warp][gate][k] (set-up only)     transposed by the load into A fragments; read coalesced, where the direct
+//                                         fragment loads were 256 two-byte loads per thread (what a one-token call waited for)
+// h' leaves the accumulator layout through one movmatrix: a thread then holds two units of row lane/4.
+template <int DH, bool TRAIN>
+struct Sl8Layout {
+  static constexpr int H_TILE = SL8_ROWS * DH * 2;                      // bytes
+  static constexpr int WX_STEP = SL8_ROWS * 4 * SL_UNITS * 2;
+  static constexpr int OFF_WX = 2 * H_TILE;
+  static constexpr int OFF_BAR = OFF_WX + SL_RING * WX_STEP;            // 2 mbarriers: h tile 0 / 1 complete
+  static constexpr int OFF_REC = OFF_BAR + 16;                          // TRAIN: staging of the records
+  static constexpr int OFF_R = OFF_REC + (TRAIN ? SL_REC_SLOTS * SL8_REC_STEP : 0);
+  static constexpr int TOTAL = OFF_R + DH * 4 * SL_UNITS * 2;
+};
+
+template <int DH, bool TRAIN>
+__global__ void __launch_bounds__(SL_THREADS, 1) slstm_forward_rows8_kernel(const xl_slstm_params p) {
+  using LY = Sl8Layout<DH, TRAIN>;
+  constexpr int KSTEPS = DH / 16, NCTA = DH / SL_UNITS;
+  extern __shared__ __align__(16) unsigned char sl_smem[];
+  const uint32_t s_h = smem_u32(sl_smem), s_wx = s_h + LY::OFF_WX, s_bar = s_h + LY::OFF_BAR, s_r = s_h + LY::OFF_R;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t rank = cluster_ctarank();       // which 32-unit slice of the head
+  const int head = blockIdx.y, bgroup = blockIdx.z;
+  const int B = p.B, S = p.S, NH = p.NH, H = NH * DH;
+  const int unit_h = (int)rank * SL_UNITS + warp * 8 + (lane >> 2);                 // this thread's unit within the head
+  const int gb0 = bgroup * SL8_ROWS + 2 * (lane & 3);                               // its two batch rows: gb0, gb0 + 1
+  const bool ok_row[2] = {gb0 < B, gb0 + 1 < B};
+
+  if (tid == 0) {
+    mbar_init(s_bar, 1);      // one arrival per phase: the local expect_tx
+    mbar_init(s_bar + 8, 1);
+    fence_barrier_init();
+  }
+  for (int i = tid; i < 2 * LY::H_TILE / 16; i += SL_THREADS) reinterpret_cast<uint4*>(sl_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+  grid_dependency_wait();
+
+  // ---- this CTA's slice of R, (NH, DH_in, 4, DH_out), into shared memory; then the first Wx steps behind it
+  {
+    const __nv_bfloat16* R = reinterpret_cast<const __nv_bfloat16*>(p.R) + (size_t)head * DH * 4 * DH + rank * SL_UNITS;
+#pragma unroll 8
+    for (int i = tid; i < DH * 16; i += SL_THREADS) {
+      const int w = i & 3, g = (i >> 2) & 3, k = i >> 4;
+      cp_async16(s_r + ((w * 4 + g) * DH + k) * 16, R + ((size_t)k * 4 + g) * DH + w * 8);
+    }
+    cp_async_commit();
+  }
+  // ---- Wx ring: one 16-byte granule (row, gate, eight units) per thread and step
+  const int wrow = tid >> 4, wgate = (tid >> 2) & 3, wpart = tid & 3;
+  const __nv_bfloat16* wx_src;
+  {
+    int gb = bgroup * SL8_ROWS + wrow;
+    gb = gb < B ? gb : B - 1;                          // padded rows re-read a valid row (result unused)
+    wx_src = reinterpret_cast<const __nv_bfloat16*>(p.wx) + ((size_t)gb * S * 4 + wgate) * H + (size_t)head * DH + rank * SL_UNITS + wpart * 8;
+  }
+  const uint32_t wx_dst = s_wx + ((wgate * 4 + wpart) * SL8_ROWS + wrow) * 16;
+  auto issue_wx = [&](int t) {
+    if (t < S) cp_async16(wx_dst + (t % SL_RING) * LY::WX_STEP, wx_src + (size_t)t * 4 * H);
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int t = 0; t < SL_RING - 1; ++t) issue_wx(t);
+
+  // ---- bias, state and document boundaries of this thread's unit and rows
+  float bias[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) bias[g] = p.bias[((size_t)head * 4 + g) * DH + unit_h];
+  float c_[2], n_[2], m_[2], hlast[2];
+  int nxt_idx[2] = {0, 0}, nxt_t[2] = {0x7fffffff, 0x7fffffff};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const size_t off = (size_t)(gb0 + i) * H + (size_t)head * DH + unit_h;
+    const bool have = p.state0 != nullptr && ok_row[i];
+    hlast[i] = have ? p.state0[0 * (size_t)B * H + off] : 0.f;
+    c_[i] = have ? p.state0[1 * (size_t)B * H + off] : 0.f;
+    n_[i] = have ? p.state0[2 * (size_t)B * H + off] : 0.f;
+    m_[i] = have ? p.state0[3 * (size_t)B * H + off] : 0.f;
+    if (p.cu_seqlens && ok_row[i]) {
+      nxt_idx[i] = first_boundary_after(p, gb0 + i);
+      nxt_t[i] = next_boundary(p, gb0 + i, 0, nxt_idx[i]);
+    }
+  }
+  __syncthreads();   // (the zeroed h tiles)
+  if (p.state0) {    // tile 0 holds h_{-1}; every CTA fills its own copy completely
+    for (int i = tid; i < SL8_ROWS * DH; i += SL_THREADS) {
+      const int r = i / DH, d = i % DH, gb = bgroup * SL8_ROWS + r;
+      if (gb < B) reinterpret_cast<__nv_bfloat16*>(sl_smem)[(d >> 3) * 64 + r * 8 + (d & 7)] = __float2bfloat16_rn(p.state0[(size_t)gb * H + (size_t)head * DH + d]);
+    }
+  }
+
+  // ---- R -> A fragments: [k-step][gate][k half], a register = (unit lane/4; k = 2 (lane%4) and + 1)
+  cp_async_wait<SL_RING - 1>();
+  __syncthreads();
+  uint32_t rfrag[KSTEPS][4][2];
+  {
+    // lanes 0-7, 8-15: the two k halves of one gate; 16-23, 24-31: those of the next
+    const uint32_t src = s_r + ((warp * 4 + (lane >> 4)) * DH + ((lane >> 3) & 1) * 8 + (lane & 7)) * 16;
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ++ks)
+#pragma unroll
+      for (int g = 0; g < 4; g += 2)
+        ldmatrix_x4_trans(src + (g * DH + ks * 16) * 16, rfrag[ks][g][0], rfrag[ks][g][1], rfrag[ks][g + 1][0], rfrag[ks][g + 1][1]);
+  }
+  cp_async_wait<SL_RING - 2>();   // step 0 has landed (this thread's part)
+  cluster_barrier();              // all CTAs of the cluster initialised; also a CTA-wide barrier
+
+  // Pushes: eight lanes send the warp's eight granules (one batch row each) to one CTA, so a store reaches four CTAs.
+  const int prow = lane & 7;
+  const uint32_t pslot = (uint32_t)((((int)rank * 4 + warp) * SL8_ROWS + prow) * 16);
+  const uint32_t ldm_h = s_h + (uint32_t)lane * 16;                                            // + 512 B per pair of k-steps
+  const uint32_t ldm_wx = s_wx + (uint32_t)((((lane >> 3) * 4 + warp) * SL8_ROWS + (lane & 7)) * 16);   // matrix = gate
+
+  // output: row lane/4, two units
+  const int orow = bgroup * SL8_ROWS + (lane >> 2);
+  uint32_t* hout = reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(p.h_out) +
+                                               ((size_t)(orow < B ? orow : 0) * NH + head) * (size_t)S * DH + rank * SL_UNITS + warp * 8 + 2 * (lane & 3));
+  unsigned char* rec = nullptr;
+  if constexpr (TRAIN)
+    rec = reinterpret_cast<unsigned char*>(p.train_cache) + (((size_t)bgroup * NH + head) * NCTA + rank) * (size_t)S * SL8_REC_STEP;
+
+  bool ok = true;
+  for (int t = 0; t < S; ++t) {
+    issue_wx(t + SL_RING - 1);
+    const int cur = t & 1, nxt = cur ^ 1;
+    // this step's h_t will land in tile `nxt` of this CTA: announce its size on that tile's barrier
+    if (tid == 0) mbar_expect_tx(s_bar + 8u * nxt, LY::H_TILE);
+    // accumulators start from Wx + bias; the second set takes every other k-step (a chain of dependent products runs at
+    // its latency, not at its issue rate)
+    float acc[2][4], acb[2][4];
+    {
+      uint32_t w[4];
+      ldmatrix_x4_trans(ldm_wx + (t % SL_RING) * LY::WX_STEP, w[0], w[1], w[2], w[3]);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const float2 v = unpack_bf16x2(w[g]);
+        acc[g >> 1][2 * (g & 1)] = v.x + bias[g];
+        acc[g >> 1][2 * (g & 1) + 1] = v.y + bias[g];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acb[0][i] = acb[1][i] = 0.f;
+    }
+    // h_{t-1} complete in tile `cur` (phases as in the sixteen-row kernel; an expired wait is acted on at the step's barrier)
+    if (t >= 1 && !sl_wait(s_bar + 8u * cur, (uint32_t)((t >> 1) - (cur == 0 ? 1 : 0)) & 1u)) ok = false;
+    const uint32_t hbase = ldm_h + cur * LY::H_TILE;
+#pragma unroll
+    for (int kp = 0; kp < KSTEPS / 2; ++kp) {
+      uint32_t b0, b1, b2, b3;
+      ldmatrix_x4(hbase + kp * 512, b0, b1, b2, b3);
+      mma_bf16_16816(acc[0], rfrag[2 * kp][0][0], rfrag[2 * kp][1][0], rfrag[2 * kp][0][1], rfrag[2 * kp][1][1], b0, b1);
+      mma_bf16_16816(acc[1], rfrag[2 * kp][2][0], rfrag[2 * kp][3][0], rfrag[2 * kp][2][1], rfrag[2 * kp][3][1], b0, b1);
+      mma_bf16_16816(acb[0], rfrag[2 * kp + 1][0][0], rfrag[2 * kp + 1][1][0], rfrag[2 * kp + 1][0][1], rfrag[2 * kp + 1][1][1], b2, b3);
+      mma_bf16_16816(acb[1], rfrag[2 * kp + 1][2][0], rfrag[2 * kp + 1][3][0], rfrag[2 * kp + 1][2][1], rfrag[2 * kp + 1][3][1], b2, b3);
+    }
+    float hn[2];
+    [[maybe_unused]] float gi[2], gf[2], gz[2], go[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float ir = acc[0][i] + acb[0][i], fr = acc[0][2 + i] + acb[0][2 + i], zr = acc[1][i] + acb[1][i], orr = acc[1][2 + i] + acb[1][2 + i];
+      const float lfm = m_[i] + fast_logsigmoid(fr);
+      const bool fresh = n_[i] == 0.f;
+      const float d = lfm - ir;
+      const float mn = (fresh || d <= 0.f) ? ir : lfm;
+      const float e = __expf(-fabsf(d));
+      const float ig = (d > 0.f && !fresh) ? e : 1.f;
+      const float fg = (d <= 0.f) ? e : 1.f;
+      const float zt = tanh_approx(zr), os = fmaf(0.5f, tanh_approx(0.5f * orr), 0.5f);
+      c_[i] = fmaf(fg, c_[i], ig * zt);
+      n_[i] = fmaf(fg, n_[i], ig);
+      m_[i] = mn;
+      hn[i] = __fdividef(c_[i], n_[i]) * os;
+      if constexpr (TRAIN) { gi[i] = ig; gf[i] = fr; gz[i] = zt; go[i] = os; }
+    }
+    const uint32_t hp = pack_bf16x2(hn[0], hn[1]);
+    // a row whose next token opens a new document restarts from the zero state
+    uint32_t push = hp;
+    if (p.cu_seqlens) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (t + 1 == nxt_t[i]) {
+          push &= i == 0 ? 0xffff0000u : 0x0000ffffu;
+          c_[i] = n_[i] = m_[i] = 0.f;
+          nxt_t[i] = next_boundary(p, gb0 + i, t + 1, nxt_idx[i]);
+        }
+    }
+    // broadcast h_t into tile `nxt` of every CTA in the cluster
+    const uint32_t pw = movmatrix_trans(push);
+    {
+      uint32_t gr[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) gr[i] = __shfl_sync(0xffffffffu, pw, 4 * prow + i);
+      const uint32_t dst_tile = s_h + nxt * LY::H_TILE + pslot;
+#pragma unroll
+      for (int r = 0; r < NCTA; r += 4) {
+        const uint32_t dst = (uint32_t)(r + (lane >> 3));
+        if (NCTA >= 4 || dst < (uint32_t)NCTA) st_async_v4(map_to_cta(dst_tile, dst), gr, map_to_cta(s_bar + 8u * nxt, dst));
+      }
+    }
+    if constexpr (TRAIN) {
+      uint4* r = reinterpret_cast<uint4*>(sl_smem + LY::OFF_REC + (t % SL_REC_SLOTS) * SL8_REC_STEP + tid * SL8_REC_BYTES);
+      r[0] = make_uint4(pack_bf16x2(gi[0], gi[1]), pack_bf16x2(gf[0], gf[1]), pack_bf16x2(gz[0], gz[1]), pack_bf16x2(go[0], go[1]));
+      r[1] = make_uint4(hp, 0u, __float_as_uint(c_[0]), __float_as_uint(c_[1]));
+      r[2] = make_uint4(__float_as_uint(n_[0]), __float_as_uint(n_[1]), __float_as_uint(m_[0]), __float_as_uint(m_[1]));
+      fence_proxy_async_smem();
+    }
+    // output h_t, (B, NH, S, DH) -- after the pushes: they are on the step-to-step chain, this store is not
+    {
+      const uint32_t ow = p.cu_seqlens ? movmatrix_trans(hp) : pw;
+      if (orow < B) hout[(size_t)t * (DH / 2)] = ow;
+    }
+    hlast[0] = hn[0];
+    hlast[1] = hn[1];
+    cp_async_wait<SL_RING - 2>();  // this thread's part of step t+1 has landed
+    // ... and everybody else's (CTA-wide only); the same barrier tells every thread whether any wait expired
+    if (__syncthreads_or(ok ? 0 : 1)) { ok = false; break; }
+    if constexpr (TRAIN) {
+      if (tid == 0) {
+        bulk_store(rec + (size_t)t * SL8_REC_STEP, s_h + LY::OFF_REC + (t % SL_REC_SLOTS) * SL8_REC_STEP, SL8_REC_STEP);
+        bulk_commit();
+        bulk_wait_read<1>();   // the copy of step t-1 has read its slot: step t+2, which reuses it, may stage (behind the next barrier)
+      }
+    }
+  }
+  if constexpr (TRAIN) {
+    if (tid == 0) bulk_wait<0>();
+  }
+  // the pushes of h_{S-1} are waited for before anybody may leave (see the sixteen-row kernel)
+  if (ok) {
+    const int last = S & 1;
+    if (!sl_wait(s_bar + 8u * last, (uint32_t)((S >> 1) - (last == 0 ? 1 : 0)) & 1u)) ok = false;
+  }
+  if (!ok && p.status) atomicExch(p.status, 1);
+  cluster_barrier();  // nobody leaves while a peer may still push into its tile
+
+  // final state (4, B, H): h, c, n, m
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (!ok_row[i]) continue;
+    const size_t off = (size_t)(gb0 + i) * H + (size_t)head * DH + unit_h;
+    p.state_out[0 * (size_t)B * H + off] = hlast[i];
+    p.state_out[1 * (size_t)B * H + off] = c_[i];
+    p.state_out[2 * (size_t)B * H + off] = n_[i];
+    p.state_out[3 * (size_t)B * H + off] = m_[i];
+  }
+}
+
+template <int DH, bool TRAIN>
+static constexpr size_t slstm_smem() {
+  return 2 * SL_ROWS * DH * 2 + (size_t)SL_RING * SL_WX_STEP_BYTES + 16 +  // + 2 mbarriers
+         (TRAIN ? (size_t)SL_REC_SLOTS * SL_REC_STEP : 0);
+}
+
 template <int DH, bool TRAIN>
 static int launch_slstm(const xl_slstm_params* p, cudaStream_t st) {
   constexpr int NCTA = DH / SL_UNITS;
-  const size_t smem = 2 * SL_ROWS * DH * 2 + (size_t)SL_RING * SL_WX_STEP_BYTES + 16 +  // + 2 mbarriers
-                      (TRAIN ? (size_t)SL_REC_SLOTS * SL_REC_STEP : 0);
-  XL_CUDA_TRY(cudaFuncSetAttribute(slstm_forward_kernel<DH, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(NCTA, p->NH, (p->B + SL_ROWS - 1) / SL_ROWS);
-  cfg.blockDim = dim3(SL_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = NCTA;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  XL_CUDA_TRY(cudaLaunchKernelEx(&cfg, slstm_forward_kernel<DH, TRAIN>, *p));
+  if (slstm_rows8(p->B, p->NH, DH, TRAIN)) {
+    constexpr size_t smem = Sl8Layout<DH, TRAIN>::TOTAL;
+    auto kern = slstm_forward_rows8_kernel<DH, TRAIN>;
+    XL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    XL_CUDA_TRY(slstm_launch(kern, *p, NCTA, (p->B + SL8_ROWS - 1) / SL8_ROWS, SL_THREADS, smem, st));
+  } else {
+    constexpr size_t smem = slstm_smem<DH, TRAIN>();
+    auto kern = slstm_forward_kernel<DH, TRAIN>;
+    XL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    XL_CUDA_TRY(slstm_launch(kern, *p, NCTA, (p->B + SL_ROWS - 1) / SL_ROWS, SL_THREADS, smem, st));
+  }
   return check_launch("xl_slstm_forward");
+}
+
+template <int DH>
+static int max_clusters_fwd8(bool train) {
+  return train ? slstm_resident_clusters(slstm_forward_rows8_kernel<DH, true>, DH / SL_UNITS, SL_THREADS, Sl8Layout<DH, true>::TOTAL)
+               : slstm_resident_clusters(slstm_forward_rows8_kernel<DH, false>, DH / SL_UNITS, SL_THREADS, Sl8Layout<DH, false>::TOTAL);
+}
+int slstm_max_clusters_fwd8(int DH, bool train) {
+  return DH == 64 ? max_clusters_fwd8<64>(train) : DH == 128 ? max_clusters_fwd8<128>(train) : max_clusters_fwd8<256>(train);
+}
+
+bool slstm_rows8(int B, int NH, int DH, bool train) {
+  // residency per device and head size, asked for once: [device][DH][train]
+  static std::atomic<int> limits[64][3][2];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { (void)cudaGetLastError(); return false; }
+  std::atomic<int>& slot = limits[dev][DH == 64 ? 0 : DH == 128 ? 1 : 2][train];
+  int limit = slot.load(std::memory_order_relaxed);   // 1 + clusters; 0: not asked yet
+  if (limit == 0) {
+    limit = slstm_max_clusters_fwd8(DH, train);
+    if (train) {
+      const int bwd = slstm_max_clusters_bwd8(DH);
+      limit = bwd < limit ? bwd : limit;
+    }
+    slot.store(++limit, std::memory_order_relaxed);
+  }
+  return (long long)((B + SL8_ROWS - 1) / SL8_ROWS) * NH < limit;
 }
 
 }  // namespace xl

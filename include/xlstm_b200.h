@@ -183,8 +183,8 @@ int64_t xl_slstm_cache_bytes(int32_t B, int32_t S, int32_t NH, int32_t DH);
  * SLSTMPointwiseBackward (slstm_pointwise.cu:118-196).  Per step the gate gradients are formed in registers from the
  * cache, written out as dWx, and carried back through the recurrent matrix (held in registers) with a reduce-scatter
  * between the CTAs of a cluster.  The stabiliser state m gets no gradient (dstate0[3] = 0), as in the reference.
- * The gradients of R and of the bias are sums over (b,t) of h_{t-1} (x) dWx_t and of dWx_t -- plain matrix products
- * over this kernel's output that the caller's GEMM library forms (the reference does the same after its loop). */
+ * The gradients of R and of the bias are sums over (b,t) of h_{t-1} (x) dWx_t and of dWx_t over this kernel's output:
+ * xl_slstm_weight_grads (the reference forms them after its loop, too). */
 typedef struct xl_slstm_bwd_params {
   const void* cache;        /* written by xl_slstm_forward with train_cache set, same B,S,NH,DH */
   const void* R;            /* (NH, DH_in, 4, DH_out), dtype `dtype` */
@@ -200,6 +200,25 @@ typedef struct xl_slstm_bwd_params {
 
 /* Requires DH in {64,128,256}, dtype XL_BF16; no document offsets. */
 int xl_slstm_backward(const xl_slstm_bwd_params* p, void* cuda_stream);
+
+/* Gradients of the recurrent matrix and of the bias from dWx and the forward's h, one pass over both on the tensor cores
+ * (the GEMMs behind the time loop of the reference's BackwardPass::Run, slstm_backward.cu). */
+typedef struct xl_slstm_wgrad_params {
+  const void* dwx;          /* (B, S, 4, NH, DH), contiguous, 16-byte aligned */
+  const void* h;            /* (B, NH, S, DH), contiguous, 16-byte aligned */
+  const void* h0;           /* (B, NH, DH) initial h, or NULL = zeros */
+  float* dR;                /* out (NH, DH_in, 4, DH_out) */
+  float* dbias;             /* out (NH, 4, DH) */
+  void* scratch;            /* xl_slstm_weight_grads_scratch_bytes, 16-byte aligned */
+  int64_t scratch_bytes;
+  int32_t* status;
+  int32_t B, S, NH, DH;
+  int32_t dtype;            /* of dwx, h, h0 */
+} xl_slstm_wgrad_params;
+
+/* Requires DH in {64,128,256}, dtype XL_BF16. */
+int xl_slstm_weight_grads(const xl_slstm_wgrad_params* p, void* cuda_stream);
+int64_t xl_slstm_weight_grads_scratch_bytes(int32_t B, int32_t S, int32_t NH, int32_t DH);
 
 /* ------------------------------------------------------------------------------------------------
  * Operators next to the mLSTM cell in the reference's layer (xlstm/xlstm_large/model.py:379-452), each one pass

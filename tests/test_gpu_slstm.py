@@ -216,3 +216,34 @@ def test_forward_and_backward_are_bit_identical_from_run_to_run():
         else:
             assert all(torch.equal(a, b) for a, b in zip(first, cur))
     xlstm_b200.check_device_status()
+
+
+@pytest.mark.parametrize("B,S,NH,DH,with_state", [(1, 1, 1, 64, False), (3, 1, 2, 128, True), (1, 2, 3, 256, False), (2, 65, 2, 64, True),
+                                                  (3, 66, 1, 128, False), (5, 257, 4, 256, True), (16, 640, 4, 256, False), (1, 300, 40, 256, True)])
+def test_weight_grads_kernel(B, S, NH, DH, with_state):
+    """dR and dbias against 64 bits: tile edges (S - 1 = 64 n and + 1), one and many splits, more units than SMs.  Products
+    of bf16 values are exact in fp32 and the sums are fp32, so 1e-5 is many times their error.  h_{S-1} never enters, dWx_0
+    enters dbias and (with an initial state) the product with h0 only: a NaN and an infinity there must not leak."""
+    from xlstm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(B * S + DH)
+    dwx = torch.randn(B, S, 4 * NH * DH, generator=g, device="cuda").bfloat16()
+    h = torch.randn(B, NH, S, DH, generator=g, device="cuda").bfloat16()
+    st = torch.randn(4, B, NH * DH, generator=g, device="cuda") if with_state else None
+    assert ops._weight_grads_native(dwx.reshape(B, S, 4, NH, DH), h, st)
+    w64 = dwx.double().reshape(B, S, 4, NH, DH)
+    ref = torch.einsum("bntk,btgnu->nkgu", h.double()[:, :, :-1], w64[:, 1:])
+    if with_state:
+        ref = ref + torch.einsum("bnk,bgnu->nkgu", st[0].bfloat16().double().reshape(B, NH, DH), w64[:, 0])
+    h[:, :, -1] = float("nan")
+    dR, db = ops.slstm_weight_grads(dwx, h, st)
+    import xlstm_b200
+    xlstm_b200.check_device_status()
+    assert dR.shape == (NH, DH, 4, DH) and db.shape == (NH, 4, DH)
+    assert float((dR - ref).norm()) <= 1e-5 * float(ref.norm())
+    assert float((db - w64.sum((0, 1)).permute(1, 0, 2)).norm()) <= 1e-5 * float(w64.sum((0, 1)).norm())
+    again = ops.slstm_weight_grads(dwx, h, st)
+    assert torch.equal(again[0], dR) and torch.equal(again[1], db)
+    if not with_state:
+        dwx[:, 0] = float("inf")
+        dR, db = ops.slstm_weight_grads(dwx, h)
+        assert float((dR - ref).norm()) <= 1e-5 * float(ref.norm()) and bool(torch.isinf(db).all())

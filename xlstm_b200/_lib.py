@@ -21,7 +21,7 @@ EXPORTS = (
     "xl_add_rmsnorm", "xl_headnorm_gate", "xl_soft_cap", "xl_causal_conv1d",
     "xl_softcap_argmax", "xl_softcap_argmax_scratch_bytes", "xl_swiglu",
     "xl_softcap_argmax_noalloc", "xl_softcap_argmax_noalloc_max_rows", "xl_peer_reduce_add_rmsnorm", "xl_headwise_proj", "xl_mlstm_decode_cell",
-    "xl_slstm_backward", "xl_slstm_cache_bytes",
+    "xl_slstm_backward", "xl_slstm_cache_bytes", "xl_slstm_weight_grads", "xl_slstm_weight_grads_scratch_bytes",
 )
 
 
@@ -71,6 +71,14 @@ class SlstmBwdParams(C.Structure):
     _fields_ = [
         ("cache", C.c_void_p), ("R", C.c_void_p), ("dh", C.c_void_p), ("dstate_out", C.c_void_p),
         ("state0", C.c_void_p), ("dwx", C.c_void_p), ("dstate0", C.c_void_p), ("status", C.c_void_p),
+        ("B", C.c_int32), ("S", C.c_int32), ("NH", C.c_int32), ("DH", C.c_int32), ("dtype", C.c_int32),
+    ]
+
+
+class SlstmWgradParams(C.Structure):
+    _fields_ = [
+        ("dwx", C.c_void_p), ("h", C.c_void_p), ("h0", C.c_void_p), ("dR", C.c_void_p), ("dbias", C.c_void_p),
+        ("scratch", C.c_void_p), ("scratch_bytes", C.c_int64), ("status", C.c_void_p),
         ("B", C.c_int32), ("S", C.c_int32), ("NH", C.c_int32), ("DH", C.c_int32), ("dtype", C.c_int32),
     ]
 
@@ -187,7 +195,7 @@ def lib() -> C.CDLL:
                             ("xl_soft_cap", SoftCapParams), ("xl_causal_conv1d", Conv1dParams),
                             ("xl_softcap_argmax", GreedyParams), ("xl_swiglu", SwigluParams),
                             ("xl_softcap_argmax_noalloc", GreedyParams), ("xl_peer_reduce_add_rmsnorm", PeerReduceParams),
-                            ("xl_slstm_backward", SlstmBwdParams)):
+                            ("xl_slstm_backward", SlstmBwdParams), ("xl_slstm_weight_grads", SlstmWgradParams)):
             fn = getattr(l, name)
             fn.restype = C.c_int
             fn.argtypes = [C.POINTER(ptype), C.c_void_p]
@@ -200,6 +208,8 @@ def lib() -> C.CDLL:
         l.xl_softcap_argmax_noalloc_max_rows.restype = C.c_int32
         l.xl_slstm_cache_bytes.restype = C.c_int64
         l.xl_slstm_cache_bytes.argtypes = [C.c_int32] * 4
+        l.xl_slstm_weight_grads_scratch_bytes.restype = C.c_int64
+        l.xl_slstm_weight_grads_scratch_bytes.argtypes = [C.c_int32] * 4
         _lib = l
     return _lib
 

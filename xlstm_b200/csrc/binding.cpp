@@ -364,6 +364,35 @@ PyObject* slstm_backward(PyObject*, PyObject* const* a, Py_ssize_t na) {
   END_HANDLE_TH_ERRORS
 }
 
+// (dwx (B,S,4,NH,DH), h (B,NH,S,DH), h0 (B,NH,DH) or None) -> (dR, dbias); all bf16 and as the kernel takes them (see ops.py)
+PyObject* slstm_weight_grads(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  want_args(na, 3);
+  const Tensor &dwx = tensor_arg(a[0], "dwx"), &h = tensor_arg(a[1], "h");
+  const Tensor* h0 = optional_arg(a[2], "h0");
+  for (const Tensor* t : {&dwx, &h, h0}) {
+    require_cuda(t);
+    TORCH_CHECK_VALUE(!t || (t->scalar_type() == at::kBFloat16 && t->is_contiguous() && t->device() == dwx.device()),
+                      "slstm_weight_grads: contiguous bf16 tensors on one device");
+  }
+  TORCH_CHECK_VALUE(h.dim() == 4, "h must be (B,NH,S,DH)");
+  const int64_t B = h.size(0), NH = h.size(1), S = h.size(2), DH = h.size(3);
+  TORCH_CHECK_VALUE(dwx.sizes() == at::IntArrayRef({B, S, 4, NH, DH}) && (!h0 || h0->sizes() == at::IntArrayRef({B, NH, DH})), "inconsistent sLSTM shapes");
+  const c10::cuda::CUDAGuard guard(h.device());
+  const Tensor dR = empty_on({NH, DH, 4, DH}, at::kFloat, h), db = empty_on({NH, 4, DH}, at::kFloat, h);
+  const int64_t bytes = xl_slstm_weight_grads_scratch_bytes(B, S, NH, DH);
+  const Tensor scratch = bytes ? empty_on({bytes}, at::kByte, h) : Tensor();   // (stream-ordered: free for the allocator at return)
+  xl_slstm_wgrad_params p = {};
+  p.dwx = dwx.data_ptr(); p.h = h.data_ptr(); p.h0 = h0 ? h0->data_ptr() : nullptr;
+  p.dR = dR.data_ptr<float>(); p.dbias = db.data_ptr<float>();
+  p.scratch = bytes ? scratch.data_ptr() : nullptr; p.scratch_bytes = bytes;
+  p.status = status_ptr(h);
+  p.B = B; p.S = S; p.NH = NH; p.DH = DH; p.dtype = XL_BF16;
+  check(xl_slstm_weight_grads(&p, stream_of(h)), "xl_slstm_weight_grads");
+  return pack({dR, db});
+  END_HANDLE_TH_ERRORS
+}
+
 // ---------------------------------------------------------------------------------------------- operators next to the cells
 // (rows, D) view of (..., D) with contiguous rows
 Tensor as_rows(const Tensor& t, int64_t D) {
@@ -653,7 +682,7 @@ PyObject* status_word(PyObject*, PyObject* index) {
 
 #define XL_FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
-    XL_FAST(mlstm_sequence), XL_FAST(mlstm_step), XL_FAST(mlstm_decode_cell), XL_FAST(slstm_forward), XL_FAST(slstm_backward),
+    XL_FAST(mlstm_sequence), XL_FAST(mlstm_step), XL_FAST(mlstm_decode_cell), XL_FAST(slstm_forward), XL_FAST(slstm_backward), XL_FAST(slstm_weight_grads),
     XL_FAST(add_rmsnorm), XL_FAST(headnorm_gate), XL_FAST(soft_cap), XL_FAST(causal_conv1d), XL_FAST(headwise_proj), XL_FAST(softcap_argmax),
     XL_FAST(document_offsets), XL_FAST(slot_vector),
     {"swiglu", swiglu, METH_O, nullptr}, {"status_word", status_word, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};

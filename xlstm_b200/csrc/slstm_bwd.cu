@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(SLB_THREADS, 1) slstm_backward_kernel(const xl
 // ---------------------------------------------------------------------------------------------
 // Clusters of EIGHT batch rows (the counterpart of slstm_forward_rows8_kernel): the rows are the N = 8 side of the products
 // and R the A operand, dh_{t-1}^T [DH x 8] = R [DH x 128] dg^T [128 x 8], so a step costs 16 products per warp instead of 32,
-// half the exchange and one (row, unit) pair of gate arithmetic per thread, on twice the SMs: 2.79 -> SL8_BWD_MS ms at B = 16,
+// half the exchange and one (row, unit) pair of gate arithmetic per thread, on twice the SMs: 2.79 -> 2.04 ms at B = 16,
 // S = 2048, 4 x 256.
 //
 // Eight warps: warps 2w and 2w+1 share the pairs of forward warp w -- thread (w, lane) of the forward owns unit 8w + lane/4 and

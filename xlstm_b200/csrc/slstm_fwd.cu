@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) slstm_forward_kernel(const xl_s
 // The same recurrence for clusters of EIGHT batch rows: the rows are the N = 8 side of m16n8k16 and the recurrent matrix the
 // A operand, so that a step costs 32 products per warp instead of 64, two (row, unit) pairs of gate arithmetic per thread
 // instead of four, and 4 KB of h per CTA instead of 8.  The step chain is what the kernel is bound by, and a batch of 16 rows
-// now uses 64 SMs where it used 32: 1.90 -> SL8_FWD_MS ms at B = 16, S = 2048, 4 x 256.
+// now uses 64 SMs where it used 32: 1.90 -> 1.13 ms at B = 16, S = 2048, 4 x 256.
 //
 // Rows of an A tile are (gate, unit): tile 0 = input gate of the warp's eight units, then their forget gate; tile 1 = z, o.
 // A thread's accumulators are then all four gates of unit lane/4 for batch rows 2 (lane%4) and + 1.  Tiles in shared memory

@@ -191,13 +191,32 @@ def slstm_backward(cache, R, dh, dstate_out=None, state0=None):
     return native().slstm_backward(cache, R, dh, dstate_out, state0)
 
 
+def _weight_grads_native(dw, h, state0) -> bool:
+    """Whether ``slstm_weight_grads`` runs on its kernel: contiguous, aligned bf16 tensors of one device, and nobody
+    who would have to see the single operators (autograd in either direction, function transforms, dispatch modes)."""
+    ts = [dw, h] + ([] if state0 is None else [state0])
+    if any(type(t) is not torch.Tensor or t.device != h.device for t in ts) or not h.is_cuda or h.numel() == 0:
+        return False
+    if torch.is_grad_enabled() and any(t.requires_grad for t in ts):
+        return False
+    if torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack() or torch.autograd.forward_ad._current_level >= 0:
+        return False
+    return (h.shape[-1] in (64, 128, 256) and h.shape[1] <= 4096 and
+            all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (dw, h)))
+
+
 def slstm_weight_grads(dwx, h, state0=None):
     """Gradients of the recurrent matrix and the bias from the backward kernel's output: with h_{t-1} the forward's h
     shifted by one step (h_{-1} from state0), dR[n,k,g,u] = sum_{b,t} h_{t-1}[b,n,k] dwx[b,t,g,n,u] and
     dbias[n,g,u] = sum_{b,t} dwx[b,t,g,n,u] (the reference forms the same products after its time loop,
-    slstm_backward.cu).  Plain batched matrix products, fp32 results: (NH,DH,4,DH) and (NH,4,DH)."""
+    slstm_backward.cu).  fp32 results: (NH,DH,4,DH) and (NH,4,DH).  What the backward kernel writes goes through one
+    tensor-core kernel; anything else (other devices, dtypes and head sizes, differentiable or traced calls) is formed by
+    plain batched matrix products."""
     B, NH, S, DH = h.shape
     dw = dwx.reshape(B, S, 4, NH, DH)
+    if _weight_grads_native(dw, h, state0):
+        h0 = None if state0 is None else state0[0].reshape(B, NH, DH).to(torch.bfloat16).contiguous()
+        return native().slstm_weight_grads(dw, h, h0)
 
     def mm(a, b):   # fp32 result; half-precision operands stay as they are where the GEMM library accumulates in fp32
         if a.is_cuda and a.dtype in (torch.bfloat16, torch.float16):

@@ -247,3 +247,39 @@ def test_headwise_proj_kernel_matches_oracle(rows, NH, DH, nslots):
         got3 = xlstm_b200.headwise_proj([x.cuda().view(2, rows // 2, D)], [ws[0].cuda()])
         assert got3.shape == (2, rows // 2, D)
         assert torch.equal(got3.reshape(rows, D), xlstm_b200.headwise_proj([x.cuda()], [ws[0].cuda()]))
+
+
+@pytest.mark.parametrize("NH,DH,gate,dt", [(4, 64, True, torch.bfloat16), (4, 256, False, torch.bfloat16), (3, 512, True, torch.bfloat16),
+                                           (5, 128, False, torch.float32), (4, 200, True, torch.float32)])
+def test_headnorm_with_several_tokens_per_warp_equals_one_token_per_warp(NH, DH, gate, dt):
+    """Many rows take the variant with several tokens per warp; a batch row alone takes the other one.  The arithmetic is the
+    same, so the results are equal bit for bit, ragged last groups included."""
+    import xlstm_b200
+    B = 4
+    S = 148 * 64 * 8 // (B * NH) + 2
+    S += (S + 1) % 2   # odd
+    g = torch.Generator(device="cuda").manual_seed(DH)
+    h = torch.randn(B, S, NH, DH, generator=g, device="cuda", dtype=torch.float32).to(dt).transpose(1, 2)
+    o = torch.randn(B, S, NH * DH, generator=g, device="cuda").to(dt) if gate else None
+    w = torch.randn(NH * DH, generator=g, device="cuda").to(dt)
+    got = xlstm_b200.headnorm_gate(h, o, w)
+    for b in range(B):
+        assert torch.equal(got[b:b + 1], xlstm_b200.headnorm_gate(h[b:b + 1], None if o is None else o[b:b + 1], w))
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("S", [1, 7, 8, 31, 32, 33, 75])
+def test_causal_conv1d_tile_edges_and_unaligned_weights(K, S):
+    import xlstm_b200
+    g = torch.Generator().manual_seed(31 * S + K)
+    F_ = 72
+    for dt in (torch.float32, torch.bfloat16):
+        x, w, b = (torch.randn(*s, generator=g).to(dt) for s in ((2, S, F_), (F_, K), (F_,)))
+        cu = sorted({0, S, 2 * S, min(S, 9), S + min(S, 30), S + min(S, 31)})
+        for c in (None, cu):
+            want = O.causal_conv1d(x, w, b, cu_seqlens=c)
+            got = xlstm_b200.causal_conv1d(x.cuda(), w.cuda(), b.cuda(), cu_seqlens=c)
+            _close(got, want, dt)
+            off = torch.empty(F_ * K + 1, dtype=dt, device="cuda")[1:].view(F_, K)   # starts 2 or 4 bytes past a 16-byte boundary
+            off.copy_(w)
+            assert torch.equal(xlstm_b200.causal_conv1d(x.cuda(), off, b.cuda(), cu_seqlens=c), got)

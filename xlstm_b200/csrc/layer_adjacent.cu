@@ -153,64 +153,79 @@ __global__ void __launch_bounds__(RMS_THREADS) add_rmsnorm_kernel(const xl_add_r
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// per-head LayerNorm + weight + output gate: one warp per (batch, token, head)
+// per-head LayerNorm + weight + output gate: one warp per (batch, R consecutive tokens, head)
 // ------------------------------------------------------------------------------------------------------------
 constexpr int HNG_WARPS = 8;
+// Vectors of h a warp has in flight where there are enough rows to fill the machine all the same.  With one token per warp
+// a block lived for one load latency and the launch rate of blocks bound it: 16 x 2048 tokens, 4 heads of 256 (134 MB):
+// 40 us, 36 with four tokens.
+constexpr int HNG_IN_FLIGHT = 4;
+constexpr long long HNG_FULL = 148 * 64 * 8;   // rows (token, head) from which on
 
-template <typename T, int NC>
+template <typename T, int NC, int R>
 __global__ void __launch_bounds__(HNG_WARPS * 32) headnorm_gate_kernel(const xl_headnorm_gate_params p) {
   constexpr int V = Vec16<T>::N;
   const int lane = threadIdx.x & 31;
   // 32-bit index arithmetic on purpose (grid.y = batch row): with 64-bit divisions for (batch, token, head) the index
   // computation alone was more than half of the warp's instructions
-  const unsigned unit = blockIdx.x * HNG_WARPS + (threadIdx.x >> 5);   // (token, head) within the batch row
-  if (unit >= (unsigned)p.S * (unsigned)p.NH) return;
-  const unsigned s = unit / (unsigned)p.NH, head = unit - s * (unsigned)p.NH;
+  const unsigned unit = blockIdx.x * HNG_WARPS + (threadIdx.x >> 5);   // (group of R tokens, head) within the batch row
+  if (unit >= ((unsigned)p.S + R - 1) / R * (unsigned)p.NH) return;
+  const unsigned sg = unit / (unsigned)p.NH, head = unit - sg * (unsigned)p.NH, s0 = sg * R;
   const long long b = blockIdx.y;
-  const T* h = static_cast<const T*>(p.h) + b * p.h_sb + head * p.h_sh + s * p.h_st;
-  const T* o = static_cast<const T*>(p.o) + b * p.o_sb + s * p.o_st + (long long)head * p.DH;
+  const T* h = static_cast<const T*>(p.h) + b * p.h_sb + head * p.h_sh + s0 * p.h_st;
+  const T* o = static_cast<const T*>(p.o) + b * p.o_sb + s0 * p.o_st + (long long)head * p.DH;
   const T* w = static_cast<const T*>(p.weight) + (long long)head * p.DH;
-  T* out = static_cast<T*>(p.out) + ((b * p.S + s) * p.NH + head) * p.DH;
+  T* out = static_cast<T*>(p.out) + ((b * p.S + s0) * p.NH + head) * p.DH;
 
-  // every load of the row is issued before the first use
-  Vec16<T> hv[NC], ov[NC], wv[NC];
+  // every load of the rows is issued before the first use
+  Vec16<T> hv[R][NC], ov[R][NC], wv[NC];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int e = (c * 32 + lane) * V;
-    if (e < p.DH) {
-      hv[c] = load16(h + e);
-      if (p.o) ov[c] = load16(o + e);
-      wv[c] = load16(w + e);
-    }
-  }
-  float sum = 0.f;
+  for (int r = 0; r < R; ++r)
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int e = (c * 32 + lane) * V;
-    if (e < p.DH) {
-#pragma unroll
-      for (int i = 0; i < V; ++i) sum += to_float(hv[c].v[i]);
-    }
-  }
-  const float mean = warp_sum(sum) / (float)p.DH;
-  float sq = 0.f;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int e = (c * 32 + lane) * V;
-    if (e < p.DH) {
-#pragma unroll
-      for (int i = 0; i < V; ++i) {
-        const float d = to_float(hv[c].v[i]) - mean;
-        sq = fmaf(d, d, sq);
+    for (int c = 0; c < NC; ++c) {
+      const int e = (c * 32 + lane) * V;
+      if (e < p.DH && (R == 1 || s0 + r < (unsigned)p.S)) {
+        hv[r][c] = load16(h + r * p.h_st + e);
+        if (p.o) ov[r][c] = load16(o + r * p.o_st + e);
       }
     }
-  }
-  const float r = rsqrtf(warp_sum(sq) / (float)p.DH + p.eps);
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int e = (c * 32 + lane) * V;
-    if (e < p.DH) {
-      store16(out + e, p.o ? normalise_weight_gate(hv[c], ov[c], wv[c], mean, r) : normalise_weight<T>(hv[c], wv[c], mean, r));
+    if (e < p.DH) wv[c] = load16(w + e);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (R > 1 && s0 + r >= (unsigned)p.S) break;
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int e = (c * 32 + lane) * V;
+      if (e < p.DH) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) sum += to_float(hv[r][c].v[i]);
+      }
+    }
+    const float mean = warp_sum(sum) / (float)p.DH;
+    float sq = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int e = (c * 32 + lane) * V;
+      if (e < p.DH) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          const float d = to_float(hv[r][c].v[i]) - mean;
+          sq = fmaf(d, d, sq);
+        }
+      }
+    }
+    const float rstd = rsqrtf(warp_sum(sq) / (float)p.DH + p.eps);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int e = (c * 32 + lane) * V;
+      if (e < p.DH)
+        store16(out + (long long)r * p.NH * p.DH + e, p.o ? normalise_weight_gate(hv[r][c], ov[r][c], wv[c], mean, rstd)
+                                                          : normalise_weight<T>(hv[r][c], wv[c], mean, rstd));
     }
   }
 }
@@ -273,27 +288,51 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const T* __restrict__ gz, T
 //   y[b,t,f] = bias[f] + sum_{lag=0}^{K-1} w[f][K-1-lag] x[b,t-lag,f]      (taps that reach in front of the first token of
 //   the document -- or of the row -- read zero), out = silu(round(y)).
 // A thread owns one 16-byte vector of features and walks CONV_TILE consecutive tokens with the last K-1 inputs in
-// registers, so x is read once (plus a K-1 token halo per tile) and out written once: HBM-bound.
+// registers, so x is read once (plus a K-1 token halo per tile) and out written once: HBM-bound.  The loads of CONV_GROUP
+// tokens are issued together -- one token at a time a thread waited out a load's latency per token -- and the taps are
+// compiled for the kernel size, without a test per tap unless a document starts near.
+// 16 x 2048 tokens x 1024 features, K = 4 (134 MB): 43 us, 148 before.
 // ---------------------------------------------------------------------------------------------
-constexpr int CONV_THREADS = 128, CONV_TILE = 64, CONV_MAXK = 8;
+constexpr int CONV_THREADS = 128, CONV_TILE = 32, CONV_GROUP = 8, CONV_MAXK = 8;
 
-template <typename T>
+template <typename T, int K>
 __global__ void __launch_bounds__(CONV_THREADS) causal_conv1d_kernel(const xl_conv1d_params p) {
-  constexpr int V = Vec16<T>::N;
-  const int f0 = (blockIdx.x * CONV_THREADS + threadIdx.x) * V;
+  constexpr int V = Vec16<T>::N, W = K > 1 ? K - 1 : 1;
+  const int f0 = (blockIdx.y * CONV_THREADS + threadIdx.x) * V;
   if (f0 >= p.F) return;
-  const int b = blockIdx.z, K = p.K;
-  const int t0 = blockIdx.y * CONV_TILE, t1 = min(p.S, t0 + CONV_TILE);
+  const int b = blockIdx.z;
+  const int t0 = blockIdx.x * CONV_TILE, t1 = min(p.S, t0 + CONV_TILE);
   const T* x = static_cast<const T*>(p.x) + (long long)b * p.x_sb + f0;
   T* out = static_cast<T*>(p.out) + (long long)b * p.o_sb + f0;
-  // weights by lag: wl[l] multiplies x[t-l] (tap K-1-l of the convolution's weight; zero beyond the kernel size, so that
-  // every index below is a compile-time constant and the arrays stay in registers); win[l-1] = x[t-l]
-  float wl[CONV_MAXK][V], bias[V], win[CONV_MAXK - 1][V];
+  // win[l-1] = x[t-l]; wl[l] multiplies x[t-l] (tap K-1-l of the convolution's weight)
+  Vec16<T> win[W];
 #pragma unroll
-  for (int i = 0; i < V; ++i) {
-    bias[i] = p.bias ? to_float(static_cast<const T*>(p.bias)[f0 + i]) : 0.f;
+  for (int l = 1; l < K; ++l) {
 #pragma unroll
-    for (int l = 0; l < CONV_MAXK; ++l) wl[l][i] = l < K ? to_float(static_cast<const T*>(p.weight)[(long long)(f0 + i) * K + (K - 1 - l)]) : 0.f;
+    for (int i = 0; i < V; ++i) win[l - 1].v[i] = from_float<T>(0.f);
+    if (t0 - l >= 0) win[l - 1] = load16(x + (long long)(t0 - l) * p.x_st);
+  }
+  float wl[K][V], bias[V];
+  const T *wp = static_cast<const T*>(p.weight) + (long long)f0 * K, *bp = static_cast<const T*>(p.bias) + f0;
+  if ((reinterpret_cast<uintptr_t>(wp) | (p.bias ? reinterpret_cast<uintptr_t>(bp) : 0)) % 16 == 0) {   // V rows of K taps: K whole vectors
+    Vec16<T> raw[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) raw[j] = load16(wp + j * V);
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+#pragma unroll
+      for (int l = 0; l < K; ++l) wl[l][i] = to_float(raw[(i * K + K - 1 - l) / V].v[(i * K + K - 1 - l) % V]);
+    Vec16<T> rb;
+    if (p.bias) rb = load16(bp);
+#pragma unroll
+    for (int i = 0; i < V; ++i) bias[i] = p.bias ? to_float(rb.v[i]) : 0.f;
+  } else {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      bias[i] = p.bias ? to_float(bp[i]) : 0.f;
+#pragma unroll
+      for (int l = 0; l < K; ++l) wl[l][i] = to_float(wp[i * K + (K - 1 - l)]);
+    }
   }
   // tokens since the first token of the document that holds (b, t0); the next boundary on the flattened axis
   long long since = t0, next_b = 0x7fffffffffffffffLL;
@@ -310,42 +349,46 @@ __global__ void __launch_bounds__(CONV_THREADS) causal_conv1d_kernel(const xl_co
     if (since > t0) since = t0;   // a row start is a start whatever the offsets say
     next_b = idx + 1 <= p.num_docs ? (long long)p.cu_seqlens[idx + 1] : next_b;
   }
-#pragma unroll
-  for (int l = 1; l < CONV_MAXK; ++l) {
-    const int t = t0 - l;
-    Vec16<T> v;
-#pragma unroll
-    for (int i = 0; i < V; ++i) v.v[i] = from_float<T>(0.f);
-    if (l < K && t >= 0) v = load16(x + (long long)t * p.x_st);
-#pragma unroll
-    for (int i = 0; i < V; ++i) win[l - 1][i] = to_float(v.v[i]);
-  }
-  for (int t = t0; t < t1; ++t) {
-    const long long flat = (long long)b * p.S + t;
-    while (flat >= next_b) {   // a document starts here (empty documents are stepped over)
-      since = flat - next_b;
-      ++idx;
-      next_b = idx + 1 <= p.num_docs ? (long long)p.cu_seqlens[idx + 1] : 0x7fffffffffffffffLL;
-    }
-    const Vec16<T> cur = load16(x + (long long)t * p.x_st);
+  // one token; `reach`: tokens of its document in front of it (K and more: every tap is inside)
+  auto token = [&](const Vec16<T>& cur, int t, long long reach) {
     Vec16<T> o;
 #pragma unroll
     for (int i = 0; i < V; ++i) {
-      const float c = to_float(cur.v[i]);
-      float acc = bias[i];
-      acc = fmaf(wl[0][i], c, acc);
+      float acc = fmaf(wl[0][i], to_float(cur.v[i]), bias[i]);
 #pragma unroll
-      for (int l = 1; l < CONV_MAXK; ++l)
-        if (l <= since) acc = fmaf(wl[l][i], win[l - 1][i], acc);
+      for (int l = 1; l < K; ++l)
+        if (l <= reach) acc = fmaf(wl[l][i], to_float(win[l - 1].v[i]), acc);
       float y = to_float(from_float<T>(acc));            // the convolution's output is rounded to T ...
       if (p.act) y = y * sigmoid_for<T>(y);               // ... before the activation
       o.v[i] = from_float<T>(y);
-#pragma unroll
-      for (int l = CONV_MAXK - 1; l >= 2; --l) win[l - 1][i] = win[l - 2][i];
-      win[0][i] = c;
     }
+#pragma unroll
+    for (int l = K - 1; l >= 2; --l) win[l - 1] = win[l - 2];
+    if constexpr (K > 1) win[0] = cur;
     store16(out + (long long)t * p.o_st, o);
-    ++since;
+  };
+  for (int tg = t0; tg < t1; tg += CONV_GROUP) {
+    const long long flat = (long long)b * p.S + tg;
+    Vec16<T> cur[CONV_GROUP];
+#pragma unroll
+    for (int j = 0; j < CONV_GROUP; ++j) cur[j] = load16(x + (long long)min(tg + j, t1 - 1) * p.x_st);
+    if (tg + CONV_GROUP <= t1 && since >= K - 1 && flat + CONV_GROUP <= next_b) {   // inside one document, whole group
+#pragma unroll
+      for (int j = 0; j < CONV_GROUP; ++j) token(cur[j], tg + j, K);
+      since += CONV_GROUP;
+    } else {
+#pragma unroll
+      for (int j = 0; j < CONV_GROUP; ++j) {
+        if (tg + j >= t1) break;
+        while (flat + j >= next_b) {   // a document starts here (empty documents are stepped over)
+          since = flat + j - next_b;
+          ++idx;
+          next_b = idx + 1 <= p.num_docs ? (long long)p.cu_seqlens[idx + 1] : 0x7fffffffffffffffLL;
+        }
+        token(cur[j], tg + j, since);
+        ++since;
+      }
+    }
   }
 }
 
@@ -392,18 +435,28 @@ extern "C" int xl_headnorm_gate(const xl_headnorm_gate_params* p, void* cuda_str
   if (p->out == p->h || p->out == p->o) return XL_ERR_ALIASING;
   const long long per_row = (long long)p->S * p->NH;
   if (per_row > 0x7fffffffLL || p->B > 65535) return XL_ERR_TOO_LARGE;
-  const dim3 blocks((unsigned)((per_row + HNG_WARPS - 1) / HNG_WARPS), (unsigned)p->B);
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   const int nc = (p->DH + 32 * V - 1) / (32 * V);
-#define XL_HNG_LAUNCH(T)                                                                              \
-  do {                                                                                                \
-    if (nc <= 1) headnorm_gate_kernel<T, 1><<<blocks, HNG_WARPS * 32, 0, st>>>(*p);         \
-    else if (nc <= 2) headnorm_gate_kernel<T, 2><<<blocks, HNG_WARPS * 32, 0, st>>>(*p);    \
-    else headnorm_gate_kernel<T, 4><<<blocks, HNG_WARPS * 32, 0, st>>>(*p);                 \
+  const bool many = per_row * p->B >= HNG_FULL;
+#define XL_HNG_ROWS(T, NC, R)                                                                                                              \
+  headnorm_gate_kernel<T, NC, (R)><<<dim3((unsigned)(((p->S + (R) - 1) / (R) * (long long)p->NH + HNG_WARPS - 1) / HNG_WARPS), (unsigned)p->B), \
+                                     HNG_WARPS * 32, 0, st>>>(*p)
+#define XL_HNG_LAUNCH(T, NC)                                      \
+  do {                                                            \
+    if (many) XL_HNG_ROWS(T, NC, HNG_IN_FLIGHT / NC);             \
+    else XL_HNG_ROWS(T, NC, 1);                                   \
   } while (0)
-  if (p->dtype == XL_F32) XL_HNG_LAUNCH(float);
-  else XL_HNG_LAUNCH(__nv_bfloat16);
+#define XL_HNG_TYPE(T)                        \
+  do {                                        \
+    if (nc <= 1) XL_HNG_LAUNCH(T, 1);         \
+    else if (nc <= 2) XL_HNG_LAUNCH(T, 2);    \
+    else XL_HNG_ROWS(T, 4, 1);                \
+  } while (0)
+  if (p->dtype == XL_F32) XL_HNG_TYPE(float);
+  else XL_HNG_TYPE(__nv_bfloat16);
+#undef XL_HNG_TYPE
 #undef XL_HNG_LAUNCH
+#undef XL_HNG_ROWS
   return check_launch("xl_headnorm_gate");
 }
 
@@ -459,10 +512,18 @@ extern "C" int xl_causal_conv1d(const xl_conv1d_params* p, void* cuda_stream) {
   if (p->x_sb % V || p->x_st % V || p->o_sb % V || p->o_st % V || p->x_st < p->F || p->o_st < p->F) return XL_ERR_BAD_STRIDE;
   if (!aligned16(p->x) || !aligned16(p->out)) return XL_ERR_BAD_ALIGNMENT;
   if (p->out == p->x) return XL_ERR_ALIASING;   // a tile's halo is read by the neighbouring thread block
-  const dim3 grid((unsigned)((p->F / V + CONV_THREADS - 1) / CONV_THREADS), (unsigned)((p->S + CONV_TILE - 1) / CONV_TILE), (unsigned)p->B);
+  const dim3 grid((unsigned)((p->S + CONV_TILE - 1) / CONV_TILE), (unsigned)((p->F / V + CONV_THREADS - 1) / CONV_THREADS), (unsigned)p->B);
   if (grid.y > 65535) return XL_ERR_TOO_LARGE;
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
-  if (p->dtype == XL_F32) causal_conv1d_kernel<float><<<grid, CONV_THREADS, 0, st>>>(*p);
-  else causal_conv1d_kernel<__nv_bfloat16><<<grid, CONV_THREADS, 0, st>>>(*p);
+#define XL_CONV_LAUNCH(KK)                                                                             \
+  case KK:                                                                                             \
+    if (p->dtype == XL_F32) causal_conv1d_kernel<float, KK><<<grid, CONV_THREADS, 0, st>>>(*p);        \
+    else causal_conv1d_kernel<__nv_bfloat16, KK><<<grid, CONV_THREADS, 0, st>>>(*p);                   \
+    break
+  switch (p->K) {
+    XL_CONV_LAUNCH(1); XL_CONV_LAUNCH(2); XL_CONV_LAUNCH(3); XL_CONV_LAUNCH(4);
+    XL_CONV_LAUNCH(5); XL_CONV_LAUNCH(6); XL_CONV_LAUNCH(7); XL_CONV_LAUNCH(8);
+  }
+#undef XL_CONV_LAUNCH
   return check_launch("xl_causal_conv1d");
 }

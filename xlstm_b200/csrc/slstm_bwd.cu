@@ -425,16 +425,16 @@ __global__ void __launch_bounds__(SLB_THREADS, 1) slstm_backward_rows8_kernel(co
   float pa, pb, pig, pzt, pfg, pff, pcp, pnp, pz2, po2;
   auto pick = [&](uint32_t w) { return half ? __uint_as_float(w & 0xffff0000u) : __uint_as_float(w << 16); };   // this thread's row of a pair
   auto precompute = [&](int t) {
-    const unsigned char* rt = s_rec + (t % SL_RING) * SL8_REC_STEP + ftid * SL8_REC_BYTES;
+    const unsigned char* rt = s_rec + (t % SL_RING) * SL8_REC_STEP + ftid * 16;
     const uint4 gw = *reinterpret_cast<const uint4*>(rt);
-    const float yn = pick(*reinterpret_cast<const uint32_t*>(rt + 16));
-    const float nn = *reinterpret_cast<const float*>(rt + 32 + 4 * half), mn = *reinterpret_cast<const float*>(rt + 40 + 4 * half);
+    const float yn = pick(*reinterpret_cast<const uint32_t*>(rt + SL8_REC_PLANE));
+    const float nn = *reinterpret_cast<const float*>(rt + 2 * SL8_REC_PLANE + 4 * half), mn = *reinterpret_cast<const float*>(rt + 2 * SL8_REC_PLANE + 8 + 4 * half);
     float cp, np, mp;
     if (t > 0) {
-      const unsigned char* rp = s_rec + ((t - 1) % SL_RING) * SL8_REC_STEP + ftid * SL8_REC_BYTES;
-      cp = *reinterpret_cast<const float*>(rp + 24 + 4 * half);
-      np = *reinterpret_cast<const float*>(rp + 32 + 4 * half);
-      mp = *reinterpret_cast<const float*>(rp + 40 + 4 * half);
+      const unsigned char* rp = s_rec + ((t - 1) % SL_RING) * SL8_REC_STEP + ftid * 16;
+      cp = *reinterpret_cast<const float*>(rp + SL8_REC_PLANE + 8 + 4 * half);
+      np = *reinterpret_cast<const float*>(rp + 2 * SL8_REC_PLANE + 4 * half);
+      mp = *reinterpret_cast<const float*>(rp + 2 * SL8_REC_PLANE + 8 + 4 * half);
     } else {
       const bool have = p.state0 != nullptr && ok_r;
       cp = have ? p.state0[1 * (size_t)B * H + st_off] : 0.f;

@@ -17,11 +17,12 @@ constexpr int SL_WX_STEP_BYTES = SL_ROWS * SL_WX_ROW_BYTES;
 constexpr int SL_REC_BYTES = 96;
 
 // The eight-row kernels (the batch rows are the N = 8 side of the products, see slstm_fwd.cu): one cluster per (head, 8
-// batch rows).  A thread owns one unit and two adjacent rows; its record is 48 bytes: i', raw f, tanh z, sigmoid o and h' as
-// bf16 pairs over the rows, 4 B pad, then c', n', m' in fp32, two each.
+// batch rows).  A thread owns one unit and two adjacent rows; its record is 48 bytes in three planes of 16 bytes per thread,
+// so that a warp stores and loads each of them as 512 contiguous bytes: i', raw f, tanh z, sigmoid o as bf16 pairs over the
+// rows | h' as such a pair, 4 B pad, c' | n', m' (fp32, two each).
 constexpr int SL8_ROWS = 8;
-constexpr int SL8_REC_BYTES = 48;
-constexpr int SL8_REC_STEP = SL_THREADS * SL8_REC_BYTES;
+constexpr int SL8_REC_PLANE = SL_THREADS * 16;
+constexpr int SL8_REC_STEP = 3 * SL8_REC_PLANE;
 
 // Whether a batch of B rows runs on the eight-row kernels: where all their clusters are resident at once.  Eight rows take
 // half the products, half the gate arithmetic and half the exchange of a sixteen-row step, on twice the SMs; with more

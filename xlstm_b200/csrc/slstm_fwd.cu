@@ -378,8 +378,7 @@ struct Sl8Layout {
   static constexpr int WX_STEP = SL8_ROWS * 4 * SL_UNITS * 2;
   static constexpr int OFF_WX = 2 * H_TILE;
   static constexpr int OFF_BAR = OFF_WX + SL_RING * WX_STEP;            // 2 mbarriers: h tile 0 / 1 complete
-  static constexpr int OFF_REC = OFF_BAR + 16;                          // TRAIN: staging of the records
-  static constexpr int OFF_R = OFF_REC + (TRAIN ? SL_REC_SLOTS * SL8_REC_STEP : 0);
+  static constexpr int OFF_R = OFF_BAR + 16;
   static constexpr int TOTAL = OFF_R + DH * 4 * SL_UNITS * 2;
 };
 
@@ -487,7 +486,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) slstm_forward_rows8_kernel(cons
                                                ((size_t)(orow < B ? orow : 0) * NH + head) * (size_t)S * DH + rank * SL_UNITS + warp * 8 + 2 * (lane & 3));
   unsigned char* rec = nullptr;
   if constexpr (TRAIN)
-    rec = reinterpret_cast<unsigned char*>(p.train_cache) + (((size_t)bgroup * NH + head) * NCTA + rank) * (size_t)S * SL8_REC_STEP;
+    rec = reinterpret_cast<unsigned char*>(p.train_cache) + (((size_t)bgroup * NH + head) * NCTA + rank) * (size_t)S * SL8_REC_STEP + tid * 16;
 
   bool ok = true;
   for (int t = 0; t < S; ++t) {
@@ -567,11 +566,12 @@ __global__ void __launch_bounds__(SL_THREADS, 1) slstm_forward_rows8_kernel(cons
       }
     }
     if constexpr (TRAIN) {
-      uint4* r = reinterpret_cast<uint4*>(sl_smem + LY::OFF_REC + (t % SL_REC_SLOTS) * SL8_REC_STEP + tid * SL8_REC_BYTES);
-      r[0] = make_uint4(pack_bf16x2(gi[0], gi[1]), pack_bf16x2(gf[0], gf[1]), pack_bf16x2(gz[0], gz[1]), pack_bf16x2(go[0], go[1]));
-      r[1] = make_uint4(hp, 0u, __float_as_uint(c_[0]), __float_as_uint(c_[1]));
-      r[2] = make_uint4(__float_as_uint(n_[0]), __float_as_uint(n_[1]), __float_as_uint(m_[0]), __float_as_uint(m_[1]));
-      fence_proxy_async_smem();
+      // straight to global memory, a plane at a time: staged in shared memory and sent as one bulk copy, the records cost a
+      // proxy fence on every step's chain (1.47 -> 1.38 ms at B = 16, S = 2048, 4 x 256)
+      uint4* r = reinterpret_cast<uint4*>(rec + (size_t)t * SL8_REC_STEP);
+      __stcs(r, make_uint4(pack_bf16x2(gi[0], gi[1]), pack_bf16x2(gf[0], gf[1]), pack_bf16x2(gz[0], gz[1]), pack_bf16x2(go[0], go[1])));
+      __stcs(r + SL_THREADS, make_uint4(hp, 0u, __float_as_uint(c_[0]), __float_as_uint(c_[1])));
+      __stcs(r + 2 * SL_THREADS, make_uint4(__float_as_uint(n_[0]), __float_as_uint(n_[1]), __float_as_uint(m_[0]), __float_as_uint(m_[1])));
     }
     // output h_t, (B, NH, S, DH) -- after the pushes: they are on the step-to-step chain, this store is not
     {
@@ -583,16 +583,6 @@ __global__ void __launch_bounds__(SL_THREADS, 1) slstm_forward_rows8_kernel(cons
     cp_async_wait<SL_RING - 2>();  // this thread's part of step t+1 has landed
     // ... and everybody else's (CTA-wide only); the same barrier tells every thread whether any wait expired
     if (__syncthreads_or(ok ? 0 : 1)) { ok = false; break; }
-    if constexpr (TRAIN) {
-      if (tid == 0) {
-        bulk_store(rec + (size_t)t * SL8_REC_STEP, s_h + LY::OFF_REC + (t % SL_REC_SLOTS) * SL8_REC_STEP, SL8_REC_STEP);
-        bulk_commit();
-        bulk_wait_read<1>();   // the copy of step t-1 has read its slot: step t+2, which reuses it, may stage (behind the next barrier)
-      }
-    }
-  }
-  if constexpr (TRAIN) {
-    if (tid == 0) bulk_wait<0>();
   }
   // the pushes of h_{S-1} are waited for before anybody may leave (see the sixteen-row kernel)
   if (ok) {

@@ -221,6 +221,23 @@ int xl_slstm_weight_grads(const xl_slstm_wgrad_params* p, void* cuda_stream);
 int64_t xl_slstm_weight_grads_scratch_bytes(int32_t B, int32_t S, int32_t NH, int32_t DH);
 
 /* ------------------------------------------------------------------------------------------------
+ * y = x W^T for up to 16 rows of x (decoding), bf16 with fp32 accumulation: the linear layers around the decode cell
+ * (xlstm/xlstm_large/model.py:379-452, 268-277) as streams of W.  W is read ahead of the kernel launched directly in front on
+ * the stream: that kernel must not be the one that writes W.
+ * ---------------------------------------------------------------------------------------------- */
+typedef struct xl_rows_linear_params {
+  const void* x;         /* (rows, K), contiguous rows x_sr elements apart (a multiple of 8), 16-byte aligned */
+  const void* w;         /* (N, K), contiguous rows w_sr elements apart (a multiple of 8), 16-byte aligned */
+  void* y;               /* out (rows, N), contiguous */
+  int32_t* status;
+  int64_t x_sr, w_sr;
+  int32_t rows, N, K;
+  int32_t dtype;
+} xl_rows_linear_params;
+
+int xl_rows_linear(const xl_rows_linear_params* p, void* cuda_stream);
+
+/* ------------------------------------------------------------------------------------------------
  * Operators next to the mLSTM cell in the reference's layer (xlstm/xlstm_large/model.py:379-452), each one pass
  * over its data.  Rounding follows the reference's eager sequence: reductions in fp32, the normalised value is
  * rounded to `dtype`, multiplied by the weight and rounded again (components.py:58-63, 86-97, 171-185); the gate is rounded after

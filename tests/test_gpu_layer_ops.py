@@ -283,3 +283,24 @@ def test_causal_conv1d_tile_edges_and_unaligned_weights(K, S):
             off = torch.empty(F_ * K + 1, dtype=dt, device="cuda")[1:].view(F_, K)   # starts 2 or 4 bytes past a 16-byte boundary
             off.copy_(w)
             assert torch.equal(xlstm_b200.causal_conv1d(x.cuda(), off, b.cuda(), cu_seqlens=c), got)
+
+
+@pytest.mark.parametrize("rows,N,K", [(1, 1, 8), (1, 128, 64), (8, 129, 72), (16, 2048, 4096), (15, 127, 640), (9, 12304, 2048), (3, 300, 10944),
+                                      (16, 21888, 512), (8, 50304, 192), (5, 4096, 128)])
+def test_rows_linear_matches_64_bits(rows, N, K):
+    """Remainders of every tile (features, contraction, rows), one to eight blocks per tile.  Products of bf16 values are
+    exact in fp32, so the error is the rounding of the output to bf16 (eight significant bits: half a unit is at most 2^-8
+    of the value), plus fp32 sums."""
+    import xlstm_b200
+    from xlstm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x = torch.randn(rows, K + 8, generator=g, device="cuda").bfloat16()[:, :K]          # rows K + 8 apart
+    w = torch.randn(N, K, generator=g, device="cuda").bfloat16() / K ** 0.5
+    torch.cuda.synchronize()   # (w is complete before the kernel that reads it ahead is launched)
+    want = x.double() @ w.double().T
+    got = ops.rows_linear(x, w)
+    xlstm_b200.check_device_status()
+    assert got.shape == (rows, N) and got.dtype == torch.bfloat16
+    assert float((got.double() - want).norm()) <= (2 ** -8 + 1e-5) * float(want.norm())
+    assert torch.equal(ops.rows_linear(x, w), got)
+    assert torch.equal(ops.rows_linear(x.contiguous().view(rows, 1, K), w), got.view(rows, 1, N))

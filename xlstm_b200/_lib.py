@@ -21,7 +21,7 @@ EXPORTS = (
     "xl_add_rmsnorm", "xl_headnorm_gate", "xl_soft_cap", "xl_causal_conv1d",
     "xl_softcap_argmax", "xl_softcap_argmax_scratch_bytes", "xl_swiglu",
     "xl_softcap_argmax_noalloc", "xl_softcap_argmax_noalloc_max_rows", "xl_peer_reduce_add_rmsnorm", "xl_headwise_proj", "xl_mlstm_decode_cell",
-    "xl_slstm_backward", "xl_slstm_cache_bytes", "xl_slstm_weight_grads", "xl_slstm_weight_grads_scratch_bytes",
+    "xl_slstm_backward", "xl_slstm_cache_bytes", "xl_slstm_weight_grads", "xl_slstm_weight_grads_scratch_bytes", "xl_rows_linear",
 )
 
 
@@ -138,6 +138,13 @@ class HeadwiseParams(C.Structure):
     ]
 
 
+class RowsLinearParams(C.Structure):
+    _fields_ = [
+        ("x", C.c_void_p), ("w", C.c_void_p), ("y", C.c_void_p), ("status", C.c_void_p), ("x_sr", C.c_int64), ("w_sr", C.c_int64),
+        ("rows", C.c_int32), ("N", C.c_int32), ("K", C.c_int32), ("dtype", C.c_int32),
+    ]
+
+
 class GreedyParams(C.Structure):
     _fields_ = [
         ("logits", C.c_void_p), ("tokens", C.c_void_p), ("scratch", C.c_void_p), ("scratch_bytes", C.c_int64),
@@ -195,7 +202,8 @@ def lib() -> C.CDLL:
                             ("xl_soft_cap", SoftCapParams), ("xl_causal_conv1d", Conv1dParams),
                             ("xl_softcap_argmax", GreedyParams), ("xl_swiglu", SwigluParams),
                             ("xl_softcap_argmax_noalloc", GreedyParams), ("xl_peer_reduce_add_rmsnorm", PeerReduceParams),
-                            ("xl_slstm_backward", SlstmBwdParams), ("xl_slstm_weight_grads", SlstmWgradParams)):
+                            ("xl_slstm_backward", SlstmBwdParams), ("xl_slstm_weight_grads", SlstmWgradParams),
+                            ("xl_rows_linear", RowsLinearParams)):
             fn = getattr(l, name)
             fn.restype = C.c_int
             fn.argtypes = [C.POINTER(ptype), C.c_void_p]

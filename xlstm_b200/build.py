@@ -25,7 +25,7 @@ OBJ = os.path.join(HERE, "..", "build")
 HEADER = os.path.join(HERE, "..", "include", "xlstm_b200.h")
 LIB = os.path.join(HERE, "libxlstm_b200.so")
 NATIVE = os.path.join(HERE, "_native.so")
-SOURCES = ["capi.cu", "mlstm_step.cu", "mlstm_recurrent.cu", "mlstm_chunkwise.cu", "mlstm_parts.cu", "slstm_fwd.cu", "slstm_bwd.cu", "slstm_wgrad.cu", "layer_adjacent.cu", "greedy_head.cu", "peer_reduce.cu", "headwise_proj.cu"]
+SOURCES = ["capi.cu", "mlstm_step.cu", "mlstm_recurrent.cu", "mlstm_chunkwise.cu", "mlstm_parts.cu", "slstm_fwd.cu", "slstm_bwd.cu", "slstm_wgrad.cu", "layer_adjacent.cu", "greedy_head.cu", "peer_reduce.cu", "headwise_proj.cu", "rows_linear.cu"]
 BINDING = "binding.cpp"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]

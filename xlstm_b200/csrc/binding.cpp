@@ -430,6 +430,29 @@ PyObject* add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   END_HANDLE_TH_ERRORS
 }
 
+// (x (..., K), w (N, K)) -> (..., N), bf16, at most 16 rows of x
+PyObject* rows_linear(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  want_args(na, 2);
+  const Tensor &x = tensor_arg(a[0], "x"), &w0 = tensor_arg(a[1], "w");
+  for (const Tensor* t : {&x, &w0}) require_cuda(t);
+  TORCH_CHECK_VALUE(x.scalar_type() == at::kBFloat16 && w0.scalar_type() == at::kBFloat16 && w0.dim() == 2 && x.dim() >= 1 && x.size(-1) == w0.size(1),
+                    "rows_linear: bfloat16 x (..., K) and w (N, K)");
+  const int64_t K = x.size(-1), N = w0.size(0);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const Tensor x2 = as_rows(x, K), w = last_contig(w0);
+  c10::SmallVector<int64_t, 5> sizes(x.sizes().begin(), x.sizes().end());
+  sizes.back() = N;
+  const Tensor y = empty_on(sizes, at::kBFloat16, x);
+  xl_rows_linear_params p = {};
+  p.x = x2.data_ptr(); p.w = w.data_ptr(); p.y = y.data_ptr(); p.status = status_ptr(x);
+  p.x_sr = x2.size(0) > 1 ? x2.stride(0) : K; p.w_sr = N > 1 ? w.stride(0) : K;
+  p.rows = (int32_t)x2.size(0); p.N = (int32_t)N; p.K = (int32_t)K; p.dtype = XL_BF16;
+  check(xl_rows_linear(&p, stream_of(x)), "xl_rows_linear");
+  return THPVariable_Wrap(y);
+  END_HANDLE_TH_ERRORS
+}
+
 // (h, o_preact or None, weight, eps) -> (B, S, NH*DH)
 PyObject* headnorm_gate(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
@@ -682,7 +705,7 @@ PyObject* status_word(PyObject*, PyObject* index) {
 
 #define XL_FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
-    XL_FAST(mlstm_sequence), XL_FAST(mlstm_step), XL_FAST(mlstm_decode_cell), XL_FAST(slstm_forward), XL_FAST(slstm_backward), XL_FAST(slstm_weight_grads),
+    XL_FAST(mlstm_sequence), XL_FAST(mlstm_step), XL_FAST(mlstm_decode_cell), XL_FAST(slstm_forward), XL_FAST(slstm_backward), XL_FAST(slstm_weight_grads), XL_FAST(rows_linear),
     XL_FAST(add_rmsnorm), XL_FAST(headnorm_gate), XL_FAST(soft_cap), XL_FAST(causal_conv1d), XL_FAST(headwise_proj), XL_FAST(softcap_argmax),
     XL_FAST(document_offsets), XL_FAST(slot_vector),
     {"swiglu", swiglu, METH_O, nullptr}, {"status_word", status_word, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};

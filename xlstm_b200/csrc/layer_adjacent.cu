@@ -94,6 +94,8 @@ __global__ void __launch_bounds__(RMS_THREADS) add_rmsnorm_kernel(const xl_add_r
   __shared__ float s_part[RMS_THREADS / 32];
   const long long row = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  grid_dependency_wait();
+  grid_dependents_launch();
   const T* x = static_cast<const T*>(p.x) + row * p.x_sr;
   const T* y = p.y ? static_cast<const T*>(p.y) + row * p.y_sr : nullptr;
   const T* w = static_cast<const T*>(p.weight);
@@ -237,6 +239,8 @@ template <typename T, typename O, bool ROUND_EACH>
 __global__ void __launch_bounds__(256) soft_cap_kernel(const T* __restrict__ x, O* __restrict__ out, long long n, float cap,
                                                        long long cols, long long x_row_stride, const T* __restrict__ bias) {
   const long long stride = (long long)gridDim.x * blockDim.x;
+  grid_dependency_wait();
+  grid_dependents_launch();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     // (rows of `cols` elements `x_row_stride` apart: a column slice of a wider projection output; a bias per column is
     // added first, rounded to T as the reference's Linear rounds its output)
@@ -268,6 +272,8 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const T* __restrict__ gz, T
                                                      long long gz_row_stride) {
   constexpr int V = Vec16<T>::N;
   const long long nvec = rows * (long long)(F / V), stride = (long long)gridDim.x * blockDim.x;
+  grid_dependency_wait();
+  grid_dependents_launch();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += stride) {
     const long long r = i / (F / V);
     const int c = (int)(i - r * (F / V)) * V;
@@ -410,12 +416,12 @@ extern "C" int xl_add_rmsnorm(const xl_add_rmsnorm_params* p, void* cuda_stream)
   if (p->rows == 0) return XL_OK;
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   const int nc = (p->D + RMS_THREADS * V - 1) / (RMS_THREADS * V);
-  const unsigned grid = (unsigned)p->rows;
+  const dim3 grid((unsigned)p->rows);
 #define XL_RMS_LAUNCH(T)                                                              \
   do {                                                                                \
-    if (nc <= 1) add_rmsnorm_kernel<T, 1><<<grid, RMS_THREADS, 0, st>>>(*p);          \
-    else if (nc <= 2) add_rmsnorm_kernel<T, 2><<<grid, RMS_THREADS, 0, st>>>(*p);     \
-    else add_rmsnorm_kernel<T, 4><<<grid, RMS_THREADS, 0, st>>>(*p);                  \
+    if (nc <= 1) (void)launch_dependent(add_rmsnorm_kernel<T, 1>, grid, dim3(RMS_THREADS), 0, st, *p);          \
+    else if (nc <= 2) (void)launch_dependent(add_rmsnorm_kernel<T, 2>, grid, dim3(RMS_THREADS), 0, st, *p);     \
+    else (void)launch_dependent(add_rmsnorm_kernel<T, 4>, grid, dim3(RMS_THREADS), 0, st, *p);                  \
   } while (0)
   if (p->dtype == XL_F32) XL_RMS_LAUNCH(float);
   else XL_RMS_LAUNCH(__nv_bfloat16);
@@ -474,13 +480,13 @@ extern "C" int xl_soft_cap(const xl_soft_cap_params* p, void* cuda_stream) {
   const unsigned grid = (unsigned)(want < 148 * 16 ? want : 148 * 16);
   const long long cols = p->cols, rs = p->x_row_stride;
   if (p->dtype == XL_F32)
-    soft_cap_kernel<float, float, false><<<grid, 256, 0, st>>>(static_cast<const float*>(p->x), static_cast<float*>(p->out), p->n, p->cap, cols, rs, static_cast<const float*>(p->bias));
+    (void)launch_dependent(soft_cap_kernel<float, float, false>, dim3(grid), dim3(256), 0, st, static_cast<const float*>(p->x), static_cast<float*>(p->out), p->n, p->cap, cols, rs, static_cast<const float*>(p->bias));
   else if (p->out_f32 == 2)
-    soft_cap_kernel<__nv_bfloat16, float, false><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(p->x), static_cast<float*>(p->out), p->n, p->cap, cols, rs, static_cast<const __nv_bfloat16*>(p->bias));
+    (void)launch_dependent(soft_cap_kernel<__nv_bfloat16, float, false>, dim3(grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(p->x), static_cast<float*>(p->out), p->n, p->cap, cols, rs, static_cast<const __nv_bfloat16*>(p->bias));
   else if (p->out_f32)
-    soft_cap_kernel<__nv_bfloat16, float, true><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(p->x), static_cast<float*>(p->out), p->n, p->cap, cols, rs, static_cast<const __nv_bfloat16*>(p->bias));
+    (void)launch_dependent(soft_cap_kernel<__nv_bfloat16, float, true>, dim3(grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(p->x), static_cast<float*>(p->out), p->n, p->cap, cols, rs, static_cast<const __nv_bfloat16*>(p->bias));
   else
-    soft_cap_kernel<__nv_bfloat16, __nv_bfloat16, true><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(p->x), static_cast<__nv_bfloat16*>(p->out), p->n, p->cap, cols, rs, static_cast<const __nv_bfloat16*>(p->bias));
+    (void)launch_dependent(soft_cap_kernel<__nv_bfloat16, __nv_bfloat16, true>, dim3(grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(p->x), static_cast<__nv_bfloat16*>(p->out), p->n, p->cap, cols, rs, static_cast<const __nv_bfloat16*>(p->bias));
   return check_launch("xl_soft_cap");
 }
 
@@ -496,8 +502,8 @@ extern "C" int xl_swiglu(const xl_swiglu_params* p, void* cuda_stream) {
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   const long long want = (p->rows * (long long)(p->F / V) + 255) / 256;
   const unsigned grid = (unsigned)(want < 148 * 16 ? want : 148 * 16);
-  if (p->dtype == XL_F32) swiglu_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(p->gz), static_cast<float*>(p->out), p->rows, p->F, p->gz_row_stride);
-  else swiglu_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(p->gz), static_cast<__nv_bfloat16*>(p->out), p->rows, p->F, p->gz_row_stride);
+  if (p->dtype == XL_F32) (void)launch_dependent(swiglu_kernel<float>, dim3(grid), dim3(256), 0, st, static_cast<const float*>(p->gz), static_cast<float*>(p->out), p->rows, p->F, p->gz_row_stride);
+  else (void)launch_dependent(swiglu_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, st, static_cast<const __nv_bfloat16*>(p->gz), static_cast<__nv_bfloat16*>(p->out), p->rows, p->F, p->gz_row_stride);
   return check_launch("xl_swiglu");
 }
 

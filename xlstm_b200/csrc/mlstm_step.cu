@@ -49,6 +49,8 @@ __global__ void __launch_bounds__(STEP_THREADS) mlstm_step_kernel(const xl_mlstm
   const int b = blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * STEP_COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int DHQK = p.DHQK, DHV = p.DHV;
+  grid_dependency_wait();
+  grid_dependents_launch();
   const int64_t row = p.slot ? (int64_t)p.slot[b] : (int64_t)b;
   if (p.slot && (row < 0 || row >= p.n_slots)) {
     // a negative slot marks an inactive stream: nothing of the pool is touched, h is zero.  A slot beyond the pool is
@@ -228,9 +230,9 @@ extern "C" int xl_mlstm_step(const xl_mlstm_step_params* p, void* cuda_stream) {
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   const StepFused none = {};
   if (p->dtype == XL_F32)
-    mlstm_step_kernel<float, false><<<grid, block, smem, st>>>(*p, none);
+    (void)launch_dependent(mlstm_step_kernel<float, false>, grid, block, smem, st, *p, none);
   else
-    mlstm_step_kernel<__nv_bfloat16, false><<<grid, block, smem, st>>>(*p, none);
+    (void)launch_dependent(mlstm_step_kernel<__nv_bfloat16, false>, grid, block, smem, st, *p, none);
   return check_launch("xl_mlstm_step");
 }
 
@@ -253,10 +255,12 @@ extern "C" int xl_mlstm_decode_cell(const xl_mlstm_decode_cell_params* f, void* 
   fx.gate_cap = f->gate_cap; fx.norm_eps = f->norm_eps;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = static_cast<cudaStream_t>(cuda_stream);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = nblk; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
   if (p->dtype == XL_F32) (void)cudaLaunchKernelEx(&cfg, mlstm_step_kernel<float, true>, *p, fx);
   else (void)cudaLaunchKernelEx(&cfg, mlstm_step_kernel<__nv_bfloat16, true>, *p, fx);
   return check_launch("xl_mlstm_decode_cell");

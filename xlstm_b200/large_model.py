@@ -181,11 +181,23 @@ class LargeModel:
             torch.distributed.all_reduce(x, group=self.group)
         return x
 
+    def _linear(self, x, w):
+        """``F.linear(x, w)``.  A few rows (decoding, a last position, a very short prompt) take the weight-streaming kernel where
+        it is the faster one (measured: csrc/rows_linear.cu): weights of at least 4 MB with up to 32 tiles of 128 features,
+        which it splits further, or at least 256.  It reads `w` ahead of the kernel launched in front of it, which here is
+        always a norm, the cell or an activation."""
+        N, K = w.shape
+        if (self.fused and self.dtype == torch.bfloat16 and 0 < x.numel() <= ops.ROWS_LINEAR_MAX * K and N * K >= 1 << 21
+                and (N <= 4096 or N >= 32768) and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0
+                and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))):
+            return ops.rows_linear(x, w)
+        return F.linear(x, w)
+
     def _mlstm_layer(self, blk, x, state, cu_seqlens, slot, reduce: bool = True):
         cfg, NHl, dq, dv = self.cfg, self.nh_local, self.dq, self.dv
         B, S, _ = x.shape
         if self.fused:   # one GEMM for all six projections; the gates are capped in fp32 (they enter exponentials in the cell)
-            allp = F.linear(x, blk["qkvo_if"])
+            allp = self._linear(x, blk["qkvo_if"])
             q, k, v, o, gpre, _ = torch.split(allp, [NHl * dq, NHl * dq, NHl * dv, NHl * dv, 2 * NHl, self.gate_pad], dim=-1)
             if S == 1 and cu_seqlens is None and self.cell is ops and dv <= 1024:
                 # decode: gate cap, cell step, per-head norm and output gate in one kernel
@@ -193,7 +205,7 @@ class LargeModel:
                 hg, new_state = ops.mlstm_decode_cell(q.reshape(B, NHl, dq), k.reshape(B, NHl, dq), v.reshape(B, NHl, dv), gpre, blk["if_b"],
                                                       cfg.gate_soft_cap, o, blk["mh_norm"], c, n, m, slot=slot, eps=cfg.eps,
                                                       norm_eps=cfg.norm_eps)
-                y = F.linear(hg.reshape(B, 1, NHl * dv), blk["out_proj"])
+                y = self._linear(hg.reshape(B, 1, NHl * dv), blk["out_proj"])
                 return (self._all_reduce(y) if reduce else y), new_state
             gates = ops.soft_cap(gpre, cfg.gate_soft_cap, out_float32=True, float32_math=True, bias=blk["if_b"])
         else:
@@ -213,7 +225,7 @@ class LargeModel:
             h, new_state = self.cell.mlstm_sequence(q, k, v, ig, fg, c, n, m, cu_seqlens=cu_seqlens, eps=cfg.eps)
         if self.fused:
             hg = ops.headnorm_gate(h, o, blk["mh_norm"], eps=cfg.norm_eps)
-            y = F.linear(hg, blk["out_proj"])
+            y = self._linear(hg, blk["out_proj"])
             return (self._all_reduce(y) if reduce else y), new_state
         h = h.transpose(1, 2)                            # (B,S,NHl,dv)
         hf = h.float()
@@ -360,7 +372,7 @@ class LargeModel:
         """lm_head and soft cap; with `greedy` the argmax of the last position as well (``generate.py:13-15``), on CUDA in
         one kernel behind the GEMM."""
         cfg = self.cfg
-        logits = F.linear(xn, self.lm_head)
+        logits = self._linear(xn, self.lm_head)
         if greedy:
             if self.fused:
                 return ops.softcap_argmax(logits[:, -1], cfg.output_logit_soft_cap)[:, None]
@@ -388,7 +400,7 @@ class LargeModel:
             y, st = self._mlstm_layer(blk, xn, None if state is None else state[i], cu_seqlens, slot, reduce=False)
             new_state[i] = st
             x, xn = self._reduce_add_norm(x, y, blk["norm_ffn"])
-            pending = F.linear(self._swiglu(F.linear(xn, blk["up"])), blk["down"])
+            pending = self._linear(self._swiglu(self._linear(xn, blk["up"])), blk["down"])
         if positions is not None:
             x = x.reshape(-1, x.shape[-1])[positions][:, None]
             pending = None if pending is None else pending.reshape(-1, pending.shape[-1])[positions][:, None]

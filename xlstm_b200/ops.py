@@ -329,6 +329,16 @@ def headwise_proj(inputs, weights, in_sel=None):
     return native().headwise_proj(inputs, weights, [0] * len(weights) if in_sel is None else [int(i) for i in in_sel])
 
 
+ROWS_LINEAR_MAX = 16   # rows of x that ``rows_linear`` takes
+
+
+def rows_linear(x, w):
+    """``F.linear(x, w)`` for at most 16 rows of x (decoding): bf16 x (..., K) and w (N, K), K a multiple of 8, fp32
+    accumulation; bound by the stream of w.  The kernel launched directly in front on the stream must not be the one that
+    writes w, which is read ahead of that kernel's end."""
+    return native().rows_linear(x, w)
+
+
 def softcap_argmax(logits, cap: float):
     """Greedy tokens of un-capped logits: ``argmax(soft_cap(logits, cap), dim=-1)`` with the reference's rounding and
     tie rule (xlstm/xlstm_large/model.py:149-151, generate.py:13-15) in one kernel.  ``logits`` is (..., V) with

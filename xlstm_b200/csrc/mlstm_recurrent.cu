@@ -10,9 +10,13 @@
 //   [S | QC] = Q [K ; C^T]^T      P_jl = S_jl / sqrt(d) exp(a_l - mu_j) (l <= j)      r_j = exp(m_prev - mu_j) / sqrt(d)
 //   h_j = (r_j QC_j + sum_l P_jl v_l) / (max(|r_j q_j.n + sum_l P_jl|, exp(-(b_j + mu_j))) + eps)
 //   C <- exp(m_prev - mu_31) C + sum_l w_l k_l v_l^T,  n likewise,  w_l = exp(a_l - mu_31),  m <- b_31 + mu_31
+// The gate recurrence alone is formed in 64 bits: a_l - mu_j is a difference of sums over the chunk, and its rounding would be
+// the largest error of h.
 // Token by token the kernel was a chain of two CTA barriers and a column reduction per token, 1.6 us each; a chunk
-// is two barriers for 32 tokens, and the products run from registers at 2 x 4 outputs per thread (six 16-byte
-// shared-memory loads per 32 FMAs).  Chunks of 64 would double the redundant part of the work (S, formed by every slice).
+// is two barriers for 32 tokens, and the products run from registers at 2 x 5 outputs per thread (seven 16-byte
+// shared-memory loads per 40 FMAs).  3 x 4 heads x 256 tokens, 64 x 128: 274 us token by token, 58 in chunks, 39 with q.n and n
+// without shuffles and the head size compiled in; 1 x 8 x 203, 256 x 512: 451 -> 87 us.  h against 64 bits: 3.3e-7 (token by token
+// 3.8e-7), with the gate sums and single chains in fp32 6.5e-7.  Chunks of 64 would double the redundant part of the work (S, formed by every slice).
 #include "common.cuh"
 
 namespace xl {
@@ -28,17 +32,18 @@ __device__ __forceinline__ void rec_cp_async16(uint32_t dst, const void* src) {
 __device__ __forceinline__ void rec_cp_async4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
-  acc = fmaf(a.x, b.x, acc);
-  acc = fmaf(a.y, b.y, acc);
-  acc = fmaf(a.z, b.z, acc);
-  return fmaf(a.w, b.w, acc);
+__device__ __forceinline__ void fma4(float4& acc, const float4& a, const float4& b) {
+  acc.x = fmaf(a.x, b.x, acc.x);
+  acc.y = fmaf(a.y, b.y, acc.y);
+  acc.z = fmaf(a.z, b.z, acc.z);
+  acc.w = fmaf(a.w, b.w, acc.w);
 }
+__device__ __forceinline__ float sum4(const float4& v) { return (v.x + v.y) + (v.z + v.w); }
 
 // shared memory (floats); rows of DP = DHQK rounded up to 4, plus 4: eight rows' 16-byte pieces then lie on distinct banks
 struct RecLayout {
   int DQ4, DP, nbuf;
-  size_t q, k, vt, vw, c, pm, n, total;
+  size_t q, k, vt, vw, c, pm, n, w, total;
   __host__ __device__ explicit RecLayout(int DHQK) {
     DQ4 = (DHQK + 3) / 4;
     DP = 4 * DQ4 + 4;
@@ -50,19 +55,22 @@ struct RecLayout {
     c = vw + (size_t)REC_COLS * REC_LP;           // C^T [column][feature]
     pm = c + (size_t)REC_COLS * DP;               // P [row][token]
     n = pm + (size_t)REC_L * REC_LP;
-    total = n + (size_t)DP;
+    w = n + (size_t)DP;                           // w_l
+    total = w + REC_L;
   }
 };
 
-template <typename T>
-__global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_mlstm_seq_params p, int vec) {
+// D: DHQK where it is known at compile time (addresses and trip counts of the inner loops are constants then), 0: any
+template <typename T, int D>
+__global__ void __launch_bounds__(REC_THREADS, 1) mlstm_recurrent_kernel(const xl_mlstm_seq_params p, int vec) {
   extern __shared__ __align__(16) float smem[];
-  const RecLayout ly(p.DHQK);
-  const int DHQK = p.DHQK, DHV = p.DHV, DQ4 = ly.DQ4, DP = ly.DP;
+  const RecLayout ly(D ? D : p.DHQK);
+  const int DHQK = D ? D : p.DHQK, DHV = p.DHV, DQ4 = ly.DQ4, DP = ly.DP;
   float* s_c = smem + ly.c;
   float* s_n = smem + ly.n;
   float* s_p = smem + ly.pm;
   float* s_vw = smem + ly.vw;
+  float* s_w = smem + ly.w;
 
   const int doc = blockIdx.z, head = blockIdx.y, col0 = blockIdx.x * REC_COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -90,6 +98,7 @@ __global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_m
 
   // q, k, v of a chunk into buffer `buf`; rows past the document, features past DHQK and columns past DHV are zero.  The
   // pieces a thread loads are the same for all tiles of a shape: 16-byte copies where rows are aligned (`vec`).
+  const int r_first = tid / DQ4, d_first = tid - r_first * DQ4, r_step = REC_THREADS / DQ4, d_step = REC_THREADS - r_step * DQ4;
   auto load_chunk = [&](int chunk, int buf) {
     float* tq = smem + ly.q + (size_t)buf * REC_L * DP;
     float* tk = smem + ly.k + (size_t)buf * REC_L * DP;
@@ -97,33 +106,39 @@ __global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_m
     const int64_t t0 = (int64_t)chunk * REC_L;
     const int rows = (int)(len - t0 < REC_L ? len - t0 : REC_L);
     if (sizeof(T) == 4 && vec) {
-      for (int u = tid; u < REC_L * DQ4; u += REC_THREADS) {
-        const int r = u / DQ4, d = 4 * (u - r * DQ4);
+      const T *qc = q + t0 * p.q_st, *kc = k + t0 * p.k_st;
+      int r = r_first, d4 = d_first;
+      while (r < REC_L) {
+        const int d = 4 * d4;
         if (r < rows) {
-          rec_cp_async16(smem_u32(tq + r * DP + d), q + (t0 + r) * p.q_st + d);
-          rec_cp_async16(smem_u32(tk + r * DP + d), k + (t0 + r) * p.k_st + d);
+          rec_cp_async16(smem_u32(tq + r * DP + d), qc + r * p.q_st + d);
+          rec_cp_async16(smem_u32(tk + r * DP + d), kc + r * p.k_st + d);
         } else {
           *reinterpret_cast<float4*>(tq + r * DP + d) = make_float4(0.f, 0.f, 0.f, 0.f);
           *reinterpret_cast<float4*>(tk + r * DP + d) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
+        r += r_step;
+        d4 += d_step;
+        if (d4 >= DQ4) { d4 -= DQ4; ++r; }
       }
     } else {
-      const int D = 4 * DQ4;
+      const int W = 4 * DQ4;
 #pragma unroll 4
-      for (int u = tid; u < REC_L * D; u += REC_THREADS) {
-        const int r = u / D, d = u - r * D;
+      for (int u = tid; u < REC_L * W; u += REC_THREADS) {
+        const int r = u / W, d = u - r * W;
         const bool in = r < rows && d < DHQK;
         tq[r * DP + d] = in ? to_float(q[(t0 + r) * p.q_st + d]) : 0.f;
         tk[r * DP + d] = in ? to_float(k[(t0 + r) * p.k_st + d]) : 0.f;
       }
     }
+    const T* vc = v + (t0 + warp) * p.v_st + col0 + lane;   // a warp takes one token's columns
 #pragma unroll
-    for (int u = tid; u < REC_L * REC_COLS; u += REC_THREADS) {   // a warp takes one token's columns
-      const int r = u / REC_COLS, c = u % REC_COLS;
-      const bool in = r < rows && col0 + c < DHV;
-      const T* src = v + (t0 + r) * p.v_st + col0 + c;
-      if (sizeof(T) == 4 && in) rec_cp_async4(smem_u32(tv + c * REC_LP + r), src);
-      else tv[c * REC_LP + r] = in ? to_float(*src) : 0.f;
+    for (int i = 0; i < REC_L / 8; ++i) {
+      const int r = warp + 8 * i;
+      const bool in = r < rows && col0 + lane < DHV;
+      const T* src = vc + 8 * i * p.v_st;
+      if (sizeof(T) == 4 && in) rec_cp_async4(smem_u32(tv + lane * REC_LP + r), src);
+      else tv[lane * REC_LP + r] = in ? to_float(*src) : 0.f;
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -134,7 +149,7 @@ __global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_m
     s_c[c * DP + d] = (p.c0 && d < DHQK && col0 + c < DHV) ? p.c0[(sidx * DHQK + d) * DHV + col0 + c] : 0.f;
   }
   for (int d = tid; d < 4 * DQ4; d += REC_THREADS) s_n[d] = (p.n0 && d < DHQK) ? p.n0[sidx * DHQK + d] : 0.f;
-  float m_prev = p.m0 ? p.m0[sidx] : 0.f;
+  double m_prev = p.m0 ? p.m0[sidx] : 0.f;
 
   // output tile of a thread: rows j0, j0 + 16; S columns / value columns c0, c0 + 16
   const int j0 = (warp & 3) * 4 + (lane >> 3), c0 = (warp >> 2) * 8 + (lane & 7);
@@ -149,7 +164,7 @@ __global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_m
     const int64_t t0 = (int64_t)chunk * REC_L;
     // ---- gate recurrence of the chunk, lane = token; every warp forms it for itself
     const bool live = t0 + lane < len;
-    float bcum = live ? log_sigmoid(gf) : 0.f;
+    double bcum = live ? log_sigmoid(gf) : 0.f;
     const float iv = gi;
     {
       const int64_t tn = t0 + REC_L + lane;   // the next chunk's gates
@@ -158,84 +173,81 @@ __global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_m
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const float t = __shfl_up_sync(0xffffffffu, bcum, o);
+      const double t = __shfl_up_sync(0xffffffffu, bcum, o);
       if (lane >= o) bcum += t;
     }
-    const float al = live ? iv - bcum : -INFINITY;
-    float mu = fmaxf(al, m_prev);
+    const double al = live ? iv - bcum : -INFINITY;
+    double mu = fmax(al, m_prev);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const float t = __shfl_up_sync(0xffffffffu, mu, o);
-      if (lane >= o) mu = fmaxf(mu, t);
+      const double t = __shfl_up_sync(0xffffffffu, mu, o);
+      if (lane >= o) mu = fmax(mu, t);
     }
-    const float mu_last = __shfl_sync(0xffffffffu, mu, 31), b_last = __shfl_sync(0xffffffffu, bcum, 31);
-    const float r_tok = expf(m_prev - mu) * qscale, lower = expf(-(bcum + mu)), w_tok = expf(al - mu_last);
-    const float decay = expf(m_prev - mu_last);
+    const double mu_last = __shfl_sync(0xffffffffu, mu, 31), b_last = __shfl_sync(0xffffffffu, bcum, 31);
+    const float r_tok = expf((float)(m_prev - mu)) * qscale, lower = expf((float)-(bcum + mu)), w_tok = expf((float)(al - mu_last));
+    const float decay = expf((float)(m_prev - mu_last));
     m_prev = b_last + mu_last;
 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();   // the chunk is in shared memory; C and n of the previous chunk are complete
     if (ly.nbuf == 2 && chunk + 1 < nchunks) load_chunk(chunk + 1, buf ^ 1);
 
-    // ---- [S | QC] = Q [K ; C^T]^T, 2 x (2 + 2) outputs per thread
-    float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, qc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    // ---- [S | QC | q.n] = Q [K ; C^T ; n]^T, 2 x (2 + 2 + 1) outputs per thread: the eight threads of a row pair form the
+    // same q.n, which costs less than the shuffles that would share the work.  Four chains per sum, one per component of the
+    // 16-byte pieces: a quarter of the roundings in a row, no more instructions.
+    float s[2][2], qc[2][2], qn0, qn1;
     {
       const float *q0 = tq + j0 * DP, *q1 = q0 + 16 * DP, *k0 = tk + c0 * DP, *k1 = k0 + 16 * DP, *x0 = s_c + c0 * DP, *x1 = x0 + 16 * DP;
+      float4 acc[2][5] = {};
 #pragma unroll 4
       for (int d = 0; d < 4 * DQ4; d += 4) {
         const float4 a0 = *reinterpret_cast<const float4*>(q0 + d), a1 = *reinterpret_cast<const float4*>(q1 + d);
-        const float4 b0 = *reinterpret_cast<const float4*>(k0 + d), b1 = *reinterpret_cast<const float4*>(k1 + d);
-        const float4 e0 = *reinterpret_cast<const float4*>(x0 + d), e1 = *reinterpret_cast<const float4*>(x1 + d);
-        s[0][0] = dot4(a0, b0, s[0][0]); s[0][1] = dot4(a0, b1, s[0][1]);
-        s[1][0] = dot4(a1, b0, s[1][0]); s[1][1] = dot4(a1, b1, s[1][1]);
-        qc[0][0] = dot4(a0, e0, qc[0][0]); qc[0][1] = dot4(a0, e1, qc[0][1]);
-        qc[1][0] = dot4(a1, e0, qc[1][0]); qc[1][1] = dot4(a1, e1, qc[1][1]);
-      }
-    }
-    // ---- q_j . n of the four rows this warp's threads 8 i hold (rows 4 (warp % 4) + i and + 16): lane over features
-    float qn0 = 0.f, qn1 = 0.f;
+        const float4 b[5] = {*reinterpret_cast<const float4*>(k0 + d), *reinterpret_cast<const float4*>(k1 + d), *reinterpret_cast<const float4*>(x0 + d),
+                             *reinterpret_cast<const float4*>(x1 + d), *reinterpret_cast<const float4*>(s_n + d)};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float x = 0.f, y = 0.f;
-      const float *ra = tq + ((warp & 3) * 4 + i) * DP, *rb = ra + 16 * DP;
-      for (int d = lane; d < DHQK; d += 32) {
-        x = fmaf(ra[d], s_n[d], x);
-        y = fmaf(rb[d], s_n[d], y);
+        for (int i = 0; i < 5; ++i) {
+          fma4(acc[0][i], a0, b[i]);
+          fma4(acc[1][i], a1, b[i]);
+        }
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        x += __shfl_xor_sync(0xffffffffu, x, o);
-        y += __shfl_xor_sync(0xffffffffu, y, o);
+      for (int j = 0; j < 2; ++j) {
+        s[j][0] = sum4(acc[j][0]); s[j][1] = sum4(acc[j][1]);
+        qc[j][0] = sum4(acc[j][2]); qc[j][1] = sum4(acc[j][3]);
       }
-      if ((lane >> 3) == i) { qn0 = x; qn1 = y; }
+      qn0 = sum4(acc[0][4]);
+      qn1 = sum4(acc[1][4]);
     }
     // ---- P and the w-scaled v
-    const float mu0 = __shfl_sync(0xffffffffu, mu, j0), mu1 = __shfl_sync(0xffffffffu, mu, j0 + 16);
-    const float al0 = __shfl_sync(0xffffffffu, al, c0), al1 = __shfl_sync(0xffffffffu, al, c0 + 16);
-    s_p[j0 * REC_LP + c0] = c0 <= j0 ? s[0][0] * qscale * expf(al0 - mu0) : 0.f;
+    const double mu0 = __shfl_sync(0xffffffffu, mu, j0), mu1 = __shfl_sync(0xffffffffu, mu, j0 + 16);
+    const double al0 = __shfl_sync(0xffffffffu, al, c0), al1 = __shfl_sync(0xffffffffu, al, c0 + 16);
+    s_p[j0 * REC_LP + c0] = c0 <= j0 ? s[0][0] * qscale * expf((float)(al0 - mu0)) : 0.f;
     s_p[j0 * REC_LP + c0 + 16] = 0.f;                                              // (c0 + 16 > j0)
-    s_p[(j0 + 16) * REC_LP + c0] = s[1][0] * qscale * expf(al0 - mu1);             // (c0 < j0 + 16)
-    s_p[(j0 + 16) * REC_LP + c0 + 16] = c0 <= j0 ? s[1][1] * qscale * expf(al1 - mu1) : 0.f;
+    s_p[(j0 + 16) * REC_LP + c0] = s[1][0] * qscale * expf((float)(al0 - mu1));             // (c0 < j0 + 16)
+    s_p[(j0 + 16) * REC_LP + c0 + 16] = c0 <= j0 ? s[1][1] * qscale * expf((float)(al1 - mu1)) : 0.f;
 #pragma unroll
     for (int i = 0; i < REC_COLS / 8; ++i) s_vw[(warp * (REC_COLS / 8) + i) * REC_LP + lane] = tv[(warp * (REC_COLS / 8) + i) * REC_LP + lane] * w_tok;
-    __syncthreads();   // P and the scaled v are complete, C and n are read
+    if (warp == 0) s_w[lane] = w_tok;
+    __syncthreads();   // P, the scaled v and w are complete, C and n are read
 
     // ---- h = (r QC + P V) / den
     {
-      float o[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, rs0 = 0.f, rs1 = 0.f;
+      float4 oa[2][2] = {}, ra[2] = {};
       const float *p0 = s_p + j0 * REC_LP, *p1 = p0 + 16 * REC_LP, *v0 = tv + c0 * REC_LP, *v1 = v0 + 16 * REC_LP;
+      const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
 #pragma unroll
       for (int l = 0; l < REC_L; l += 4) {
         const float4 b0 = *reinterpret_cast<const float4*>(v0 + l), b1 = *reinterpret_cast<const float4*>(v1 + l);
         const float4 a1 = *reinterpret_cast<const float4*>(p1 + l);
         if (l < 16) {   // row j0 < 16 has no later tokens
           const float4 a0 = *reinterpret_cast<const float4*>(p0 + l);
-          o[0][0] = dot4(a0, b0, o[0][0]); o[0][1] = dot4(a0, b1, o[0][1]);
-          rs0 += (a0.x + a0.y) + (a0.z + a0.w);
+          fma4(oa[0][0], a0, b0); fma4(oa[0][1], a0, b1);
+          fma4(ra[0], a0, one);
         }
-        o[1][0] = dot4(a1, b0, o[1][0]); o[1][1] = dot4(a1, b1, o[1][1]);
-        rs1 += (a1.x + a1.y) + (a1.z + a1.w);
+        fma4(oa[1][0], a1, b0); fma4(oa[1][1], a1, b1);
+        fma4(ra[1], a1, one);
       }
+      const float o[2][2] = {{sum4(oa[0][0]), sum4(oa[0][1])}, {sum4(oa[1][0]), sum4(oa[1][1])}}, rs0 = sum4(ra[0]), rs1 = sum4(ra[1]);
       const float r0 = __shfl_sync(0xffffffffu, r_tok, j0), r1 = __shfl_sync(0xffffffffu, r_tok, j0 + 16);
       const float lo0 = __shfl_sync(0xffffffffu, lower, j0), lo1 = __shfl_sync(0xffffffffu, lower, j0 + 16);
       const float den0 = fmaxf(fabsf(fmaf(r0, qn0, rs0)), lo0) + p.eps, den1 = fmaxf(fabsf(fmaf(r1, qn1, rs1)), lo1) + p.eps;
@@ -273,12 +285,18 @@ __global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_m
       *x0 = a;
       *x1 = e;
     }
-    // ---- n <- decay n + sum_l w_l k_l: warp i takes features i, i + 8, ...; lane = token
-    for (int d = warp; d < DHQK; d += REC_THREADS / 32) {
-      float x = tk[lane * DP + d] * w_tok;
+    // ---- n <- decay n + sum_l w_l k_l: thread = feature, the last warps first (the first ones may have one more unit of C)
+    for (int d = REC_THREADS - 1 - tid; d < DHQK; d += REC_THREADS) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      if (lane == 0) s_n[d] = fmaf(decay, s_n[d], x);
+      for (int l = 0; l < REC_L; l += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(s_w + l);
+        x.x = fmaf(w.x, tk[l * DP + d], x.x);
+        x.y = fmaf(w.y, tk[(l + 1) * DP + d], x.y);
+        x.z = fmaf(w.z, tk[(l + 2) * DP + d], x.z);
+        x.w = fmaf(w.w, tk[(l + 3) * DP + d], x.w);
+      }
+      s_n[d] = fmaf(decay, s_n[d], sum4(x));
     }
     if (ly.nbuf == 1 && chunk + 1 < nchunks) {
       __syncthreads();   // the only buffer is free
@@ -294,7 +312,7 @@ __global__ void __launch_bounds__(REC_THREADS) mlstm_recurrent_kernel(const xl_m
   }
   if (blockIdx.x == 0) {
     for (int d = tid; d < DHQK; d += REC_THREADS) p.n_out[sidx * DHQK + d] = s_n[d];
-    if (tid == 0) p.m_out[sidx] = m_prev;
+    if (tid == 0) p.m_out[sidx] = (float)m_prev;
   }
 }
 
@@ -315,7 +333,10 @@ int validate_seq_common(const xl_mlstm_seq_params* p) {
 
 template <typename T>
 static int launch_recurrent(const xl_mlstm_seq_params* p, size_t smem, cudaStream_t st) {
-  auto kern = mlstm_recurrent_kernel<T>;
+  auto kern = p->DHQK == 64    ? mlstm_recurrent_kernel<T, 64>
+              : p->DHQK == 128 ? mlstm_recurrent_kernel<T, 128>
+              : p->DHQK == 256 ? mlstm_recurrent_kernel<T, 256>
+                               : mlstm_recurrent_kernel<T, 0>;
   XL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int nd = p->cu_seqlens ? p->num_docs : p->B;
   // 16-byte copies of q and k rows (fp32): every row starts on a 16-byte boundary and is a whole number of pieces

@@ -10,8 +10,8 @@ row-parallel projections) and slot-indexed states.
 
 It consumes a state dict with the reference's "single" weight-mode key names
 (``backbone.blocks.{i}.mlstm_layer.q.weight`` ...), so real checkpoints and the reference's own
-modules are interchangeable with it.  Dense layers are plain library GEMMs (``torch.nn.functional.linear``);
-the recurrent cell is the only part computed by this package's CUDA kernels.
+modules are interchangeable with it.  Dense layers are plain library GEMMs (``torch.nn.functional.linear``)
+but for a few rows at a time (``ops.rows_linear``); the recurrent cell and the operators next to it are this package's CUDA kernels.
 """
 from __future__ import annotations
 

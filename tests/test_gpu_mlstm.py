@@ -361,3 +361,19 @@ def test_fused_decode_cell_equals_cap_step_norm_gate(dtype, B, NH, DQ, DV, with_
     if with_slots:   # inactive streams: zero output, pool untouched
         idle = [j for j in range(B) if int(slot[j]) < 0]
         assert float(got[idle].float().abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("DQ", [64, 128, 256])
+@pytest.mark.parametrize("S,off", [(33, 0), (64, 1), (70, 0)])
+def test_recurrent_with_compiled_head_sizes_equals_the_general_kernel(DQ, S, off):
+    """Head sizes with an instance of their own, with and without 16-byte rows.  One zero feature more takes the general
+    instance: same sums, up to 1/sqrt(d), which q makes up for.  Both are fp32 sums, so TOL_F32 is far above their difference."""
+    import xlstm_b200
+    q, k, v, i, f = _cuda(*_inputs(61, 1, 2, S, DQ, 96, torch.float32))
+    if off:   # rows that start 4 bytes past a 16-byte boundary
+        q, k = (torch.cat([torch.zeros_like(t[..., :1]), t, torch.zeros_like(t[..., :3])], -1)[..., 1:DQ + 1] for t in (q, k))
+    h, (c, n, m) = xlstm_b200.mlstm_sequence(q, k, v, i, f, kernel="recurrent")
+    pad = lambda t: torch.cat([t, torch.zeros_like(t[..., :1])], -1)
+    h1, (c1, n1, m1) = xlstm_b200.mlstm_sequence(pad(q) * ((DQ + 1) / DQ) ** 0.5, pad(k), v, i, f, kernel="recurrent")
+    for a, b in ((h, h1), (c, c1[:, :, :DQ]), (n, n1[..., :DQ]), (m, m1)):
+        assert float((a - b).norm()) <= TOL_F32 * float(b.norm())

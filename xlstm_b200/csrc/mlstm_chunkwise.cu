@@ -259,7 +259,9 @@ static __device__ __noinline__ void cw_store_state(float* c_out, int DHV, int gr
   }
 }
 
-template <int DHQK>
+// PARTS = false: every document is one block's alone.  An instance of its own, because what the parts need (a document looked up,
+// states folded in) took registers from the loops: 4 x 8192 tokens 254.3 -> 251.4 us, 8 x 1000 tokens of 4 x 128/256 29.2 -> 28.1.
+template <int DHQK, bool PARTS>
 __global__ void __launch_bounds__(CW_THREADS, 1)
 mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_params p, const CwSplit split) {
   using LY = CwLayout<DHQK>;
@@ -293,11 +295,13 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
 
   // Behind mlstm_part_state_kernel a document's first part does not wait for it, so all it reads through this path was
   // complete when that kernel passed its own wait, and is read from L2 (__ldcg, TMA).
-  if (!split.after_states) grid_dependency_wait();
+  if (!PARTS || !split.after_states) grid_dependency_wait();
 
   // ---- this block's part of a document
   CwItem it;
-  if (split.counts) {
+  if constexpr (!PARTS) {
+    it.parts = 1; it.doc = (int)blockIdx.z; it.part = 0; it.first_chunk = 0; it.chunks = split.part_chunks; it.slot0 = 0;
+  } else if (split.counts) {
     if ((int)blockIdx.z >= __ldcg(split.counts)) { grid_dependency_wait(); return; }
     it = cw_load_item(split.items + blockIdx.z);
   } else {
@@ -991,7 +995,7 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
 
   if (!ok && p.status) atomicExch(p.status, 1);
   // (a first part has not waited yet: the end of this kernel means the end of the one in front, too)
-  if (split.after_states && it.part == 0) grid_dependency_wait();
+  if (PARTS && split.after_states && it.part == 0) grid_dependency_wait();
   tc_fence_before();
   __syncthreads();
   if (warp == W_UMMA) tmem_dealloc(tmem, CW_TMEM_COLS);
@@ -1066,7 +1070,7 @@ template <int DHQK>
 static int launch_chunkwise(const CwMaps& maps, const xl_mlstm_seq_params* p, const CwSplit& split, unsigned grid_z, cudaStream_t st) {
   using LY = CwLayout<DHQK>;
   static_assert(LY::DYN_SMEM <= 227 * 1024, "shared memory budget");
-  auto kern = mlstm_chunkwise_kernel<DHQK>;
+  auto kern = split.counts || split.parts > 1 ? mlstm_chunkwise_kernel<DHQK, true> : mlstm_chunkwise_kernel<DHQK, false>;
   XL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::DYN_SMEM));
   XL_CUDA_TRY(launch_dependent(kern, dim3(p->DHV / CW_DV, p->NH, grid_z), dim3(CW_THREADS), LY::DYN_SMEM, st, maps, *p, split));
   return check_launch("xl_mlstm_chunkwise");

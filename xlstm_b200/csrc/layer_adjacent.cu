@@ -304,10 +304,12 @@ constexpr int CONV_THREADS = 128, CONV_TILE = 32, CONV_GROUP = 8, CONV_MAXK = 8;
 template <typename T, int K>
 __global__ void __launch_bounds__(CONV_THREADS) causal_conv1d_kernel(const xl_conv1d_params p) {
   constexpr int V = Vec16<T>::N, W = K > 1 ? K - 1 : 1;
-  const int f0 = (blockIdx.y * CONV_THREADS + threadIdx.x) * V;
+  const unsigned fblocks = (unsigned)(p.F / V + CONV_THREADS - 1) / CONV_THREADS;   // (one axis for both: either may be long)
+  const unsigned tile = blockIdx.x / fblocks;
+  const int f0 = ((blockIdx.x - tile * fblocks) * CONV_THREADS + threadIdx.x) * V;
   if (f0 >= p.F) return;
-  const int b = blockIdx.z;
-  const int t0 = blockIdx.x * CONV_TILE, t1 = min(p.S, t0 + CONV_TILE);
+  const int b = blockIdx.y;
+  const int t0 = tile * CONV_TILE, t1 = min(p.S, t0 + CONV_TILE);
   const T* x = static_cast<const T*>(p.x) + (long long)b * p.x_sb + f0;
   T* out = static_cast<T*>(p.out) + (long long)b * p.o_sb + f0;
   // win[l-1] = x[t-l]; wl[l] multiplies x[t-l] (tap K-1-l of the convolution's weight)
@@ -518,8 +520,10 @@ extern "C" int xl_causal_conv1d(const xl_conv1d_params* p, void* cuda_stream) {
   if (p->x_sb % V || p->x_st % V || p->o_sb % V || p->o_st % V || p->x_st < p->F || p->o_st < p->F) return XL_ERR_BAD_STRIDE;
   if (!aligned16(p->x) || !aligned16(p->out)) return XL_ERR_BAD_ALIGNMENT;
   if (p->out == p->x) return XL_ERR_ALIASING;   // a tile's halo is read by the neighbouring thread block
-  const dim3 grid((unsigned)((p->S + CONV_TILE - 1) / CONV_TILE), (unsigned)((p->F / V + CONV_THREADS - 1) / CONV_THREADS), (unsigned)p->B);
-  if (grid.y > 65535) return XL_ERR_TOO_LARGE;
+  if (p->S > 65535 * 64) return XL_ERR_TOO_LARGE;
+  const int64_t blocks = (int64_t)((p->S + CONV_TILE - 1) / CONV_TILE) * ((p->F / V + CONV_THREADS - 1) / CONV_THREADS);
+  if (blocks > 0x7fffffff) return XL_ERR_TOO_LARGE;
+  const dim3 grid((unsigned)blocks, (unsigned)p->B);
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
 #define XL_CONV_LAUNCH(KK)                                                                             \
   case KK:                                                                                             \

@@ -149,15 +149,16 @@ typedef struct xl_mlstm_decode_cell_params {
 int xl_mlstm_decode_cell(const xl_mlstm_decode_cell_params* p, void* cuda_stream);
 
 /* ------------------------------------------------------------------------------------------------
- * sLSTM forward over a sequence, one persistent kernel: one thread-block cluster per (head, group of 16 batch
- * rows), each CTA's slice of the recurrent matrix resident in registers as tensor-core fragments, the new h
- * exchanged every time step through asynchronous distributed-shared-memory stores that complete on mbarriers.
+ * sLSTM forward over a sequence, one persistent kernel: one thread-block cluster per (head, group of 8 or 16 batch
+ * rows: 8 where all clusters are resident at once), each CTA's slice of the recurrent matrix resident in registers
+ * as tensor-core fragments, the new h exchanged every time step through asynchronous distributed-shared-memory
+ * stores that complete on mbarriers.
  * Replaces sLSTMFunc.forward (xlstm/blocks/slstm/src/cuda/slstm.cc:53-135), i.e. the host loop
  * ForwardPass::Run (slstm_forward.cu:217-267) + SLSTMPointwiseForward (slstm_pointwise.cu:24-116).
  * ---------------------------------------------------------------------------------------------- */
 typedef struct xl_slstm_params {
   const void* wx;        /* (B, S, 4, NH, DH) gate pre-activations, gates ordered i,f,z,o; dtype `dtype` */
-  const void* R;         /* (NH, DH_in, 4, DH_out) recurrent matrix, dtype `dtype` */
+  const void* R;         /* (NH, DH_in, 4, DH_out) recurrent matrix, dtype `dtype`; any address an element may have */
   const float* bias;     /* (NH, 4, DH) */
   const float* state0;   /* (4, B, NH*DH) ordered h,c,n,m; or NULL = zeros */
   void* h_out;           /* (B, NH, S, DH), dtype `dtype` */
@@ -172,7 +173,7 @@ typedef struct xl_slstm_params {
                             reference's `states` and gate caches, slstm.cc:88-101).  Not with cu_seqlens. */
 } xl_slstm_params;
 
-/* Requires DH in {64,128,256}; any B (batch rows are tiled into groups of 16), dtype XL_BF16. */
+/* Requires DH in {64,128,256}; any B, dtype XL_BF16; wx 16-byte aligned, h_out 4-byte aligned. */
 int xl_slstm_forward(const xl_slstm_params* p, void* cuda_stream);
 
 /* Size of the training cache of one forward call (0 for unsupported shapes).  Host only, no CUDA call. */

@@ -52,6 +52,28 @@ def test_matches_oracle_on_both_sides_of_the_row_split(B, S, NH, DH, with_state)
     assert rel_l2(out, out_ref) < TOL and all(rel_l2(last[i], last_ref[i]) < TOL for i in range(4))
 
 
+@pytest.mark.parametrize("off", [1, 2, 4])
+@pytest.mark.parametrize("B,NH,DH", [(3, 2, 64), (9, 1, 128), (16, 4, 256), (523, 3, 64)])
+def test_recurrent_matrix_at_any_address(B, NH, DH, off):
+    """A recurrent matrix that is a view into a flat parameter buffer starts 2, 4 or 8 bytes past a 16-byte boundary (clusters of
+    eight and of sixteen batch rows).  The same elements in the same order: equal bit for bit, the training cache too."""
+    import xlstm_b200
+    wx, R, bias, st = (t.cuda() for t in _case(77 + DH, B, 5, NH, DH, True))
+    flat = torch.empty(R.numel() + off, dtype=torch.bfloat16, device="cuda")
+    view = flat[off:].view(R.shape)
+    view.copy_(R)
+    assert view.is_contiguous() and view.data_ptr() % 16 == 2 * off and R.data_ptr() % 16 == 0
+    for train in (False, True):
+        want = xlstm_b200.slstm_forward(wx, R, bias, st, train_cache=train)
+        got = xlstm_b200.slstm_forward(wx, view, bias, st, train_cache=train)
+        xlstm_b200.check_device_status()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    if off % 2 == 0:   # (the backward kernel reads R in pairs of elements)
+        gh = torch.ones_like(got[0])
+        grads = [xlstm_b200.ops.slstm_backward(r[2], m, gh, None, st) for r, m in ((want, R), (got, view))]
+        assert torch.equal(grads[0][0], grads[1][0]) and torch.equal(grads[0][1], grads[1][1])
+
+
 def test_document_boundaries_in_several_row_groups():
     """Boundaries in both rows of a thread's pair, in neighbouring steps and in the second group of eight rows."""
     B, S, NH, DH = 11, 24, 2, 256

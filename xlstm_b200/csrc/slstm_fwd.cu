@@ -407,11 +407,23 @@ __global__ void __launch_bounds__(SL_THREADS, 1) slstm_forward_rows8_kernel(cons
 
   // ---- this CTA's slice of R, (NH, DH_in, 4, DH_out), into shared memory; then the first Wx steps behind it
   {
+    // (the contract asks nothing of R's address: a view into a flat parameter buffer may start anywhere.  All pieces have
+    // the alignment of the base, so one test decides; off a 16-byte boundary they come element by element.)
     const __nv_bfloat16* R = reinterpret_cast<const __nv_bfloat16*>(p.R) + (size_t)head * DH * 4 * DH + rank * SL_UNITS;
+    const bool whole_pieces = (reinterpret_cast<uintptr_t>(p.R) & 15u) == 0;
+    if (whole_pieces) {
 #pragma unroll 8
-    for (int i = tid; i < DH * 16; i += SL_THREADS) {
-      const int w = i & 3, g = (i >> 2) & 3, k = i >> 4;
-      cp_async16(s_r + ((w * 4 + g) * DH + k) * 16, R + ((size_t)k * 4 + g) * DH + w * 8);
+      for (int i = tid; i < DH * 16; i += SL_THREADS) {
+        const int w = i & 3, g = (i >> 2) & 3, k = i >> 4;
+        cp_async16(s_r + ((w * 4 + g) * DH + k) * 16, R + ((size_t)k * 4 + g) * DH + w * 8);
+      }
+    } else {
+      uint16_t* dst = reinterpret_cast<uint16_t*>(sl_smem + LY::OFF_R);
+#pragma unroll 8
+      for (int i = tid; i < DH * 4 * SL_UNITS; i += SL_THREADS) {   // neighbouring threads: neighbouring elements of a piece row
+        const int u = i & (SL_UNITS - 1), g = (i >> 5) & 3, k = i >> 7;
+        dst[(((u >> 3) * 4 + g) * DH + k) * 8 + (u & 7)] = *reinterpret_cast<const uint16_t*>(R + ((size_t)k * 4 + g) * DH + u);
+      }
     }
     cp_async_commit();
   }

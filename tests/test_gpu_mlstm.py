@@ -186,6 +186,25 @@ def test_chunkwise_split_into_parts_matches_oracle(B, NH, S, DQ, DV, with_state,
     _check(h, st, h_ref, st_ref, TOL_BF16)
 
 
+@pytest.mark.parametrize("lo,hi", [(0, 64), (0, 512), (256, 640), (900, 1000), (0, 1000)])
+@pytest.mark.parametrize("with_state", [False, True])
+def test_chunkwise_parts_with_masked_tokens(lo, hi, with_state):
+    """Input gates of -inf (a caller's padding) over whole parts: these add nothing, and what lies in front and behind is kept.
+    1000 tokens of four heads are cut into parts of a chunk or two."""
+    import xlstm_b200
+    q, k, v, i, f = _inputs(64, 1, 4, 1000, 64, 128, torch.bfloat16)
+    i[:, :, lo:hi] = -float("inf")
+    init = _state(65, 1, 4, 64, 128) if with_state else (None, None, None)
+    h_ref, st_ref = O.mlstm_sequence(q, k, v, i, f, *init)
+    h, st = xlstm_b200.mlstm_sequence(*_cuda(q, k, v, i, f), *_cuda(*init), kernel="chunkwise")
+    xlstm_b200.check_device_status()
+    if hi - lo == 1000 and not with_state:
+        assert all(int(torch.count_nonzero(t)) == 0 for t in (h, st[0], st[1]))
+        assert rel_l2(st[2].cpu().reshape(st_ref[2].shape), st_ref[2]) < TOL_F32
+    else:
+        _check(h, st, h_ref, st_ref, TOL_BF16)
+
+
 def test_chunkwise_packed_documents_longer_than_a_part():
     """Packed rows with documents far above and far below the length of a part, empty ones among them."""
     import xlstm_b200

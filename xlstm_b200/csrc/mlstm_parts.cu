@@ -144,7 +144,9 @@ mlstm_part_state_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_
     float mu = s_max[0];
 #pragma unroll
     for (int w = 1; w < PS_THREADS / 32; ++w) mu = fmaxf(mu, s_max[w]);
-    for (int t = t0; t < t1; ++t) s_w[t] = __expf(s_w[t] - mu);
+    // (input gates of -inf throughout, a caller's mask: the part adds nothing, its weights are 0 and its stabiliser is -inf)
+    const float frame = mu == -INFINITY ? 0.f : mu;
+    for (int t = t0; t < t1; ++t) s_w[t] = __expf(s_w[t] - frame);
     if (slice == 0 && tid == 0) split.gm[(long long)slot * p.NH + head] = make_float2(total, total + mu);
     __syncthreads();
   }

@@ -116,6 +116,21 @@ def test_recurrent_at_the_edges_of_its_tiles(dtype, tol, B, NH, S, DQ, DV, with_
     _check(h, st, h_ref, st_ref, tol)
 
 
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, TOL_F32), (torch.bfloat16, TOL_BF16)])
+@pytest.mark.parametrize("gate", [-float("inf"), -1e30, -2e6, -9e5])
+@pytest.mark.parametrize("at,with_state", [((0,), True), ((31,), False), ((32,), True), ((5, 6, 21), False), ((63, 64, 95, 96), True), ((99,), False)])
+def test_recurrent_forget_gates_that_reset_the_state(dtype, tol, gate, at, with_state):
+    """Forget gates of -inf (f = 0 exactly) and huge negative ones, at the edges of the 32-token chunks and in a row: what is
+    behind a reset depends on nothing in front of it, and the input gates there keep their precision."""
+    import xlstm_b200
+    q, k, v, i, f = _inputs(53, 1, 2, 100, 64, 64, dtype)
+    f[:, :, list(at)] = gate
+    init = _state(54, 1, 2, 64, 64) if with_state else (None, None, None)
+    h_ref, st_ref = O.mlstm_sequence(q, k, v, i, f, *init)
+    h, st = xlstm_b200.mlstm_sequence(*_cuda(q, k, v, i, f), *_cuda(*init), kernel="recurrent")
+    _check(h, st, h_ref, st_ref, tol)
+
+
 # ------------------------------------------------------------------------------------------------ chunkwise (tcgen05)
 @pytest.mark.parametrize("B,NH,S,DQ,DV,with_state", [
     (2, 2, 256, 64, 128, False),

@@ -25,6 +25,8 @@ constexpr int REC_THREADS = 256;
 constexpr int REC_L = 32;                         // tokens per chunk
 constexpr int REC_COLS = 32;                      // C columns per CTA
 constexpr int REC_LP = REC_L + 4;                 // padded row of the token-indexed tiles (floats)
+constexpr float REC_HARD = -1e6f;                 // log f below which a chunk's gates are formed without differences of their
+                                                  // sums: above it, 32 of them cost a 64-bit difference 1e-8 at most
 
 __device__ __forceinline__ void rec_cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -164,29 +166,57 @@ __global__ void __launch_bounds__(REC_THREADS, 1) mlstm_recurrent_kernel(const x
     const int64_t t0 = (int64_t)chunk * REC_L;
     // ---- gate recurrence of the chunk, lane = token; every warp forms it for itself
     const bool live = t0 + lane < len;
-    double bcum = live ? log_sigmoid(gf) : 0.f;
-    const float iv = gi;
+    const float lf = live ? log_sigmoid(gf) : 0.f, iv = live ? gi : -INFINITY;
     {
       const int64_t tn = t0 + REC_L + lane;   // the next chunk's gates
       gi = tn < len ? ig[tn * p.g_st] : 0.f;
       gf = tn < len ? fg[tn * p.g_st] : 0.f;
     }
+    double bcum = lf;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const double t = __shfl_up_sync(0xffffffffu, bcum, o);
       if (lane >= o) bcum += t;
     }
-    const double al = live ? iv - bcum : -INFINITY;
-    double mu = fmax(al, m_prev);
+    double al = iv - bcum, mu = fmax(al, m_prev);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const double t = __shfl_up_sync(0xffffffffu, mu, o);
       if (lane >= o) mu = fmax(mu, t);
     }
     const double mu_last = __shfl_sync(0xffffffffu, mu, 31), b_last = __shfl_sync(0xffffffffu, bcum, 31);
-    const float r_tok = expf((float)(m_prev - mu)) * qscale, lower = expf((float)-(bcum + mu)), w_tok = expf((float)(al - mu_last));
-    const float decay = expf((float)(m_prev - mu_last));
-    m_prev = b_last + mu_last;
+    float r_tok = expf((float)(m_prev - mu)) * qscale, lower = expf((float)-(bcum + mu)), w_tok = expf((float)(al - mu_last));
+    float decay = expf((float)(m_prev - mu_last));
+    double m_next = b_last + mu_last;
+    const bool hard = __any_sync(0xffffffffu, lf < REC_HARD);
+    if (hard) {
+      // A forget gate that resets the state (the same for every warp).  b reaches -inf, or a size beside which the input
+      // gates are lost, so nothing may be a difference of its values: the stabilisers m_j themselves by a scan over
+      // (sum of log f, max) pairs, sums in front of and behind a token on their own.  al and mu are i and m here; what lies
+      // between two tokens is added below, where P is formed.
+      double g = lf, x = iv, behind = 0.;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double tg = __shfl_up_sync(0xffffffffu, g, o), tx = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) {
+          x = fmax(x, tx + g);
+          g += tg;
+        }
+      }
+#pragma unroll 1
+      for (int t = 1; t < 32; ++t) {
+        const float ft = __shfl_sync(0xffffffffu, lf, t);
+        if (t > lane) behind += ft;
+      }
+      al = iv;
+      mu = fmax(m_prev + g, x);
+      m_next = __shfl_sync(0xffffffffu, mu, 31);
+      r_tok = expf((float)(m_prev + g - mu)) * qscale;
+      lower = expf((float)-mu);
+      w_tok = expf((float)(iv + behind - m_next));
+      decay = expf((float)(m_prev + __shfl_sync(0xffffffffu, g, 31) - m_next));
+    }
+    m_prev = m_next;
 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();   // the chunk is in shared memory; C and n of the previous chunk are complete
@@ -221,10 +251,24 @@ __global__ void __launch_bounds__(REC_THREADS, 1) mlstm_recurrent_kernel(const x
     // ---- P and the w-scaled v
     const double mu0 = __shfl_sync(0xffffffffu, mu, j0), mu1 = __shfl_sync(0xffffffffu, mu, j0 + 16);
     const double al0 = __shfl_sync(0xffffffffu, al, c0), al1 = __shfl_sync(0xffffffffu, al, c0 + 16);
-    s_p[j0 * REC_LP + c0] = c0 <= j0 ? s[0][0] * qscale * expf((float)(al0 - mu0)) : 0.f;
-    s_p[j0 * REC_LP + c0 + 16] = 0.f;                                              // (c0 + 16 > j0)
-    s_p[(j0 + 16) * REC_LP + c0] = s[1][0] * qscale * expf((float)(al0 - mu1));             // (c0 < j0 + 16)
-    s_p[(j0 + 16) * REC_LP + c0 + 16] = c0 <= j0 ? s[1][1] * qscale * expf((float)(al1 - mu1)) : 0.f;
+    float e00 = (float)(al0 - mu0), e10 = (float)(al0 - mu1), e11 = (float)(al1 - mu1);
+    if (hard) {   // the sums of log f over the tokens behind l up to j
+      double d00 = 0., d10 = 0., d11 = 0.;
+#pragma unroll 1
+      for (int t = 1; t < 32; ++t) {
+        const float ft = __shfl_sync(0xffffffffu, lf, t);
+        if (t > c0 && t <= j0) d00 += ft;
+        if (t > c0 && t <= j0 + 16) d10 += ft;
+        if (t > c0 + 16 && t <= j0 + 16) d11 += ft;
+      }
+      e00 = (float)(al0 + d00 - mu0);
+      e10 = (float)(al0 + d10 - mu1);
+      e11 = (float)(al1 + d11 - mu1);
+    }
+    s_p[j0 * REC_LP + c0] = c0 <= j0 ? s[0][0] * qscale * expf(e00) : 0.f;
+    s_p[j0 * REC_LP + c0 + 16] = 0.f;                                     // (c0 + 16 > j0)
+    s_p[(j0 + 16) * REC_LP + c0] = s[1][0] * qscale * expf(e10);          // (c0 < j0 + 16)
+    s_p[(j0 + 16) * REC_LP + c0 + 16] = c0 <= j0 ? s[1][1] * qscale * expf(e11) : 0.f;
 #pragma unroll
     for (int i = 0; i < REC_COLS / 8; ++i) s_vw[(warp * (REC_COLS / 8) + i) * REC_LP + lane] = tv[(warp * (REC_COLS / 8) + i) * REC_LP + lane] * w_tok;
     if (warp == 0) s_w[lane] = w_tok;

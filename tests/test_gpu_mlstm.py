@@ -131,6 +131,23 @@ def test_recurrent_forget_gates_that_reset_the_state(dtype, tol, gate, at, with_
     _check(h, st, h_ref, st_ref, tol)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("at", [1, 15, 16, 31, 32, 70])
+def test_recurrent_values_that_are_not_finite_stay_causal(dtype, bad, at):
+    """A NaN or an infinity among the values reaches its own column from its own token on, nothing in front and no other column."""
+    import xlstm_b200
+    q, k, v, i, f = _inputs(55, 1, 1, 80, 64, 40, dtype)
+    want, _ = xlstm_b200.mlstm_sequence(*_cuda(q, k, v, i, f), kernel="recurrent")
+    v[:, :, at, 17] = bad
+    h, (c, n, m) = xlstm_b200.mlstm_sequence(*_cuda(q, k, v, i, f), kernel="recurrent")
+    keep = [x for x in range(40) if x != 17]
+    tol = 2 ** -7 if dtype == torch.bfloat16 else 1e-6   # (the sums of a chunk with such a value run in another order)
+    for a, b in ((h[:, :, :at], want[:, :, :at]), (h[..., keep], want[..., keep])):
+        assert float((a.float() - b.float()).norm()) <= tol * float(b.float().norm())
+    assert not bool(torch.isfinite(h[:, :, at, 17]).any()) and not bool(torch.isfinite(c[..., 17]).any())
+
+
 # ------------------------------------------------------------------------------------------------ chunkwise (tcgen05)
 @pytest.mark.parametrize("B,NH,S,DQ,DV,with_state", [
     (2, 2, 256, 64, 128, False),

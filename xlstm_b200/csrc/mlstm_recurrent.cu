@@ -269,10 +269,17 @@ __global__ void __launch_bounds__(REC_THREADS, 1) mlstm_recurrent_kernel(const x
     s_p[j0 * REC_LP + c0 + 16] = 0.f;                                     // (c0 + 16 > j0)
     s_p[(j0 + 16) * REC_LP + c0] = s[1][0] * qscale * expf(e10);          // (c0 < j0 + 16)
     s_p[(j0 + 16) * REC_LP + c0 + 16] = c0 <= j0 ? s[1][1] * qscale * expf(e11) : 0.f;
+    bool odd_v = false;
 #pragma unroll
-    for (int i = 0; i < REC_COLS / 8; ++i) s_vw[(warp * (REC_COLS / 8) + i) * REC_LP + lane] = tv[(warp * (REC_COLS / 8) + i) * REC_LP + lane] * w_tok;
+    for (int i = 0; i < REC_COLS / 8; ++i) {
+      const int at = (warp * (REC_COLS / 8) + i) * REC_LP + lane;
+      const float x = tv[at];
+      odd_v |= !(fabsf(x) < INFINITY);
+      s_vw[at] = x * w_tok;
+    }
     if (warp == 0) s_w[lane] = w_tok;
-    __syncthreads();   // P, the scaled v and w are complete, C and n are read
+    // P, the scaled v and w are complete, C and n are read; and whether an infinity or a NaN is among the chunk's values
+    const bool any_odd_v = __syncthreads_or(odd_v);
 
     // ---- h = (r QC + P V) / den
     {
@@ -291,7 +298,20 @@ __global__ void __launch_bounds__(REC_THREADS, 1) mlstm_recurrent_kernel(const x
         fma4(oa[1][0], a1, b0); fma4(oa[1][1], a1, b1);
         fma4(ra[1], a1, one);
       }
-      const float o[2][2] = {{sum4(oa[0][0]), sum4(oa[0][1])}, {sum4(oa[1][0]), sum4(oa[1][1])}}, rs0 = sum4(ra[0]), rs1 = sum4(ra[1]);
+      float o[2][2] = {{sum4(oa[0][0]), sum4(oa[0][1])}, {sum4(oa[1][0]), sum4(oa[1][1])}};
+      const float rs0 = sum4(ra[0]), rs1 = sum4(ra[1]);
+      if (any_odd_v) {   // 0 x inf: the zeros of P right of the diagonal must not meet the values of later tokens
+        o[0][0] = o[0][1] = o[1][0] = o[1][1] = 0.f;
+#pragma unroll 1
+        for (int l = 0; l <= j0 + 16; ++l) {
+          if (l <= j0) {
+            o[0][0] = fmaf(p0[l], v0[l], o[0][0]);
+            o[0][1] = fmaf(p0[l], v1[l], o[0][1]);
+          }
+          o[1][0] = fmaf(p1[l], v0[l], o[1][0]);
+          o[1][1] = fmaf(p1[l], v1[l], o[1][1]);
+        }
+      }
       const float r0 = __shfl_sync(0xffffffffu, r_tok, j0), r1 = __shfl_sync(0xffffffffu, r_tok, j0 + 16);
       const float lo0 = __shfl_sync(0xffffffffu, lower, j0), lo1 = __shfl_sync(0xffffffffu, lower, j0 + 16);
       const float den0 = fmaxf(fabsf(fmaf(r0, qn0, rs0)), lo0) + p.eps, den1 = fmaxf(fabsf(fmaf(r1, qn1, rs1)), lo1) + p.eps;

@@ -223,8 +223,7 @@ int64_t xl_slstm_weight_grads_scratch_bytes(int32_t B, int32_t S, int32_t NH, in
 
 /* ------------------------------------------------------------------------------------------------
  * y = x W^T for up to 16 rows of x (decoding), bf16 with fp32 accumulation: the linear layers around the decode cell
- * (xlstm/xlstm_large/model.py:379-452, 268-277) as streams of W.  W is read ahead of the kernel launched directly in front on
- * the stream: that kernel must not be the one that writes W.
+ * (xlstm/xlstm_large/model.py:379-452, 268-277) as streams of W.
  * ---------------------------------------------------------------------------------------------- */
 typedef struct xl_rows_linear_params {
   const void* x;         /* (rows, K), contiguous rows x_sr elements apart (a multiple of 8), 16-byte aligned */
@@ -237,6 +236,10 @@ typedef struct xl_rows_linear_params {
 } xl_rows_linear_params;
 
 int xl_rows_linear(const xl_rows_linear_params* p, void* cuda_stream);
+
+/* The same, for a caller who knows what it launched in front on the stream: W is read ahead of that kernel's end, so that
+ * kernel must not be the one that writes W (nor hold up another writer of W; whatever is in front of IT is complete). */
+int xl_rows_linear_ahead(const xl_rows_linear_params* p, void* cuda_stream);
 
 /* ------------------------------------------------------------------------------------------------
  * Operators next to the mLSTM cell in the reference's layer (xlstm/xlstm_large/model.py:379-452), each one pass

@@ -304,3 +304,42 @@ def test_rows_linear_matches_64_bits(rows, N, K):
     assert float((got.double() - want).norm()) <= (2 ** -8 + 1e-5) * float(want.norm())
     assert torch.equal(ops.rows_linear(x, w), got)
     assert torch.equal(ops.rows_linear(x.contiguous().view(rows, 1, K), w), got.view(rows, 1, N))
+
+
+@pytest.mark.parametrize("rows,N,K", [(8, 4096, 4096), (3, 50304, 1024), (16, 2048, 8192), (1, 300, 72)])
+def test_rows_linear_of_a_weight_written_by_the_launch_in_front(rows, N, K):
+    """A weight computed, cast or transposed on the line before, and one whose rows are not contiguous (the call copies it): in
+    these the launch directly in front writes what the kernel reads.  `w_ahead` does not apply to a copy made by the call."""
+    from xlstm_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    x = torch.randn(rows, K, generator=g, device="cuda").bfloat16()
+    base = torch.randn(K, N, generator=g, device="cuda") / K ** 0.5
+    w16 = base.t().contiguous().bfloat16()
+    torch.cuda.synchronize()
+    want = ops.rows_linear(x, w16)
+    held = torch.empty_like(w16)
+    wt = base.bfloat16().t()                                 # (N, K), rows not contiguous
+    assert not wt.is_contiguous() or N == 1
+    for _ in range(20):
+        held.zero_()
+        held.copy_(w16)
+        assert torch.equal(ops.rows_linear(x, held), want)
+        assert torch.equal(ops.rows_linear(x, wt, w_ahead=True), want)
+        assert torch.equal(ops.rows_linear(x, base.t().contiguous().bfloat16()), want)
+    torch.cuda.synchronize()
+    assert torch.equal(ops.rows_linear(x, w16, w_ahead=True), want)
+
+
+def test_linear_layers_of_the_model_leave_weights_without_row_order_to_the_library():
+    """A weight held transposed costs the weight-streaming kernel a copy per call; the library reads it as it lies."""
+    from xlstm_b200 import ops
+    from xlstm_b200.large_model import LargeModel
+    model = LargeModel.__new__(LargeModel)
+    model.fused, model.dtype = True, torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(4, 1, 2048, generator=g, device="cuda").bfloat16()
+    w = torch.randn(2048, 2048, generator=g, device="cuda").bfloat16()
+    with torch.no_grad():
+        assert torch.equal(model._linear(x, w.t()), torch.nn.functional.linear(x, w.t()))
+        torch.cuda.synchronize()
+        assert torch.equal(model._linear(x, w), ops.rows_linear(x, w))

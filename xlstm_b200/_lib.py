@@ -21,7 +21,7 @@ EXPORTS = (
     "xl_add_rmsnorm", "xl_headnorm_gate", "xl_soft_cap", "xl_causal_conv1d",
     "xl_softcap_argmax", "xl_softcap_argmax_scratch_bytes", "xl_swiglu",
     "xl_softcap_argmax_noalloc", "xl_softcap_argmax_noalloc_max_rows", "xl_peer_reduce_add_rmsnorm", "xl_headwise_proj", "xl_mlstm_decode_cell",
-    "xl_slstm_backward", "xl_slstm_cache_bytes", "xl_slstm_weight_grads", "xl_slstm_weight_grads_scratch_bytes", "xl_rows_linear",
+    "xl_slstm_backward", "xl_slstm_cache_bytes", "xl_slstm_weight_grads", "xl_slstm_weight_grads_scratch_bytes", "xl_rows_linear", "xl_rows_linear_ahead",
 )
 
 
@@ -203,7 +203,7 @@ def lib() -> C.CDLL:
                             ("xl_softcap_argmax", GreedyParams), ("xl_swiglu", SwigluParams),
                             ("xl_softcap_argmax_noalloc", GreedyParams), ("xl_peer_reduce_add_rmsnorm", PeerReduceParams),
                             ("xl_slstm_backward", SlstmBwdParams), ("xl_slstm_weight_grads", SlstmWgradParams),
-                            ("xl_rows_linear", RowsLinearParams)):
+                            ("xl_rows_linear", RowsLinearParams), ("xl_rows_linear_ahead", RowsLinearParams)):
             fn = getattr(l, name)
             fn.restype = C.c_int
             fn.argtypes = [C.POINTER(ptype), C.c_void_p]

@@ -430,10 +430,10 @@ PyObject* add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   END_HANDLE_TH_ERRORS
 }
 
-// (x (..., K), w (N, K)) -> (..., N), bf16, at most 16 rows of x
+// (x (..., K), w (N, K), w_ahead) -> (..., N), bf16, at most 16 rows of x; w_ahead: the caller knows that the launch in front does not write w
 PyObject* rows_linear(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
-  want_args(na, 2);
+  want_args(na, 3);
   const Tensor &x = tensor_arg(a[0], "x"), &w0 = tensor_arg(a[1], "w");
   for (const Tensor* t : {&x, &w0}) require_cuda(t);
   TORCH_CHECK_VALUE(x.scalar_type() == at::kBFloat16 && w0.scalar_type() == at::kBFloat16 && w0.dim() == 2 && x.dim() >= 1 && x.size(-1) == w0.size(1),
@@ -448,7 +448,8 @@ PyObject* rows_linear(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.x = x2.data_ptr(); p.w = w.data_ptr(); p.y = y.data_ptr(); p.status = status_ptr(x);
   p.x_sr = x2.size(0) > 1 ? x2.stride(0) : K; p.w_sr = N > 1 ? w.stride(0) : K;
   p.rows = (int32_t)x2.size(0); p.N = (int32_t)N; p.K = (int32_t)K; p.dtype = XL_BF16;
-  check(xl_rows_linear(&p, stream_of(x)), "xl_rows_linear");
+  const bool ahead = a[2] == Py_True && w.is_same(w0);   // (a copy of w made here is the launch in front)
+  check(ahead ? xl_rows_linear_ahead(&p, stream_of(x)) : xl_rows_linear(&p, stream_of(x)), "xl_rows_linear");
   return THPVariable_Wrap(y);
   END_HANDLE_TH_ERRORS
 }

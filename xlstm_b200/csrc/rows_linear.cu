@@ -3,8 +3,9 @@
 // The whole cost is the stream of W from HBM, so W is the 128-row side of the products and the rows of x the narrow one
 // (D^T [128 features x MB] = W [128 x K] x^T), and the kernel is built around bytes in flight: ~100 KB of TMA stages per
 // block, two blocks per SM, the contraction of a 128-feature tile split over the blocks of a cluster (as many as fill the
-// machine), which add their partial tiles through distributed shared memory in rank order.  W does not depend on the kernel in
-// front, so its first stages are requested before the wait for that kernel: the stream does not stop between the layers.
+// machine), which add their partial tiles through distributed shared memory in rank order.  For a caller who knows that the
+// kernel in front does not write W (xl_rows_linear_ahead), W's first stages are requested before the wait for that kernel: the
+// stream does not stop between the layers.  xl_rows_linear waits first.
 // Eight rows, cold W, a small norm in front of every call, against the library GEMM (us): 4096 x 4096 9.3 / 13.0, 4096 x 10944
 // 18.4 / 27.9, 2048 x 4096 7.5 / 12.1, 2048 x 5504 8.4 / 14.7, 50304 x 4096 67 / 72 (the bytes alone: 5.1, 13.7, 2.6, 3.4, 63).
 // Where 33 to 255 tiles fill the machine unevenly the library is as fast or faster (12304 x 4096: 21.2 / 21.0, 6160 x 2048:
@@ -48,7 +49,7 @@ __device__ __forceinline__ float rl_ld_cluster(uint32_t addr) {
   return v;
 }
 
-__global__ void __launch_bounds__(RL_THREADS) rows_linear_kernel(const __grid_constant__ RlMaps maps, const xl_rows_linear_params p) {
+__global__ void __launch_bounds__(RL_THREADS) rows_linear_kernel(const __grid_constant__ RlMaps maps, const xl_rows_linear_params p, int ahead) {
   using LY = RlLayout;
   constexpr int STAGES = LY::STAGES;
   extern __shared__ unsigned char rl_smem_raw[];
@@ -61,14 +62,16 @@ __global__ void __launch_bounds__(RL_THREADS) rows_linear_kernel(const __grid_co
   const int kb = (p.K + RL_KB - 1) / RL_KB;
   const int first = (int)((long long)kb * part / parts), count = (int)((long long)kb * (part + 1) / parts) - first;
 
-  if (tid == 0) {
-    for (int s = 0; s < 2 * STAGES + 1; ++s) mbar_init(bar0 + 8u * s, 1);
-    fence_barrier_init();
-    // the first stages: W only (what x adds to a stage is announced here as well)
+  auto load_first_w = [&]() {   // one thread: W's part of the first stages (what x adds to a stage is announced here as well)
     for (int c = 0; c < STAGES && c < count; ++c) {
       mbar_expect_tx(bar0 + 8u * c, LY::STAGE_BYTES);
       rl_load(sbase + c * LY::STAGE_BYTES, &maps.w, bar0 + 8u * c, (first + c) * RL_KB, n0);
     }
+  };
+  if (tid == 0) {
+    for (int s = 0; s < 2 * STAGES + 1; ++s) mbar_init(bar0 + 8u * s, 1);
+    fence_barrier_init();
+    if (ahead) load_first_w();
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(s_tmem), LY::TMEM_COLS);
@@ -84,6 +87,7 @@ __global__ void __launch_bounds__(RL_THREADS) rows_linear_kernel(const __grid_co
   bool ok = true;
   if (warp == 0) {
     if (lane == 0) {
+      if (!ahead) load_first_w();
       for (int c = 0; c < STAGES && c < count; ++c)
         rl_load(sbase + c * LY::STAGE_BYTES + RL_W_BYTES, &maps.x, bar0 + 8u * c, (first + c) * RL_KB, 0);
       int st = 0;
@@ -184,7 +188,7 @@ static int rl_make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t K
   return XL_OK;
 }
 
-static int launch_rows_linear(const xl_rows_linear_params* p, cudaStream_t st) {
+static int launch_rows_linear(const xl_rows_linear_params* p, bool ahead, cudaStream_t st) {
   using LY = RlLayout;
   RlMaps maps;
   int rc = rl_make_map(&maps.w, p->w, p->N, p->K, p->w_sr, RL_TILE);
@@ -210,14 +214,11 @@ static int launch_rows_linear(const xl_rows_linear_params* p, cudaStream_t st) {
   attr[1].val.clusterDim.x = parts; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  XL_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, maps, *p));
+  XL_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, maps, *p, ahead ? 1 : 0));
   return check_launch("xl_rows_linear");
 }
 
-}  // namespace xl
-
-extern "C" int xl_rows_linear(const xl_rows_linear_params* p, void* cuda_stream) {
-  using namespace xl;
+static int rows_linear(const xl_rows_linear_params* p, bool ahead, void* cuda_stream) {
   if (!p || !p->x || !p->w || !p->y) return XL_ERR_NULL_POINTER;
   if (p->dtype != XL_BF16) return XL_ERR_BAD_DTYPE;
   if (p->rows <= 0 || p->N <= 0 || p->K <= 0) return XL_ERR_BAD_SHAPE;
@@ -225,5 +226,10 @@ extern "C" int xl_rows_linear(const xl_rows_linear_params* p, void* cuda_stream)
   if (p->x_sr < p->K || p->w_sr < p->K || p->x_sr % 8 || p->w_sr % 8) return XL_ERR_BAD_STRIDE;
   if (!aligned16(p->x) || !aligned16(p->w) || (reinterpret_cast<uintptr_t>(p->y) & 1u)) return XL_ERR_BAD_ALIGNMENT;
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
-  return launch_rows_linear(p, st);
+  return launch_rows_linear(p, ahead, st);
 }
+
+}  // namespace xl
+
+extern "C" int xl_rows_linear(const xl_rows_linear_params* p, void* cuda_stream) { return xl::rows_linear(p, false, cuda_stream); }
+extern "C" int xl_rows_linear_ahead(const xl_rows_linear_params* p, void* cuda_stream) { return xl::rows_linear(p, true, cuda_stream); }

@@ -184,13 +184,13 @@ class LargeModel:
     def _linear(self, x, w):
         """``F.linear(x, w)``.  A few rows (decoding, a last position, a very short prompt) take the weight-streaming kernel where
         it is the faster one (measured: csrc/rows_linear.cu): weights of at least 4 MB with up to 32 tiles of 128 features,
-        which it splits further, or at least 256.  It reads `w` ahead of the kernel launched in front of it, which here is
-        always a norm, the cell or an activation."""
+        which it splits further, or at least 256.  `w` is read ahead of the kernel launched in front, which here is always a
+        norm, the cell or an activation."""
         N, K = w.shape
         if (self.fused and self.dtype == torch.bfloat16 and 0 < x.numel() <= ops.ROWS_LINEAR_MAX * K and N * K >= 1 << 21
-                and (N <= 4096 or N >= 32768) and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0
+                and (N <= 4096 or N >= 32768) and w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0
                 and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))):
-            return ops.rows_linear(x, w)
+            return ops.rows_linear(x, w, w_ahead=True)
         return F.linear(x, w)
 
     def _mlstm_layer(self, blk, x, state, cu_seqlens, slot, reduce: bool = True):

@@ -332,11 +332,12 @@ def headwise_proj(inputs, weights, in_sel=None):
 ROWS_LINEAR_MAX = 16   # rows of x that ``rows_linear`` takes
 
 
-def rows_linear(x, w):
+def rows_linear(x, w, w_ahead: bool = False):
     """``F.linear(x, w)`` for at most 16 rows of x (decoding): bf16 x (..., K) and w (N, K), K a multiple of 8, fp32
-    accumulation; bound by the stream of w.  The kernel launched directly in front on the stream must not be the one that
-    writes w, which is read ahead of that kernel's end."""
-    return native().rows_linear(x, w)
+    accumulation; bound by the stream of w.  ``w_ahead`` is for a caller who knows every launch on the stream: w is then read
+    ahead of the end of the kernel directly in front, which must not be the one that writes w (a weight that stays as it is
+    between steps; a w computed, cast or copied on the line before is not one)."""
+    return native().rows_linear(x, w, bool(w_ahead))
 
 
 def softcap_argmax(logits, cap: float):

@@ -237,6 +237,23 @@ def test_chunkwise_parts_with_masked_tokens(lo, hi, with_state):
         _check(h, st, h_ref, st_ref, TOL_BF16)
 
 
+@pytest.mark.parametrize("S", [400, 2048])   # one block per document, and documents in parts
+@pytest.mark.parametrize("DQ", [64, 128, 256])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_chunkwise_queries_that_are_not_finite_stay_in_their_document(S, DQ, bad):
+    """The tile of a document's last chunk holds the next document's first tokens: a NaN or an infinity among their queries must
+    not enter what the first document's tokens are computed from."""
+    import xlstm_b200
+    q, k, v, i, f = _cuda(*_inputs(66, 1, 8, S, DQ, 256, torch.bfloat16))
+    cu = [0, 20, S]
+    want, st = xlstm_b200.mlstm_sequence(q, k, v, i, f, cu_seqlens=cu, kernel="chunkwise")
+    q[:, :, 30] = bad
+    h, (c, n, m) = xlstm_b200.mlstm_sequence(q, k, v, i, f, cu_seqlens=cu, kernel="chunkwise")
+    xlstm_b200.check_device_status()
+    assert torch.equal(h[:, :, :30], want[:, :, :30]) and torch.equal(h[:, :, 31:], want[:, :, 31:])
+    assert all(torch.equal(a, b) for a, b in zip((c, n, m), st))   # (no state depends on q)
+
+
 def test_chunkwise_packed_documents_longer_than_a_part():
     """Packed rows with documents far above and far below the length of a part, empty ones among them."""
     import xlstm_b200

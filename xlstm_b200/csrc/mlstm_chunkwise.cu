@@ -814,18 +814,23 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       return true;
     };
     if (zero_start) {
+      // the bf16 copy, so that phase A runs in chunk 0 like in any other: a loop bound of its own for the first chunk cost every
+      // chunk of a long document (4 x 8192 tokens: 264 us against 256).  The columns it shares with q.n come last, like a
+      // converted block's: 0 x q is not 0 where q is infinite or NaN.
       const uint32_t z[32] = {};
-      tmem_st_x32(tH, z);
-      tmem_st_x32(tH + 32, z);
-      // ... and the bf16 copy, so that phase A runs in chunk 0 like in any other: a loop bound of its own for the first chunk
-      // cost every chunk of a long document (4 x 8192 tokens: 264 us against 256)
 #pragma unroll 1
-      for (int i = 0; i < DHQK / 2; i += 32) tmem_st_x32(tCb + i, z);
+      for (int i = 0; i + 32 <= DHQK / 2 - (LY::TAIL_SHARED ? 8 : 0); i += 32) tmem_st_x32(tCb + i, z);
+      if constexpr (LY::TAIL_SHARED) {
+        const uint32_t z16[16] = {}, z8[8] = {};
+        tmem_st_x16(tCb + DHQK / 2 - 32, z16);
+        tmem_st_x8(tCb + DHQK / 2 - 16, z8);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) tail[i] = 0u;
+      }
     }
     init_state(2);
     mbar_arrive(bar0 + 8u * BAR_A);  // the accumulator is free for chunk 0
-    if (zero_start) mbar_arrive(bar0 + 8u * BAR_A);
-    else if (!convert_block(0) || !finish_block(0)) ok = false;
+    if ((!zero_start && !convert_block(0)) || !finish_block(0)) ok = false;
     // Denominators of chunk c: ready long before H^T(c) is (they depend on the previous phase of UMMAs only).
     auto denominators_ready = [&](int c) -> bool {
       if (!mbar_wait(bar0 + 8u * BAR_INV, (uint32_t)c & 1u)) return false;

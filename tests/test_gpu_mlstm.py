@@ -254,6 +254,31 @@ def test_chunkwise_queries_that_are_not_finite_stay_in_their_document(S, DQ, bad
     assert all(torch.equal(a, b) for a, b in zip((c, n, m), st))   # (no state depends on q)
 
 
+@pytest.mark.parametrize("NH,S,DQ,DV", [(8, 8192, 256, 512), (16, 16384, 64, 256), (4, 4096, 128, 128), (4, 1000, 64, 128)])
+@pytest.mark.parametrize("f_mean", [3.0, 0.0, -6.0, -12.0])
+def test_chunkwise_part_states_against_64_bits(NH, S, DQ, DV, f_mean):
+    """n and m (formed in fp32) where the final state is that of a part in the middle: it forgets at f_mean but for its last 64
+    tokens, and behind it nothing is forgotten and next to nothing added.  The sums that matter span the ~50 tokens that carry
+    the weight, at 2^-21.4 each (the hardware logarithm's bound): 1.8e-5.  C has weights rounded to bf16."""
+    import xlstm_b200
+    q, k, v, i, f = _cuda(*_inputs(67, 1, NH, S, DQ, DV, torch.bfloat16, f_mean=f_mean))
+    half = S // 128 * 64
+    f[:, :, half - 64:half] += 3.0 - f_mean
+    f[:, :, half:] = 30.0
+    i[:, :, half:] -= 40.0
+    h, (c, n, m) = xlstm_b200.mlstm_sequence(q, k, v, i, f, kernel="chunkwise")
+    xlstm_b200.check_device_status()
+    lf = torch.nn.functional.logsigmoid(f.double())
+    behind = lf.flip(-1).cumsum(-1).flip(-1) - lf
+    m64 = torch.maximum((i.double() + behind).amax(-1), lf.sum(-1))
+    w = torch.exp(i.double() + behind - m64[..., None])
+    n64 = torch.einsum("bns,bnsd->bnd", w, k.double())
+    c64 = torch.einsum("bnsd,bnse->bnde", w[..., None] * k.double(), v.double())
+    assert float((m.double()[..., 0] - m64).abs().max()) <= 1.8e-5
+    assert float((n.double() - n64).norm()) <= 1.8e-5 * float(n64.norm())
+    assert float((c.double() - c64).norm()) <= TOL_BF16 * float(c64.norm())
+
+
 def test_chunkwise_packed_documents_longer_than_a_part():
     """Packed rows with documents far above and far below the length of a part, empty ones among them."""
     import xlstm_b200

@@ -372,20 +372,21 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
   if (it.part > 0) {
     grid_dependency_wait();   // (the first part of a document needs nothing of the launch in front)
     if (warp == 0) {
-      const float2 v = lane < it.part ? split.gm[(long long)(it.slot0 + lane) * p.NH + head] : make_float2(0.f, -INFINITY);
-      float g = v.x;   // inclusive sum over the lanes from here on
+      const double2 v = lane < it.part ? split.gm[(long long)(it.slot0 + lane) * p.NH + head] : make_double2(0., -INFINITY);
+      double from = v.x;   // this part and those behind it
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const float t = __shfl_down_sync(0xffffffffu, g, o);
-        if (lane + o < 32) g += t;
+        const double t = __shfl_down_sync(0xffffffffu, from, o);
+        if (lane + o < 32) from += t;
       }
-      const float mine = v.y + (g - v.x), first = (p.m0 ? p.m0[sidx] : 0.f) + __shfl_sync(0xffffffffu, g, 0);
-      float m = mine;
+      const double behind = __shfl_down_sync(0xffffffffu, from, 1);   // (lane 31 never holds a part)
+      const double mine = lane < it.part ? v.y + behind : -INFINITY, first = (p.m0 ? p.m0[sidx] : 0.f) + __shfl_sync(0xffffffffu, from, 0);
+      float m = (float)mine;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      m = fmaxf(m, first);
-      s_coef[lane] = expf(mine - m);
-      if (lane == 0) { s_coef[CW_MAX_PARTS] = expf(first - m); s_coef[CW_MAX_PARTS + 1] = m; }
+      m = fmaxf(m, (float)first);
+      s_coef[lane] = expf((float)(mine - m));
+      if (lane == 0) { s_coef[CW_MAX_PARTS] = expf((float)(first - m)); s_coef[CW_MAX_PARTS + 1] = m; }
     }
   }
   tc_fence_before();

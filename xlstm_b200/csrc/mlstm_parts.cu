@@ -5,7 +5,7 @@
 // 112 us.  Four heads of 128 x 256: 199 -> 36 us, of 64 x 128: 181 -> 26 us.
 //
 // The part states are a plain product, C_loc^T [128 x DHQK] = (w V)^T K over the tokens of a part, because the gates of the
-// whole part are scanned first: w_l = exp(a_l - mu) with the part's final stabiliser, so there is one frame and nothing is
+// whole part are scanned first: w_l = exp(a_l - mu) with the part's own stabiliser mu, so there is one frame and nothing is
 // rescaled on the way.  Per 64-token chunk that is the four widest UMMAs of the chunkwise kernel (520 cycles of ~3 400), the
 // scaling of v (in place in its TMA stage) and n_loc on the scaling threads, in fp32.  A value slice forms the 64-feature
 // blocks of n_loc whose index is congruent to its own.
@@ -62,7 +62,8 @@ mlstm_part_state_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_
   float* s_w = reinterpret_cast<float*>(smem + LY::OFF_W);
   float* s_red = reinterpret_cast<float*>(smem + LY::OFF_RED);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + LY::OFF_BAR + (3 * PS_STAGES + 2) * 8);
-  __shared__ float s_part[PS_THREADS / 32], s_max[PS_THREADS / 32];
+  __shared__ double s_part[PS_THREADS / 32];
+  __shared__ float s_max[PS_THREADS / 32];
   auto full = [&](int st) { return bar0 + 8u * st; };
   auto scaled = [&](int st) { return bar0 + 8u * (PS_STAGES + st); };
   auto empty = [&](int st) { return bar0 + 8u * (2 * PS_STAGES + st); };
@@ -106,36 +107,41 @@ mlstm_part_state_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_
   if (tid == 0)
     for (int c = 0; c < PS_STAGES && c < chunks; ++c) load_stage(c);   // under the scan
 
-  // ---- gates of the whole part: every thread owns `per` consecutive tokens
+  // ---- gates of the whole part: every thread owns `per` consecutive tokens.  a_l = i_l + (sum of log f over the tokens behind
+  // l in the part), summed from the part's end and in 64 bits: the tokens that matter are those with small sums, and nothing
+  // is a difference.  (As i_l minus the sum up to l, in fp32, the weights of a strongly forgetting part of 2048 tokens and the
+  // part's stabiliser were off by 1e-3; this way the error is that of a chunk's own scan.)
   {
     const int per = (chunks * CW_L + PS_THREADS - 1) / PS_THREADS, t0 = tid * per, t1 = min(t0 + per, chunks * CW_L);
     const float* ig = p.igate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
     const float* fg = p.fgate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
-    float sum = 0.f;
+    double sum = 0.;
 #pragma unroll 4
-    for (int t = t0; t < t1; ++t) {   // s_w[t] <- i_t - (sum of log f from this thread's first token to t)
-      const float iv = ig[t * p.g_st];
+    for (int t = t1 - 1; t >= t0; --t) {   // s_w[t] <- i_t + (sum of log f behind t up to this thread's last token)
+      s_w[t] = (float)(ig[t * p.g_st] + sum);
       sum += fast_log_sigmoid(fg[t * p.g_st]);
-      s_w[t] = iv - sum;
     }
-    float incl = sum;
+    double from = sum;   // this thread's tokens and those of the lanes behind it
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const float x = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += x;
+      const double x = __shfl_down_sync(0xffffffffu, from, o);
+      if (lane + o < 32) from += x;
     }
-    if (lane == 31) s_part[warp] = incl;
+    if (lane == 0) s_part[warp] = from;
+    double behind = __shfl_down_sync(0xffffffffu, from, 1);
+    if (lane == 31) behind = 0.;
     __syncthreads();
-    float before = incl - sum, total = 0.f;
+    double total = 0.;
 #pragma unroll
-    for (int w = 0; w < PS_THREADS / 32; ++w) {
-      if (w < warp) before += s_part[w];
+    for (int w = PS_THREADS / 32 - 1; w >= 0; --w) {
+      if (w > warp) behind += s_part[w];
       total += s_part[w];
     }
     float mx = -INFINITY;
     for (int t = t0; t < t1; ++t) {
-      s_w[t] -= before;
-      mx = fmaxf(mx, s_w[t]);
+      const float al = (float)(s_w[t] + behind);
+      s_w[t] = al;
+      mx = fmaxf(mx, al);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -147,7 +153,7 @@ mlstm_part_state_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_
     // (input gates of -inf throughout, a caller's mask: the part adds nothing, its weights are 0 and its stabiliser is -inf)
     const float frame = mu == -INFINITY ? 0.f : mu;
     for (int t = t0; t < t1; ++t) s_w[t] = __expf(s_w[t] - frame);
-    if (slice == 0 && tid == 0) split.gm[(long long)slot * p.NH + head] = make_float2(total, total + mu);
+    if (slice == 0 && tid == 0) split.gm[(long long)slot * p.NH + head] = make_double2(total, mu);
     __syncthreads();
   }
 
@@ -378,7 +384,7 @@ static SplitScratch scratch_layout(const xl_mlstm_seq_params* p, const CwChoice&
   s.items = packed ? 256 : 0;
   s.slots = s.items + (packed ? up(c.items * (int64_t)sizeof(CwItem)) : 0);
   s.gm = s.slots + (packed ? up(c.slots * (int64_t)sizeof(CwItem)) : 0);
-  s.n_loc = s.gm + up(c.slots * p->NH * (int64_t)sizeof(float2));
+  s.n_loc = s.gm + up(c.slots * p->NH * (int64_t)sizeof(double2));
   s.c_loc = s.n_loc + up(c.slots * p->NH * (int64_t)p->DHQK * 4);
   s.total = s.c_loc + up(c.slots * p->NH * (int64_t)p->DHQK * p->DHV * 4);
   return s;
@@ -406,7 +412,7 @@ int cw_prepare_split(const CwMaps& maps, const xl_mlstm_seq_params* p, void* scr
   const SplitScratch s = scratch_layout(p, c);
   if (scratch_bytes < s.total) return XL_ERR_TOO_LARGE;
   unsigned char* base = static_cast<unsigned char*>(scratch);
-  split->gm = reinterpret_cast<float2*>(base + s.gm);
+  split->gm = reinterpret_cast<double2*>(base + s.gm);
   split->n_loc = reinterpret_cast<float*>(base + s.n_loc);
   split->c_loc = reinterpret_cast<float*>(base + s.c_loc);
   *grid_z = (unsigned)c.items;

@@ -259,12 +259,17 @@ static __device__ __noinline__ void cw_store_state(float* c_out, int DHV, int gr
   }
 }
 
-// PARTS = false: every document is one block's alone.  An instance of its own, because what the parts need (a document looked up,
-// states folded in) took registers from the loops: 4 x 8192 tokens 254.3 -> 251.4 us, 8 x 1000 tokens of 4 x 128/256 29.2 -> 28.1.
-template <int DHQK, bool PARTS>
+// An instance each for documents in parts, whole documents that start from a given state, and whole documents that start from
+// zero (the state then is zeroed, not loaded, folded or converted): what one needs takes registers from the loops of the others.
+// us, against one instance for all whole documents, same run: 4 x 8192 tokens of 8 x 256/512 from zero 285.9 -> 280.4, from a
+// state 309 -> 304; 1 x 203 from zero 13.5 -> 12.5; 16 x 4096 of 4 x 128/256 107 -> 103.
+enum CwKind { CW_PARTS, CW_WHOLE, CW_WHOLE_FROM_ZERO };
+
+template <int DHQK, CwKind KIND>
 __global__ void __launch_bounds__(CW_THREADS, 1)
 mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_params p, const CwSplit split) {
   using LY = CwLayout<DHQK>;
+  constexpr bool PARTS = KIND == CW_PARTS;
   constexpr int NKB = LY::NKB;
   constexpr int NB = NKB;  // 64-feature blocks of the normaliser state n
   static_assert(NB == 1 || NB == 2 || NB == 4, "feature blocks");
@@ -320,8 +325,12 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
   tok0 += (long long)it.first_chunk * CW_L;
   len = last_part ? len - (long long)it.first_chunk * CW_L : (long long)it.chunks * CW_L;
   const long long sidx = (long long)doc * p.NH + head;
-  // From the zero state nothing is converted for chunk 0: T, H^T and the bf16 copy are zeroed.
-  const bool zero_start = it.part == 0 && !p.c0;
+  // The final state leaves through the state and the gate group, or the state group alone: shared, a block ends sooner, and with
+  // 256 features that pays; alone, the gate group's loop keeps the registers (16 x 4096 tokens of 4 x 128/256 107 us shared, 103
+  // alone; 4 x 8192 of 8 x 256/512 from a state 309 and 304, from zero 280 and 305).
+  constexpr bool STORE_SHARED = PARTS || (KIND == CW_WHOLE_FROM_ZERO && DHQK == 256);
+  // From the zero state nothing is converted for chunk 0: T and the bf16 copy are zeroed.
+  const bool zero_start = KIND == CW_WHOLE_FROM_ZERO || (PARTS && it.part == 0 && !p.c0);
 
   if (len <= 0) {  // empty document: the state passes through unchanged
     grid_dependency_wait();
@@ -406,6 +415,15 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
   constexpr int CB_SPLIT = DHQK / 64 >= 2 ? DHQK / 64 - 1 : 1;
 
   auto init_state = [&](int group) {
+    if constexpr (KIND == CW_WHOLE_FROM_ZERO) {   // (the state group alone: T is not read before the UMMAs of chunk 0 add to it)
+      if (group != 1) return;
+      const uint32_t z[32] = {};
+#pragma unroll 1
+      for (int cb = 0; cb < DHQK / 32; ++cb) tmem_st_x32(tC + cb * 32, z);
+      tc_wait_st();
+      tc_fence_before();
+      return;
+    }
     const int dv = (warp & 3) * 32 + lane;
     cw_init_state<DHQK>(p.c0 ? p.c0 + (sidx * DHQK) * DHV + col0 + dv : nullptr, DHV,
                         reinterpret_cast<const float4*>(split.c_loc) + cw_c_loc_offset<DHQK>(p, it.slot0, head, slice) + dv,
@@ -663,7 +681,7 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       if ((lane & 2) == 0) s_inv[jd] = __fdividef(1.f, fmaxf(fabsf(fmaf(dot, qn_scale, (lane & 1) ? rs1 : rs0)), lower) + eps_j);
       mbar_arrive(bar0 + 8u * BAR_INV);
     }
-    if (ok && last_part) {
+    if (STORE_SHARED && ok && last_part) {
       if (mbar_wait(bar0 + 8u * BAR_HC, (uint32_t)(nchunks - 1) & 1u)) store_C(1, back_last);
       else ok = false;
     }
@@ -746,8 +764,23 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       mbar_arrive(bar0 + 8u * (BAR_GEMPTY0 + buf));
     }
     if (ok && last_part) {
-      if (mbar_wait(bar0 + 8u * BAR_HC, (uint32_t)(nchunks - 1) & 1u)) store_C(0, expf(rho_last));
-      else ok = false;
+      if (!mbar_wait(bar0 + 8u * BAR_HC, (uint32_t)(nchunks - 1) & 1u)) {
+        ok = false;
+      } else if constexpr (STORE_SHARED) {
+        store_C(0, expf(rho_last));
+      } else {
+        tc_fence_after();
+        const float back = expf(rho_last);
+        float* c_out = p.c_out + (sidx * DHQK) * DHV + col0 + (warp & 3) * 32 + lane;
+#pragma unroll 1
+        for (int cb = 0; cb < DHQK / 32; ++cb) {
+          uint32_t r[32];
+          tmem_ld_x32(tC + cb * 32, r);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) c_out[(long long)(cb * 32 + i) * DHV] = __uint_as_float(r[i]) * back;
+        }
+      }
     }
   } else if (warp < W_UMMA) {
     // =========================================================================================== epilogue group
@@ -1076,7 +1109,9 @@ template <int DHQK>
 static int launch_chunkwise(const CwMaps& maps, const xl_mlstm_seq_params* p, const CwSplit& split, unsigned grid_z, cudaStream_t st) {
   using LY = CwLayout<DHQK>;
   static_assert(LY::DYN_SMEM <= 227 * 1024, "shared memory budget");
-  auto kern = split.counts || split.parts > 1 ? mlstm_chunkwise_kernel<DHQK, true> : mlstm_chunkwise_kernel<DHQK, false>;
+  auto kern = split.counts || split.parts > 1 ? mlstm_chunkwise_kernel<DHQK, CW_PARTS>
+              : p->c0                         ? mlstm_chunkwise_kernel<DHQK, CW_WHOLE>
+                                              : mlstm_chunkwise_kernel<DHQK, CW_WHOLE_FROM_ZERO>;
   XL_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::DYN_SMEM));
   XL_CUDA_TRY(launch_dependent(kern, dim3(p->DHV / CW_DV, p->NH, grid_z), dim3(CW_THREADS), LY::DYN_SMEM, st, maps, *p, split));
   return check_launch("xl_mlstm_chunkwise");

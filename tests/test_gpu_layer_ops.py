@@ -343,3 +343,42 @@ def test_linear_layers_of_the_model_leave_weights_without_row_order_to_the_libra
         assert torch.equal(model._linear(x, w.t()), torch.nn.functional.linear(x, w.t()))
         torch.cuda.synchronize()
         assert torch.equal(model._linear(x, w), ops.rows_linear(x, w))
+
+
+def test_other_python_threads_run_while_a_launch_waits_for_room_in_the_queue():
+    """Behind a kernel of a second or so a thread launches more than a stream's queue holds, so one of its launches blocks.  The
+    other thread must go on: its longest pause is the interpreter's switch interval, not the rest of that second."""
+    import threading
+    import time
+    import xlstm_b200
+    x = torch.randn(8, 64, device="cuda")
+    xlstm_b200.soft_cap(x, 15.0)
+    torch.cuda.synchronize()
+    e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    torch.cuda._sleep(1000)
+    e[0].record()
+    torch.cuda._sleep(10 ** 7)
+    e[1].record()
+    torch.cuda.synchronize()
+    cycles = int(10 ** 7 * 800 / e[0].elapsed_time(e[1]))   # 0.8 s
+    blocked = []
+
+    def launch():
+        torch.cuda._sleep(cycles)
+        for _ in range(6000):
+            t0 = time.perf_counter()
+            xlstm_b200.soft_cap(x, 15.0)
+            blocked.append(time.perf_counter() - t0)
+
+    t = threading.Thread(target=launch)
+    t.start()
+    pause, last = 0.0, time.perf_counter()
+    while t.is_alive():
+        time.sleep(0.001)
+        now = time.perf_counter()
+        pause, last = max(pause, now - last), now
+    t.join()
+    torch.cuda.synchronize()
+    if max(blocked) < 0.2:
+        pytest.skip("the queue held every launch")
+    assert pause < 0.2, (pause, max(blocked))

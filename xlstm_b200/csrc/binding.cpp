@@ -5,6 +5,8 @@
 // What bounds a small call is the host: the kernels of a decode step or of a short prompt take 3 - 10 us, while the same
 // work in Python (ctypes field by field, a device guard and a stream object per call) took 16 - 25 us.  Therefore plain
 // METH_FASTCALL functions with positional arguments and no argument parser in between, and the allocator called directly.
+// The interpreter lock is given up between the unpacking of the arguments and the wrapping of the results: an allocation or a
+// launch on a full queue may block.
 // No arithmetic happens here and there is no fallback: what the kernels do not cover raises.
 #include <Python.h>
 
@@ -16,6 +18,9 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "../../include/xlstm_b200.h"
 
 namespace {
@@ -23,6 +28,22 @@ namespace {
 using at::Tensor;
 
 constexpr int MAX_DEVICES = 64;
+
+// Gives up the interpreter lock until lock() or the end of the scope (an exception on its way out, too).
+class Unlocked {
+ public:
+  Unlocked() : state_(PyEval_SaveThread()) {}
+  Unlocked(const Unlocked&) = delete;
+  Unlocked& operator=(const Unlocked&) = delete;
+  ~Unlocked() { lock(); }
+  void lock() {
+    if (state_) PyEval_RestoreThread(state_);
+    state_ = nullptr;
+  }
+
+ private:
+  PyThreadState* state_;
+};
 
 // ---------------------------------------------------------------------------------------------- arguments
 const Tensor& tensor_arg(PyObject* o, const char* name) {
@@ -65,12 +86,21 @@ Tensor empty_on(at::IntArrayRef sizes, at::ScalarType dtype, const Tensor& like)
 }
 
 // The status word of a device: one int32 that kernels set when a bounded wait expires.  Lives until the process exits.
-Tensor* status_tensors[MAX_DEVICES];
+// Called without the interpreter lock (the allocation under the mutex may need it).
 Tensor& status_tensor(int64_t index) {
+  static std::mutex mutex;
+  static std::atomic<Tensor*> words[MAX_DEVICES];
   TORCH_CHECK_VALUE(index >= 0 && index < MAX_DEVICES, "device index out of range");
-  if (!status_tensors[index])   // (the interpreter lock is held)
-    status_tensors[index] = new Tensor(at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, (int8_t)index)));
-  return *status_tensors[index];
+  Tensor* word = words[index].load(std::memory_order_acquire);
+  if (!word) {
+    const std::lock_guard<std::mutex> hold(mutex);
+    word = words[index].load(std::memory_order_relaxed);
+    if (!word) {
+      word = new Tensor(at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, (int8_t)index)));
+      words[index].store(word, std::memory_order_release);
+    }
+  }
+  return *word;
 }
 int32_t* status_ptr(const Tensor& like) { return static_cast<int32_t*>(status_tensor(like.device().index()).data_ptr()); }
 
@@ -115,6 +145,9 @@ PyObject* mlstm_sequence(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const Tensor &i0 = tensor_arg(a[3], "i"), &f0 = tensor_arg(a[4], "f");
   const Tensor *c_in = optional_arg(a[5], "c_initial"), *n_in = optional_arg(a[6], "n_initial"), *m_in = optional_arg(a[7], "m_initial");
   const Tensor* cu = optional_arg(a[8], "cu_seqlens");
+  const int64_t docs = int_arg(a[9]), choice = int_arg(a[11]);
+  const double eps = double_arg(a[10]);
+  Unlocked unlocked;
   for (const Tensor* t : {&q0, &k0, &v0, &i0, &f0, c_in, n_in, m_in, cu}) require_cuda(t);
   TORCH_CHECK_VALUE(known_dtype(q0) && k0.scalar_type() == q0.scalar_type() && v0.scalar_type() == q0.scalar_type(),
                     "q,k,v must share a dtype (float32 or bfloat16), got ", q0.scalar_type(), ",", k0.scalar_type(), ",", v0.scalar_type());
@@ -127,14 +160,14 @@ PyObject* mlstm_sequence(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const Tensor q = last_contig(q0), k = last_contig(k0), v = last_contig(v0);
   Tensor i = as_float(i0), f = as_float(f0);
   if (i.strides() != f.strides()) { i = i.contiguous(); f = f.contiguous(); }
-  int64_t kernel = int_arg(a[11]);
+  int64_t kernel = choice;
   if (kernel == 0) {
     bool chunk = q.scalar_type() == at::kBFloat16 && (DQ == 64 || DQ == 128 || DQ == 256) && DV % 128 == 0;
     for (const Tensor* t : {&q, &k, &v})
       chunk = chunk && t->stride(0) % 8 == 0 && t->stride(1) % 8 == 0 && t->stride(2) % 8 == 0 && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0;
     kernel = chunk ? 1 : 2;
   }
-  const int64_t nd = cu ? int_arg(a[9]) : B;
+  const int64_t nd = cu ? docs : B;
   Tensor c0, n0, m0;
   if (c_in) {
     TORCH_CHECK_VALUE(n_in && m_in, "c_initial, n_initial and m_initial must be given together");
@@ -157,13 +190,17 @@ PyObject* mlstm_sequence(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.v_sb = v.stride(0); p.v_sh = v.stride(1); p.v_st = v.stride(2);
   p.h_sb = h.stride(0); p.h_sh = h.stride(1); p.h_st = h.stride(2);
   p.g_sb = i.stride(0); p.g_sh = i.stride(1); p.g_st = i.stride(2);
-  p.eps = (float)double_arg(a[10]); p.dtype = dtype_code(q);
+  p.eps = (float)eps; p.dtype = dtype_code(q);
+  int rc;
   if (kernel == 1) {
     const int64_t bytes = xl_mlstm_chunkwise_scratch_bytes(&p);
     const Tensor scratch = bytes ? empty_on({bytes}, at::kByte, q) : Tensor();   // (stream-ordered: free for the allocator at return)
-    check(xl_mlstm_chunkwise_parts(&p, bytes ? scratch.data_ptr() : nullptr, bytes, stream_of(q)), "xl_mlstm_chunkwise");
+    rc = xl_mlstm_chunkwise_parts(&p, bytes ? scratch.data_ptr() : nullptr, bytes, stream_of(q));
+  } else {
+    rc = xl_mlstm_recurrent(&p, stream_of(q));
   }
-  else check(xl_mlstm_recurrent(&p, stream_of(q)), "xl_mlstm_recurrent");
+  unlocked.lock();
+  check(rc, kernel == 1 ? "xl_mlstm_chunkwise" : "xl_mlstm_recurrent");
   return pack_pair(THPVariable_Wrap(h), pack({c, n, m}));
   END_HANDLE_TH_ERRORS
 }
@@ -232,12 +269,14 @@ PyObject* mlstm_step(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const Tensor &q = tensor_arg(a[0], "q"), &k = tensor_arg(a[1], "k"), &v = tensor_arg(a[2], "v");
   const Tensor &i0 = tensor_arg(a[3], "i"), &f0 = tensor_arg(a[4], "f");
   const Tensor *c = optional_arg(a[5], "c"), *n = optional_arg(a[6], "n"), *m = optional_arg(a[7], "m"), *slot = optional_arg(a[8], "slot");
+  const double eps = double_arg(a[9]);
+  const bool inplace = a[10] == Py_True;
+  Unlocked unlocked;
   for (const Tensor* t : {&q, &k, &v, &i0, &f0, c, n, m}) require_cuda(t);
   const c10::cuda::CUDAGuard guard(q.device());
-  const bool inplace = a[10] == Py_True;
   StepArgs s;
   xl_mlstm_step_params p = {};
-  s.fill(p, q, k, v, c, n, m, slot, double_arg(a[9]), inplace);
+  s.fill(p, q, k, v, c, n, m, slot, eps, inplace);
   auto gate = [&](const Tensor& t) {   // (B,NH) or (B,NH,1), or whatever reshapes to (B,NH)
     const Tensor g = as_float(t);
     const bool direct = (g.dim() == 2 || (g.dim() == 3 && g.size(2) == 1)) && g.size(0) == s.B && g.size(1) == s.NH;
@@ -250,7 +289,9 @@ PyObject* mlstm_step(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.igate = i.const_data_ptr<float>(); p.fgate = f.const_data_ptr<float>();
   p.h_sb = h.stride(0); p.h_sh = h.stride(1);
   p.g_sb = i.stride(0); p.g_sh = i.stride(1);
-  check(xl_mlstm_step(&p, stream_of(q)), "xl_mlstm_step");
+  const int rc = xl_mlstm_step(&p, stream_of(q));
+  unlocked.lock();
+  check(rc, "xl_mlstm_step");
   return s.result(THPVariable_Wrap(h), a[5], inplace);
   END_HANDLE_TH_ERRORS
 }
@@ -263,12 +304,14 @@ PyObject* mlstm_decode_cell(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const Tensor* bias0 = optional_arg(a[4], "gate_bias");
   const Tensor &o0 = tensor_arg(a[6], "ogate"), &w0 = tensor_arg(a[7], "norm_weight");
   const Tensor *c = optional_arg(a[8], "c"), *n = optional_arg(a[9], "n"), *m = optional_arg(a[10], "m"), *slot = optional_arg(a[11], "slot");
+  const double cap = double_arg(a[5]), eps = double_arg(a[12]), norm_eps = double_arg(a[13]);
+  Unlocked unlocked;
   for (const Tensor* t : {&q, &k, &v, &gates0, bias0, &o0, &w0, c, n, m}) require_cuda(t);
   const c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK_VALUE(v.size(-1) <= 1024, "mlstm_decode_cell: head value width above 1024");
   StepArgs s;
   xl_mlstm_decode_cell_params p = {};
-  s.fill(p.step, q, k, v, c, n, m, slot, double_arg(a[12]), true);
+  s.fill(p.step, q, k, v, c, n, m, slot, eps, true);
   const int64_t H = s.NH * s.DV;
   // (B, width) rows with a contiguous last dimension: column slices of a wider projection output as they are
   auto rows = [&](const Tensor& t, int64_t width) {
@@ -284,8 +327,10 @@ PyObject* mlstm_decode_cell(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.gates_raw = gates.data_ptr(); p.gate_bias = bias0 ? bias.data_ptr() : nullptr;
   p.ogate = o.data_ptr(); p.norm_weight = w.data_ptr(); p.hg = hg.data_ptr();
   p.gr_sb = gates.stride(0); p.o_sb = o.stride(0); p.hg_sb = hg.stride(0);
-  p.gate_cap = (float)double_arg(a[5]); p.norm_eps = (float)double_arg(a[13]);
-  check(xl_mlstm_decode_cell(&p, stream_of(q)), "xl_mlstm_decode_cell");
+  p.gate_cap = (float)cap; p.norm_eps = (float)norm_eps;
+  const int rc = xl_mlstm_decode_cell(&p, stream_of(q));
+  unlocked.lock();
+  check(rc, "xl_mlstm_decode_cell");
   return s.result(THPVariable_Wrap(hg), a[8], true);
   END_HANDLE_TH_ERRORS
 }
@@ -297,6 +342,9 @@ PyObject* slstm_forward(PyObject*, PyObject* const* a, Py_ssize_t na) {
   want_args(na, 7);
   const Tensor &wx0 = tensor_arg(a[0], "wx"), &R0 = tensor_arg(a[1], "R"), &bias0 = tensor_arg(a[2], "bias");
   const Tensor *st0 = optional_arg(a[3], "state0"), *cu = optional_arg(a[4], "cu_seqlens");
+  const int64_t docs = int_arg(a[5]);
+  const bool train = a[6] == Py_True;
+  Unlocked unlocked;
   for (const Tensor* t : {&wx0, &R0, &bias0, st0, cu}) require_cuda(t);
   TORCH_CHECK_VALUE(wx0.scalar_type() == at::kBFloat16, "the sLSTM kernel computes on bf16 inputs (fp32 state); cast wx and R to bfloat16");
   TORCH_CHECK_VALUE(wx0.dim() == 3 && R0.dim() == 4, "inconsistent sLSTM shapes");
@@ -316,15 +364,16 @@ PyObject* slstm_forward(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.h_out = out.data_ptr(); p.state_out = st.data_ptr<float>();
   p.cu_seqlens = cu ? cu->const_data_ptr<int32_t>() : nullptr;
   p.status = status_ptr(wx);
-  p.B = B; p.S = S; p.NH = NH; p.DH = DH; p.num_docs = cu ? int_arg(a[5]) : 0; p.dtype = XL_BF16;
-  const bool train = a[6] == Py_True;
+  p.B = B; p.S = S; p.NH = NH; p.DH = DH; p.num_docs = cu ? docs : 0; p.dtype = XL_BF16;
   if (train) {
     const int64_t bytes = xl_slstm_cache_bytes(B, S, NH, DH);
     TORCH_CHECK_VALUE(bytes > 0, "the sLSTM training path needs a head size of 64, 128 or 256");
     cache = empty_on({bytes}, at::kByte, wx);
     p.train_cache = cache.data_ptr();
   }
-  check(xl_slstm_forward(&p, stream_of(wx)), "xl_slstm_forward");
+  const int rc = xl_slstm_forward(&p, stream_of(wx));
+  unlocked.lock();
+  check(rc, "xl_slstm_forward");
   return train ? pack({out, st, cache}) : pack({out, st});
   END_HANDLE_TH_ERRORS
 }
@@ -335,6 +384,7 @@ PyObject* slstm_backward(PyObject*, PyObject* const* a, Py_ssize_t na) {
   want_args(na, 5);
   const Tensor &cache = tensor_arg(a[0], "cache"), &R0 = tensor_arg(a[1], "R"), &dh0 = tensor_arg(a[2], "dh");
   const Tensor *ds = optional_arg(a[3], "dstate_out"), *st0 = optional_arg(a[4], "state0");
+  Unlocked unlocked;
   for (const Tensor* t : {&cache, &R0, &dh0, ds, st0}) require_cuda(t);
   TORCH_CHECK_VALUE(dh0.dim() == 4, "dh must be (B,NH,S,DH)");
   const int64_t B = dh0.size(0), NH = dh0.size(1), S = dh0.size(2), DH = dh0.size(3), H = NH * DH;
@@ -359,7 +409,9 @@ PyObject* slstm_backward(PyObject*, PyObject* const* a, Py_ssize_t na) {
   }
   p.status = status_ptr(dh);
   p.B = B; p.S = S; p.NH = NH; p.DH = DH; p.dtype = XL_BF16;
-  check(xl_slstm_backward(&p, stream_of(dh)), "xl_slstm_backward");
+  const int rc = xl_slstm_backward(&p, stream_of(dh));
+  unlocked.lock();
+  check(rc, "xl_slstm_backward");
   return pack({dwx, ds0});
   END_HANDLE_TH_ERRORS
 }
@@ -370,6 +422,7 @@ PyObject* slstm_weight_grads(PyObject*, PyObject* const* a, Py_ssize_t na) {
   want_args(na, 3);
   const Tensor &dwx = tensor_arg(a[0], "dwx"), &h = tensor_arg(a[1], "h");
   const Tensor* h0 = optional_arg(a[2], "h0");
+  Unlocked unlocked;
   for (const Tensor* t : {&dwx, &h, h0}) {
     require_cuda(t);
     TORCH_CHECK_VALUE(!t || (t->scalar_type() == at::kBFloat16 && t->is_contiguous() && t->device() == dwx.device()),
@@ -388,7 +441,9 @@ PyObject* slstm_weight_grads(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.scratch = bytes ? scratch.data_ptr() : nullptr; p.scratch_bytes = bytes;
   p.status = status_ptr(h);
   p.B = B; p.S = S; p.NH = NH; p.DH = DH; p.dtype = XL_BF16;
-  check(xl_slstm_weight_grads(&p, stream_of(h)), "xl_slstm_weight_grads");
+  const int rc = xl_slstm_weight_grads(&p, stream_of(h));
+  unlocked.lock();
+  check(rc, "xl_slstm_weight_grads");
   return pack({dR, db});
   END_HANDLE_TH_ERRORS
 }
@@ -406,6 +461,9 @@ PyObject* add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   want_args(na, 5);
   const Tensor &x = tensor_arg(a[0], "x"), &w0 = tensor_arg(a[1], "weight");
   const Tensor* y = optional_arg(a[2], "y");
+  const double eps = double_arg(a[3]);
+  const bool inplace = a[4] == Py_True;
+  Unlocked unlocked;
   for (const Tensor* t : {&x, &w0, y}) require_cuda(t);
   TORCH_CHECK_VALUE(known_dtype(x) && w0.scalar_type() == x.scalar_type() && (!y || (y->scalar_type() == x.scalar_type() && y->sizes() == x.sizes())),
                     "add_rmsnorm: x, y and weight must share one dtype (float32 or bfloat16) and x, y one shape");
@@ -414,7 +472,7 @@ PyObject* add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const c10::cuda::CUDAGuard guard(x.device());
   const Tensor x2 = as_rows(x, D), w = w0.contiguous(), y2 = y ? as_rows(*y, D) : Tensor();
   const int64_t rows = x2.size(0);
-  const bool over_x = y && a[4] == Py_True && x2.data_ptr() == x.data_ptr();
+  const bool over_x = y && inplace && x2.data_ptr() == x.data_ptr();
   const Tensor xo = !y || over_x ? x2 : empty_on(x.sizes(), x.scalar_type(), x);
   const Tensor normed = empty_on(x.sizes(), x.scalar_type(), x);
   xl_add_rmsnorm_params p = {};
@@ -424,8 +482,10 @@ PyObject* add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
     p.y = y2.data_ptr(); p.x_out = xo.data_ptr();
     p.y_sr = y2.stride(0); p.xo_sr = over_x ? x2.stride(0) : D;
   }
-  p.eps = (float)double_arg(a[3]); p.dtype = dtype_code(x);
-  check(xl_add_rmsnorm(&p, stream_of(x)), "xl_add_rmsnorm");
+  p.eps = (float)eps; p.dtype = dtype_code(x);
+  const int rc = xl_add_rmsnorm(&p, stream_of(x));
+  unlocked.lock();
+  check(rc, "xl_add_rmsnorm");
   return pack_pair(!y || over_x ? Py_NewRef(a[0]) : THPVariable_Wrap(xo), THPVariable_Wrap(normed));
   END_HANDLE_TH_ERRORS
 }
@@ -435,6 +495,8 @@ PyObject* rows_linear(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   want_args(na, 3);
   const Tensor &x = tensor_arg(a[0], "x"), &w0 = tensor_arg(a[1], "w");
+  const bool w_ahead = a[2] == Py_True;
+  Unlocked unlocked;
   for (const Tensor* t : {&x, &w0}) require_cuda(t);
   TORCH_CHECK_VALUE(x.scalar_type() == at::kBFloat16 && w0.scalar_type() == at::kBFloat16 && w0.dim() == 2 && x.dim() >= 1 && x.size(-1) == w0.size(1),
                     "rows_linear: bfloat16 x (..., K) and w (N, K)");
@@ -448,8 +510,10 @@ PyObject* rows_linear(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.x = x2.data_ptr(); p.w = w.data_ptr(); p.y = y.data_ptr(); p.status = status_ptr(x);
   p.x_sr = x2.size(0) > 1 ? x2.stride(0) : K; p.w_sr = N > 1 ? w.stride(0) : K;
   p.rows = (int32_t)x2.size(0); p.N = (int32_t)N; p.K = (int32_t)K; p.dtype = XL_BF16;
-  const bool ahead = a[2] == Py_True && w.is_same(w0);   // (a copy of w made here is the launch in front)
-  check(ahead ? xl_rows_linear_ahead(&p, stream_of(x)) : xl_rows_linear(&p, stream_of(x)), "xl_rows_linear");
+  const bool ahead = w_ahead && w.is_same(w0);   // (a copy of w made here is the launch in front)
+  const int rc = ahead ? xl_rows_linear_ahead(&p, stream_of(x)) : xl_rows_linear(&p, stream_of(x));
+  unlocked.lock();
+  check(rc, "xl_rows_linear");
   return THPVariable_Wrap(y);
   END_HANDLE_TH_ERRORS
 }
@@ -460,6 +524,8 @@ PyObject* headnorm_gate(PyObject*, PyObject* const* a, Py_ssize_t na) {
   want_args(na, 4);
   const Tensor &h0 = tensor_arg(a[0], "h"), &w0 = tensor_arg(a[2], "weight");
   const Tensor* o0 = optional_arg(a[1], "o_preact");
+  const double eps = double_arg(a[3]);
+  Unlocked unlocked;
   for (const Tensor* t : {&h0, o0, &w0}) require_cuda(t);
   TORCH_CHECK_VALUE(h0.dim() == 4 && known_dtype(h0) && (!o0 || o0->scalar_type() == h0.scalar_type()) && w0.scalar_type() == h0.scalar_type(),
                     "headnorm_gate: h must be (B,NH,S,DH); h, o_preact and weight must share float32 or bfloat16");
@@ -474,8 +540,10 @@ PyObject* headnorm_gate(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.B = B; p.NH = NH; p.S = S; p.DH = DH;
   p.h_sb = h.stride(0); p.h_sh = h.stride(1); p.h_st = h.stride(2);
   if (o0) { p.o = o.data_ptr(); p.o_sb = o.stride(0); p.o_st = o.stride(1); }
-  p.eps = (float)double_arg(a[3]); p.dtype = dtype_code(h);
-  check(xl_headnorm_gate(&p, stream_of(h)), "xl_headnorm_gate");
+  p.eps = (float)eps; p.dtype = dtype_code(h);
+  const int rc = xl_headnorm_gate(&p, stream_of(h));
+  unlocked.lock();
+  check(rc, "xl_headnorm_gate");
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -486,14 +554,17 @@ PyObject* soft_cap(PyObject*, PyObject* const* a, Py_ssize_t na) {
   want_args(na, 4);
   const Tensor& x = tensor_arg(a[0], "x");
   const Tensor* bias0 = optional_arg(a[3], "bias");
+  const double cap = double_arg(a[1]);
+  const int64_t mode = int_arg(a[2]);
+  Unlocked unlocked;
   for (const Tensor* t : {&x, bias0}) require_cuda(t);
   TORCH_CHECK_VALUE(known_dtype(x), "soft_cap: float32 or bfloat16 only");
-  const int64_t cols = x.size(-1), mode = int_arg(a[2]);
+  const int64_t cols = x.size(-1);
   const c10::cuda::CUDAGuard guard(x.device());
   const Tensor x2 = as_rows(x, cols), bias = bias0 ? bias0->contiguous() : Tensor();
   const Tensor out = empty_on(x.sizes(), mode ? at::kFloat : x.scalar_type(), x);
   xl_soft_cap_params p = {};
-  p.x = x2.data_ptr(); p.out = out.data_ptr(); p.n = x.numel(); p.cap = (float)double_arg(a[1]);
+  p.x = x2.data_ptr(); p.out = out.data_ptr(); p.n = x.numel(); p.cap = (float)cap;
   p.dtype = dtype_code(x); p.out_f32 = (int32_t)mode;
   if (x2.size(0) > 0 && (x2.stride(0) != cols || bias0)) {
     p.cols = cols;
@@ -504,7 +575,9 @@ PyObject* soft_cap(PyObject*, PyObject* const* a, Py_ssize_t na) {
       p.bias = bias.data_ptr();
     }
   }
-  check(xl_soft_cap(&p, stream_of(x)), "xl_soft_cap");
+  const int rc = xl_soft_cap(&p, stream_of(x));
+  unlocked.lock();
+  check(rc, "xl_soft_cap");
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -512,6 +585,7 @@ PyObject* soft_cap(PyObject*, PyObject* const* a, Py_ssize_t na) {
 PyObject* swiglu(PyObject*, PyObject* gz_obj) {
   HANDLE_TH_ERRORS
   const Tensor& gz = tensor_arg(gz_obj, "gz");
+  Unlocked unlocked;
   require_cuda(gz);
   TORCH_CHECK_VALUE(known_dtype(gz) && gz.size(-1) % 2 == 0, "swiglu: float32 or bfloat16, even last dimension");
   const int64_t F = gz.size(-1) / 2;
@@ -522,7 +596,9 @@ PyObject* swiglu(PyObject*, PyObject* gz_obj) {
   const Tensor out = empty_on(sizes, gz.scalar_type(), gz);
   xl_swiglu_params p = {};
   p.gz = g2.data_ptr(); p.out = out.data_ptr(); p.rows = g2.size(0); p.F = (int32_t)F; p.gz_row_stride = g2.stride(0); p.dtype = dtype_code(gz);
-  check(xl_swiglu(&p, stream_of(gz)), "xl_swiglu");
+  const int rc = xl_swiglu(&p, stream_of(gz));
+  unlocked.lock();
+  check(rc, "xl_swiglu");
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -533,6 +609,9 @@ PyObject* causal_conv1d(PyObject*, PyObject* const* a, Py_ssize_t na) {
   want_args(na, 6);
   const Tensor &x0 = tensor_arg(a[0], "x"), &w0 = tensor_arg(a[1], "weight");
   const Tensor *bias0 = optional_arg(a[2], "bias"), *cu = optional_arg(a[3], "cu_seqlens");
+  const int64_t docs = int_arg(a[4]);
+  const bool silu = a[5] == Py_True;
+  Unlocked unlocked;
   for (const Tensor* t : {&x0, &w0, bias0, cu}) require_cuda(t);
   TORCH_CHECK_VALUE(x0.dim() == 3 && known_dtype(x0), "causal_conv1d: x must be (B,S,F) in float32 or bfloat16");
   const int64_t B = x0.size(0), S = x0.size(1), F = x0.size(2), K = w0.size(-1);
@@ -545,11 +624,13 @@ PyObject* causal_conv1d(PyObject*, PyObject* const* a, Py_ssize_t na) {
   xl_conv1d_params p = {};
   p.x = x.data_ptr(); p.weight = w.data_ptr(); p.bias = bias0 ? bias.data_ptr() : nullptr; p.out = out.data_ptr();
   p.cu_seqlens = cu ? cu->const_data_ptr<int32_t>() : nullptr;
-  p.B = B; p.S = S; p.F = F; p.K = K; p.num_docs = cu ? int_arg(a[4]) : 0; p.act = a[5] == Py_True;
+  p.B = B; p.S = S; p.F = F; p.K = K; p.num_docs = cu ? docs : 0; p.act = silu;
   p.x_sb = x.stride(0); p.x_st = x.stride(1);
   p.o_sb = out.stride(0); p.o_st = out.stride(1);
   p.dtype = dtype_code(x);
-  check(xl_causal_conv1d(&p, stream_of(x)), "xl_causal_conv1d");
+  const int rc = xl_causal_conv1d(&p, stream_of(x));
+  unlocked.lock();
+  check(rc, "xl_causal_conv1d");
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -572,6 +653,7 @@ PyObject* headwise_proj(PyObject*, PyObject* const* a, Py_ssize_t na) {
     TORCH_CHECK_VALUE(sel >= 0 && sel < nx, "headwise_proj: one to four weights, one or two inputs, in_sel entries index the inputs");
     p.in_sel[j] = (int32_t)sel;
   }
+  Unlocked unlocked;
   TORCH_CHECK_VALUE(ws[0].dim() == 3, "headwise_proj: weights must be bfloat16 (NH, DH, DH)");
   const int64_t NH = ws[0].size(0), DH = ws[0].size(1), D = NH * DH;
   TORCH_CHECK_VALUE(ws[0].size(2) == DH && (DH == 64 || DH == 128 || DH == 256), "headwise_proj: square per-head blocks of 64, 128 or 256 features only");
@@ -596,38 +678,50 @@ PyObject* headwise_proj(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.out = out.data_ptr(); p.out_row_stride = n * D;
   p.status = status_ptr(out);
   p.rows = xs[0].size(0); p.NH = NH; p.DH = DH; p.n_slots = (int32_t)n; p.dtype = XL_BF16;
-  check(xl_headwise_proj(&p, stream_of(out)), "xl_headwise_proj");
+  const int rc = xl_headwise_proj(&p, stream_of(out));
+  unlocked.lock();
+  check(rc, "xl_headwise_proj");
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
 
-// Scratch of the greedy head, once per device (grown when more rows come) and shared by all calls on the device.
-Tensor* greedy_scratch[MAX_DEVICES];
+// Scratch of the greedy head, once per device (grown when more rows come) and shared by all calls on the device.  Called
+// without the interpreter lock.
+Tensor greedy_scratch(int64_t index, int64_t need, const Tensor& like) {
+  static std::mutex mutex;
+  static Tensor* scratch[MAX_DEVICES];
+  TORCH_CHECK_VALUE(index < MAX_DEVICES, "device index out of range");
+  const std::lock_guard<std::mutex> hold(mutex);
+  if (!scratch[index] || scratch[index]->numel() < need) {
+    const int64_t bytes = std::max(need, xl_softcap_argmax_scratch_bytes(256));
+    Tensor* fresh = new Tensor(at::zeros({bytes}, at::TensorOptions().dtype(at::kByte).device(like.device())));
+    delete scratch[index];
+    scratch[index] = fresh;
+  }
+  return *scratch[index];
+}
 
 // (logits, cap) -> int64 tokens of shape logits.shape[:-1]
 PyObject* softcap_argmax(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   want_args(na, 2);
   const Tensor& logits = tensor_arg(a[0], "logits");
+  const double cap = double_arg(a[1]);
+  Unlocked unlocked;
   require_cuda(logits);
   TORCH_CHECK_VALUE(known_dtype(logits), "softcap_argmax: float32 or bfloat16 only");
   const int64_t V = logits.size(-1);
   const c10::cuda::CUDAGuard guard(logits.device());
   const Tensor x = as_rows(logits, V);
   const int64_t rows = x.size(0), need = xl_softcap_argmax_scratch_bytes((int32_t)rows), index = x.device().index();
-  TORCH_CHECK_VALUE(index < MAX_DEVICES, "device index out of range");
-  if (!greedy_scratch[index] || greedy_scratch[index]->numel() < need) {
-    const int64_t bytes = std::max(need, xl_softcap_argmax_scratch_bytes(256));
-    Tensor* fresh = new Tensor(at::zeros({bytes}, at::TensorOptions().dtype(at::kByte).device(x.device())));
-    delete greedy_scratch[index];
-    greedy_scratch[index] = fresh;
-  }
-  const Tensor& sc = *greedy_scratch[index];
+  const Tensor sc = greedy_scratch(index, need, x);
   const Tensor out = empty_on(logits.sizes().slice(0, logits.dim() - 1), at::kLong, x);
   xl_greedy_params p = {};
   p.logits = x.data_ptr(); p.tokens = out.data_ptr<int64_t>(); p.scratch = sc.data_ptr(); p.scratch_bytes = sc.numel();
-  p.rows = (int32_t)rows; p.V = (int32_t)V; p.row_stride = x.stride(0); p.cap = (float)double_arg(a[1]); p.dtype = dtype_code(x);
-  check(xl_softcap_argmax(&p, stream_of(x)), "xl_softcap_argmax");
+  p.rows = (int32_t)rows; p.V = (int32_t)V; p.row_stride = x.stride(0); p.cap = (float)cap; p.dtype = dtype_code(x);
+  const int rc = xl_softcap_argmax(&p, stream_of(x));
+  unlocked.lock();
+  check(rc, "xl_softcap_argmax");
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -671,12 +765,16 @@ PyObject* document_offsets(PyObject*, PyObject* const* a, Py_ssize_t na) {
   want_args(na, 4);
   const std::vector<int64_t> cu = host_integers(a[0]);
   const int64_t B = int_arg(a[1]), S = int_arg(a[2]), n = (int64_t)cu.size();
+  const int64_t device = int_arg(a[3]);
+  Unlocked unlocked;
   TORCH_CHECK_VALUE(n >= 2 && cu.front() == 0 && cu.back() == B * S, "cu_seqlens must start at 0 and end at B*S=", B * S);
   for (int64_t j = 0; j + 1 < n; ++j) {
     TORCH_CHECK_VALUE(cu[j + 1] >= cu[j], "cu_seqlens must be non-decreasing");
     TORCH_CHECK_VALUE(cu[j + 1] == cu[j] || cu[j] / S == (cu[j + 1] - 1) / S, "document [", cu[j], ",", cu[j + 1], ") straddles two rows of length ", S);
   }
-  return pack_pair(THPVariable_Wrap(int32_vector(cu, int_arg(a[3]))), PyLong_FromLongLong(n - 1));
+  const Tensor offsets = int32_vector(cu, device);
+  unlocked.lock();
+  return pack_pair(THPVariable_Wrap(offsets), PyLong_FromLongLong(n - 1));
   END_HANDLE_TH_ERRORS
 }
 
@@ -685,7 +783,8 @@ PyObject* slot_vector(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   want_args(na, 4);
   const std::vector<int64_t> slots = host_integers(a[0]);
-  const int64_t B = int_arg(a[1]), n = int_arg(a[2]);
+  const int64_t B = int_arg(a[1]), n = int_arg(a[2]), device = int_arg(a[3]);
+  Unlocked unlocked;
   TORCH_CHECK_VALUE((int64_t)slots.size() == B, "slot must have one entry per stream (", B, "), got ", slots.size());
   std::vector<bool> taken((size_t)std::max<int64_t>(n, 0), false);
   for (const int64_t s : slots) TORCH_CHECK_VALUE(s < n, "slot entries must be below the pool size ", n);
@@ -694,13 +793,19 @@ PyObject* slot_vector(PyObject*, PyObject* const* a, Py_ssize_t na) {
     TORCH_CHECK_VALUE(!taken[(size_t)s], "two active streams name the same pool row");
     taken[(size_t)s] = true;
   }
-  return THPVariable_Wrap(int32_vector(slots, int_arg(a[3])));
+  const Tensor rows = int32_vector(slots, device);
+  unlocked.lock();
+  return THPVariable_Wrap(rows);
   END_HANDLE_TH_ERRORS
 }
 
 PyObject* status_word(PyObject*, PyObject* index) {
   HANDLE_TH_ERRORS
-  return THPVariable_Wrap(status_tensor(int_arg(index)));
+  const int64_t device = int_arg(index);
+  Unlocked unlocked;
+  const Tensor& word = status_tensor(device);
+  unlocked.lock();
+  return THPVariable_Wrap(word);
   END_HANDLE_TH_ERRORS
 }
 

@@ -299,8 +299,9 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
   const int DHV = p.DHV;
 
   // Behind mlstm_part_state_kernel a document's first part does not wait for it, so all it reads through this path was
-  // complete when that kernel passed its own wait, and is read from L2 (__ldcg, TMA).
+  // complete when that kernel passed its own wait, and is read from L2 (`input`, TMA).
   if (!PARTS || !split.after_states) grid_dependency_wait();
+  auto input = [](const float* x) { return PARTS ? __ldcg(x) : *x; };
 
   // ---- this block's part of a document
   CwItem it;
@@ -403,7 +404,6 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
   // (No early launch of the kernel behind: its blocks waiting on the idle SMs cost this one 12 % at 128 blocks, 250 -> 285 us.)
-  const float m_start = it.part > 0 ? s_coef[CW_MAX_PARTS + 1] : (p.m0 ? __ldcg(p.m0 + sidx) : 0.f);
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;  // tcgen05.ld/st: a warp reaches lanes 32*(warp%4)..+31
   const uint32_t tC = tmem + LY::T_C + lane_base, tCb = tmem + LY::T_CB + lane_base;
   const uint32_t tH = tmem + LY::T_H + lane_base, tS = tmem + LY::T_S + lane_base;
@@ -439,15 +439,15 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
     // Carries the gate recurrence one or two chunks ahead of everybody else: lane L owns tokens 2L and 2L+1.
     const float* ig = p.igate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
     const float* fg = p.fgate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
-    float m_prev = m_start;
+    float m_prev = it.part > 0 ? s_coef[CW_MAX_PARTS + 1] : (p.m0 ? input(p.m0 + sidx) : 0.f);
     float rho = 0.f;
     // Gate loads are issued one chunk ahead, unconditionally and from clamped addresses; the tail mask is applied
     // when the values are used.
     float gi0, gi1, gf0, gf1;
     {
       const long long t0 = 2 * lane, ta = t0 < len ? t0 : len - 1, tb = t0 + 1 < len ? t0 + 1 : len - 1;
-      gi0 = __ldcg(ig + ta * p.g_st); gf0 = __ldcg(fg + ta * p.g_st);
-      gi1 = __ldcg(ig + tb * p.g_st); gf1 = __ldcg(fg + tb * p.g_st);
+      gi0 = input(ig + ta * p.g_st); gf0 = input(fg + ta * p.g_st);
+      gi1 = input(ig + tb * p.g_st); gf1 = input(fg + tb * p.g_st);
     }
 #pragma unroll 1
     for (int chunk = 0; chunk < nchunks; ++chunk) {
@@ -460,8 +460,8 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
       {
         const long long tn = (long long)(chunk + 1) * CW_L + 2 * lane;
         const long long ta = tn < len ? tn : len - 1, tb = tn + 1 < len ? tn + 1 : len - 1;
-        gi0 = __ldcg(ig + ta * p.g_st); gf0 = __ldcg(fg + ta * p.g_st);
-        gi1 = __ldcg(ig + tb * p.g_st); gf1 = __ldcg(fg + tb * p.g_st);
+        gi0 = input(ig + ta * p.g_st); gf0 = input(fg + ta * p.g_st);
+        gi1 = input(ig + tb * p.g_st); gf1 = input(fg + tb * p.g_st);
       }
       const int t0 = 2 * lane, t1 = t0 + 1;
       const float lf0 = (t0 < len_c) ? fast_log_sigmoid(cf0) : 0.f;
@@ -543,7 +543,7 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
     // n(j) and its hi/lo rows for the S product of chunk j+1, and the denominators of chunk j.
     const int g = tid;  // 0..127
     for (int d = g; d < DHQK; d += 128) {
-      float nv = p.n0 ? __ldcg(p.n0 + sidx * DHQK + d) : 0.f;
+      float nv = p.n0 ? input(p.n0 + sidx * DHQK + d) : 0.f;
       if (it.part > 0) {
         nv *= s_coef[CW_MAX_PARTS];
         for (int j = 0; j < it.part; ++j) nv = fmaf(s_coef[j], split.n_loc[((long long)(it.slot0 + j) * p.NH + head) * DHQK + d], nv);

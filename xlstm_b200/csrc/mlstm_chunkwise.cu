@@ -382,7 +382,7 @@ mlstm_chunkwise_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_p
   if (it.part > 0) {
     grid_dependency_wait();   // (the first part of a document needs nothing of the launch in front)
     if (warp == 0) {
-      const double2 v = lane < it.part ? split.gm[(long long)(it.slot0 + lane) * p.NH + head] : make_double2(0., -INFINITY);
+      const float2 v = lane < it.part ? split.gm[(long long)(it.slot0 + lane) * p.NH + head] : make_float2(0.f, -INFINITY);
       double from = v.x;   // this part and those behind it
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {

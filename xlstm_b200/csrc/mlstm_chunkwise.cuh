@@ -45,7 +45,7 @@ struct CwSplit {
   int parts, part_chunks; // equal rows: parts per row (1 = no split) and chunks per part
   float* c_loc;           // [slot][NH][value slice][DHQK / 4][128][4]: what a tensor-memory lane (value column) holds, in 16-byte pieces
   float* n_loc;           // [slot][NH][DHQK]
-  double2* gm;            // [slot][NH]: (sum of log f, stabiliser of the part's own state)
+  float2* gm;             // [slot][NH]: (sum of log f, stabiliser of the part's own state)
 };
 
 __device__ __forceinline__ float fast_log_sigmoid(float x) { return fminf(x, 0.f) - __logf(1.f + __expf(-fabsf(x))); }

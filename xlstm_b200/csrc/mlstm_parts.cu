@@ -62,8 +62,7 @@ mlstm_part_state_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_
   float* s_w = reinterpret_cast<float*>(smem + LY::OFF_W);
   float* s_red = reinterpret_cast<float*>(smem + LY::OFF_RED);
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + LY::OFF_BAR + (3 * PS_STAGES + 2) * 8);
-  __shared__ double s_part[PS_THREADS / 32];
-  __shared__ float s_max[PS_THREADS / 32];
+  __shared__ float s_part[PS_THREADS / 32], s_max[PS_THREADS / 32];
   auto full = [&](int st) { return bar0 + 8u * st; };
   auto scaled = [&](int st) { return bar0 + 8u * (PS_STAGES + st); };
   auto empty = [&](int st) { return bar0 + 8u * (2 * PS_STAGES + st); };
@@ -108,30 +107,30 @@ mlstm_part_state_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_
     for (int c = 0; c < PS_STAGES && c < chunks; ++c) load_stage(c);   // under the scan
 
   // ---- gates of the whole part: every thread owns `per` consecutive tokens.  a_l = i_l + (sum of log f over the tokens behind
-  // l in the part), summed from the part's end and in 64 bits: the tokens that matter are those with small sums, and nothing
-  // is a difference.  (As i_l minus the sum up to l, in fp32, the weights of a strongly forgetting part of 2048 tokens and the
-  // part's stabiliser were off by 1e-3; this way the error is that of a chunk's own scan.)
+  // l in the part), summed from the part's end: the tokens that matter are those with small sums, and nothing is a difference.
+  // (As i_l minus the sum up to l, the weights of a strongly forgetting part of 2048 tokens and the part's stabiliser were off
+  // by 1e-3; this way the error is that of a chunk's own scan.)
   {
     const int per = (chunks * CW_L + PS_THREADS - 1) / PS_THREADS, t0 = tid * per, t1 = min(t0 + per, chunks * CW_L);
     const float* ig = p.igate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
     const float* fg = p.fgate + b * p.g_sb + head * p.g_sh + tok0 * p.g_st;
-    double sum = 0.;
+    float sum = 0.f;
 #pragma unroll 4
     for (int t = t1 - 1; t >= t0; --t) {   // s_w[t] <- i_t + (sum of log f behind t up to this thread's last token)
-      s_w[t] = (float)(ig[t * p.g_st] + sum);
+      s_w[t] = ig[t * p.g_st] + sum;
       sum += fast_log_sigmoid(fg[t * p.g_st]);
     }
-    double from = sum;   // this thread's tokens and those of the lanes behind it
+    float from = sum;   // this thread's tokens and those of the lanes behind it
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const double x = __shfl_down_sync(0xffffffffu, from, o);
+      const float x = __shfl_down_sync(0xffffffffu, from, o);
       if (lane + o < 32) from += x;
     }
     if (lane == 0) s_part[warp] = from;
-    double behind = __shfl_down_sync(0xffffffffu, from, 1);
-    if (lane == 31) behind = 0.;
+    float behind = __shfl_down_sync(0xffffffffu, from, 1);
+    if (lane == 31) behind = 0.f;
     __syncthreads();
-    double total = 0.;
+    float total = 0.f;
 #pragma unroll
     for (int w = PS_THREADS / 32 - 1; w >= 0; --w) {
       if (w > warp) behind += s_part[w];
@@ -139,7 +138,7 @@ mlstm_part_state_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_
     }
     float mx = -INFINITY;
     for (int t = t0; t < t1; ++t) {
-      const float al = (float)(s_w[t] + behind);
+      const float al = s_w[t] + behind;
       s_w[t] = al;
       mx = fmaxf(mx, al);
     }
@@ -153,7 +152,7 @@ mlstm_part_state_kernel(const __grid_constant__ CwMaps maps, const xl_mlstm_seq_
     // (input gates of -inf throughout, a caller's mask: the part adds nothing, its weights are 0 and its stabiliser is -inf)
     const float frame = mu == -INFINITY ? 0.f : mu;
     for (int t = t0; t < t1; ++t) s_w[t] = __expf(s_w[t] - frame);
-    if (slice == 0 && tid == 0) split.gm[(long long)slot * p.NH + head] = make_double2(total, mu);
+    if (slice == 0 && tid == 0) split.gm[(long long)slot * p.NH + head] = make_float2(total, mu);
     __syncthreads();
   }
 
@@ -384,7 +383,7 @@ static SplitScratch scratch_layout(const xl_mlstm_seq_params* p, const CwChoice&
   s.items = packed ? 256 : 0;
   s.slots = s.items + (packed ? up(c.items * (int64_t)sizeof(CwItem)) : 0);
   s.gm = s.slots + (packed ? up(c.slots * (int64_t)sizeof(CwItem)) : 0);
-  s.n_loc = s.gm + up(c.slots * p->NH * (int64_t)sizeof(double2));
+  s.n_loc = s.gm + up(c.slots * p->NH * (int64_t)sizeof(float2));
   s.c_loc = s.n_loc + up(c.slots * p->NH * (int64_t)p->DHQK * 4);
   s.total = s.c_loc + up(c.slots * p->NH * (int64_t)p->DHQK * p->DHV * 4);
   return s;
@@ -412,7 +411,7 @@ int cw_prepare_split(const CwMaps& maps, const xl_mlstm_seq_params* p, void* scr
   const SplitScratch s = scratch_layout(p, c);
   if (scratch_bytes < s.total) return XL_ERR_TOO_LARGE;
   unsigned char* base = static_cast<unsigned char*>(scratch);
-  split->gm = reinterpret_cast<double2*>(base + s.gm);
+  split->gm = reinterpret_cast<float2*>(base + s.gm);
   split->n_loc = reinterpret_cast<float*>(base + s.n_loc);
   split->c_loc = reinterpret_cast<float*>(base + s.c_loc);
   *grid_z = (unsigned)c.items;

@@ -470,3 +470,43 @@ def test_recurrent_with_compiled_head_sizes_equals_the_general_kernel(DQ, S, off
     h1, (c1, n1, m1) = xlstm_b200.mlstm_sequence(pad(q) * ((DQ + 1) / DQ) ** 0.5, pad(k), v, i, f, kernel="recurrent")
     for a, b in ((h, h1), (c, c1[:, :, :DQ]), (n, n1[..., :DQ]), (m, m1)):
         assert float((a - b).norm()) <= TOL_F32 * float(b.norm())
+
+
+def test_chunkwise_without_room_for_its_scratch_keeps_documents_whole():
+    """A packed row of 32768 tokens asks for 37 MB of part states.  With room for the outputs alone the call still works, and
+    equals the C entry without scratch bit for bit."""
+    import ctypes
+    import xlstm_b200
+    from xlstm_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(5)
+    S, NH, DQ, DV = 32768, 8, 256, 512
+    q, k, v, i, f = (torch.randn(1, NH, S, *d, generator=g, device="cuda") for d in ((DQ,), (DQ,), (DV,), (), ()))
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    cu = torch.tensor([0, S], dtype=torch.int32, device="cuda")
+    p = _lib.MlstmSeqParams()
+    p.B, p.NH, p.S, p.DHQK, p.DHV, p.num_docs, p.cu_seqlens = 1, NH, S, DQ, DV, 1, cu.data_ptr()
+    need = _lib.lib().xl_mlstm_chunkwise_scratch_bytes(ctypes.byref(p))
+    assert need > 32 << 20
+    want = [torch.empty(1, NH, S, DV, dtype=torch.bfloat16, device="cuda"), torch.empty(1, NH, DQ, DV, device="cuda"),
+            torch.empty(1, NH, DQ, device="cuda"), torch.empty(1, NH, 1, device="cuda")]
+    p.q, p.k, p.v, p.igate, p.fgate = (t.data_ptr() for t in (q, k, v, i, f))
+    p.h, p.c_out, p.n_out, p.m_out = (t.data_ptr() for t in want)
+    p.status = xlstm_b200.ops.status_word("cuda").data_ptr()
+    p.q_sb, p.q_sh, p.q_st = p.k_sb, p.k_sh, p.k_st = q.stride()[:3]
+    p.v_sb, p.v_sh, p.v_st = p.h_sb, p.h_sh, p.h_st = v.stride()[:3]
+    p.g_sb, p.g_sh, p.g_st = i.stride()
+    p.eps, p.dtype = 1e-6, _lib.XL_BF16
+    assert _lib.lib().xl_mlstm_chunkwise(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    # h is 256 MB, c comes out of a 20 MB block, n and m out of a 2 MB one
+    limit = torch.cuda.memory_reserved() + (256 + 20 + 2 + 8 << 20)
+    ooms = torch.cuda.memory_stats()["num_ooms"]
+    torch.cuda.set_per_process_memory_fraction(limit / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        h, st = xlstm_b200.mlstm_sequence(q, k, v, i, f, cu_seqlens=cu, kernel="chunkwise")
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    xlstm_b200.check_device_status()
+    assert torch.cuda.memory_stats()["num_ooms"] > ooms
+    assert all(torch.equal(a, b) for a, b in zip((h, *st), want))

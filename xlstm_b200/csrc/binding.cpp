@@ -193,8 +193,17 @@ PyObject* mlstm_sequence(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.eps = (float)eps; p.dtype = dtype_code(q);
   int rc;
   if (kernel == 1) {
-    const int64_t bytes = xl_mlstm_chunkwise_scratch_bytes(&p);
-    const Tensor scratch = bytes ? empty_on({bytes}, at::kByte, q) : Tensor();   // (stream-ordered: free for the allocator at return)
+    // (stream-ordered: free for the allocator at return.  Where there is no room for it the documents stay whole, as for callers
+    // of the C entry without scratch.)
+    int64_t bytes = xl_mlstm_chunkwise_scratch_bytes(&p);
+    Tensor scratch;
+    if (bytes) {
+      try {
+        scratch = empty_on({bytes}, at::kByte, q);
+      } catch (const c10::OutOfMemoryError&) {
+        bytes = 0;
+      }
+    }
     rc = xl_mlstm_chunkwise_parts(&p, bytes ? scratch.data_ptr() : nullptr, bytes, stream_of(q));
   } else {
     rc = xl_mlstm_recurrent(&p, stream_of(q));

@@ -234,3 +234,22 @@ def test_slstm_weight_grads_equal_autograd_over_the_oracle():
     # a single step: only the initial h contributes
     dR1, _ = ops.slstm_weight_grads(wx.grad[:, :1], h.detach()[:, :, :1], None)
     assert float(dR1.abs().max()) == 0.0
+
+
+def test_host_vectors_take_one_dimension_only():
+    """Document offsets and slots from the host: lists, and vectors of any number type as their `tolist` reads.  A scalar and a
+    matrix are refused."""
+    from xlstm_b200 import ops
+    for make in (list, torch.tensor, lambda v: torch.tensor(v, dtype=torch.int32), lambda v: torch.tensor(v, dtype=torch.int16),
+                 lambda v: torch.tensor(v, dtype=torch.float64), lambda v: torch.arange(9)[::2][:len(v)]):
+        off, n = ops.prepare_cu_seqlens(make([0, 2, 4]), 1, 4, "cpu")
+        assert n == 2 and off.dtype == torch.int32 and off.tolist() == [0, 2, 4]
+        assert ops.prepare_slots(make([0, 2, 4]), 3, 5, "cpu").tolist() == [0, 2, 4]
+    assert ops.prepare_slots(torch.tensor([2.9, -1.5]), 2, 5, "cpu").tolist() == [2, -1]
+    for bad in (torch.tensor(3), torch.tensor([[3]]), 3, [[3]]):
+        with pytest.raises(TypeError):
+            ops.prepare_slots(bad, 1, 5, "cpu")
+    with pytest.raises(TypeError):
+        ops.prepare_cu_seqlens(torch.tensor([[0, 4]]), 1, 4, "cpu")
+    with pytest.raises(ValueError):
+        ops.prepare_slots(torch.tensor([float("nan")]), 1, 5, "cpu")

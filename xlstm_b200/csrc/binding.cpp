@@ -736,15 +736,23 @@ PyObject* softcap_argmax(PyObject*, PyObject* const* a, Py_ssize_t na) {
 }
 
 // ---------------------------------------------------------------------------------------------- host-side vectors
-// A Python sequence of integers, or an integer tensor on the host.
+// A Python sequence of integers, or a tensor on the host that is one.
 std::vector<int64_t> host_integers(PyObject* o) {
   std::vector<int64_t> out;
+  PyObject* list = nullptr;   // (other tensors go the way their `tolist` goes: numbers truncate, a scalar or a matrix is no sequence of numbers)
   if (THPVariable_Check(o)) {
-    const Tensor t = THPVariable_Unpack(o).to(at::kLong).contiguous();
-    out.assign(t.const_data_ptr<int64_t>(), t.const_data_ptr<int64_t>() + t.numel());
-    return out;
+    const Tensor& t0 = THPVariable_Unpack(o);
+    if (t0.dim() == 1 && (t0.scalar_type() == at::kInt || t0.scalar_type() == at::kLong)) {
+      const Tensor t = t0.to(at::kLong).contiguous();
+      out.assign(t.const_data_ptr<int64_t>(), t.const_data_ptr<int64_t>() + t.numel());
+      return out;
+    }
+    list = PyObject_CallMethod(o, "tolist", nullptr);
+    if (!list) throw python_error();
+    o = list;
   }
   PyObject* seq = PySequence_Fast(o, "a sequence of integers is wanted");
+  Py_XDECREF(list);
   if (!seq) throw python_error();
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
   out.reserve((size_t)n);

@@ -253,3 +253,14 @@ def test_host_vectors_take_one_dimension_only():
         ops.prepare_cu_seqlens(torch.tensor([[0, 4]]), 1, 4, "cpu")
     with pytest.raises(ValueError):
         ops.prepare_slots(torch.tensor([float("nan")]), 1, 5, "cpu")
+
+
+def test_host_vectors_do_not_wrap_to_32_bits():
+    """-2^32 + 5 would be an inactive stream to the check and pool row 5 to the kernel."""
+    from xlstm_b200 import ops
+    assert ops.prepare_slots([-2 ** 31], 1, 8, "cpu").tolist() == [-2 ** 31]
+    for bad in ([-2 ** 32 + 5], torch.tensor([-2 ** 31 - 1])):
+        with pytest.raises(RuntimeError):
+            ops.prepare_slots(bad, 1, 8, "cpu")
+    with pytest.raises(RuntimeError):
+        ops.prepare_cu_seqlens([0, 2 ** 31, 2 ** 32], 2, 2 ** 31, "cpu")

@@ -772,7 +772,10 @@ std::vector<int64_t> host_integers(PyObject* o) {
 Tensor int32_vector(const std::vector<int64_t>& vals, int64_t device) {
   Tensor host = at::empty({(int64_t)vals.size()}, at::TensorOptions().dtype(at::kInt).pinned_memory(device >= 0));
   int32_t* dst = host.data_ptr<int32_t>();
-  for (size_t j = 0; j < vals.size(); ++j) dst[j] = (int32_t)vals[j];
+  for (size_t j = 0; j < vals.size(); ++j) {
+    TORCH_CHECK(vals[j] >= INT32_MIN && vals[j] <= INT32_MAX, vals[j], " does not fit into 32 bits");
+    dst[j] = (int32_t)vals[j];
+  }
   return device < 0 ? host : host.to(at::Device(at::kCUDA, (int8_t)device), at::kInt, /*non_blocking=*/true);
 }
 

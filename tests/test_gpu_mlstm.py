@@ -510,3 +510,26 @@ def test_chunkwise_without_room_for_its_scratch_keeps_documents_whole():
     xlstm_b200.check_device_status()
     assert torch.cuda.memory_stats()["num_ooms"] > ooms
     assert all(torch.equal(a, b) for a, b in zip((h, *st), want))
+
+
+def test_host_vectors_are_refused_under_capture():
+    """A replay would read the host buffer of the capture.  The device forms are captured."""
+    import xlstm_b200
+    q, k, v, i, f = _cuda(*_inputs(68, 2, 2, 64, 64, 128, torch.bfloat16))
+    c, n, m = _cuda(*_state(69, 3, 2, 64, 128))
+    step = lambda slot: xlstm_b200.mlstm_step(q[:, :, 0], k[:, :, 0], v[:, :, 0], i[:, :, 0], f[:, :, 0], c, n, m, slot=slot, inplace=False)
+    seq = lambda cu: xlstm_b200.mlstm_sequence(q, k, v, i, f, cu_seqlens=cu)
+    slot, cu = torch.tensor([2, 0], dtype=torch.int32, device="cuda"), torch.tensor([0, 20, 64, 128], dtype=torch.int32, device="cuda")
+    want = step([2, 0]), seq([0, 20, 64, 128])
+    torch.cuda.synchronize()
+    for call in (lambda: step([2, 0]), lambda: seq([0, 20, 64, 128])):
+        with pytest.raises(RuntimeError, match="CUDA graph"):
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                call()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step(slot), seq(cu)
+    graph.replay()
+    torch.cuda.synchronize()
+    for (h, st), (h1, st1) in zip(got, want):
+        assert torch.equal(h, h1) and all(torch.equal(a, b) for a, b in zip(st, st1))

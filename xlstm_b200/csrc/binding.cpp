@@ -13,6 +13,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -768,8 +769,14 @@ std::vector<int64_t> host_integers(PyObject* o) {
 }
 
 // int32 vector on `device` (index; below 0: the host).  The copy leaves from pinned memory and is not waited for: from
-// pageable memory every packed call synchronised the stream.
+// pageable memory every packed call synchronised the stream.  Not under capture, where that synchronisation was an error.
 Tensor int32_vector(const std::vector<int64_t>& vals, int64_t device) {
+  if (device >= 0) {
+    // (a captured copy would read the host buffer at every replay, long after it has gone to somebody else)
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+    TORCH_CHECK(c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None,
+                "offsets and slots from the host cannot enter a CUDA graph: pass an int32 tensor on the device");
+  }
   Tensor host = at::empty({(int64_t)vals.size()}, at::TensorOptions().dtype(at::kInt).pinned_memory(device >= 0));
   int32_t* dst = host.data_ptr<int32_t>();
   for (size_t j = 0; j < vals.size(); ++j) {

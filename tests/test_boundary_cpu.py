@@ -264,3 +264,19 @@ def test_host_vectors_do_not_wrap_to_32_bits():
             ops.prepare_slots(bad, 1, 8, "cpu")
     with pytest.raises(RuntimeError):
         ops.prepare_cu_seqlens([0, 2 ** 31, 2 ** 32], 2, 2 ** 31, "cpu")
+
+
+def test_binding_of_another_pytorch_is_rebuilt_and_refused(monkeypatch, tmp_path):
+    from xlstm_b200 import _lib, build
+    stamp = tmp_path / "binding.stamp"
+    monkeypatch.setattr(build, "STAMP", str(stamp))
+    assert build._binding_stale() and build.needs_build()   # no record of what it was built for
+    stamp.write_text(build._binding_stamp())
+    assert not build._binding_stale()
+    monkeypatch.setattr(torch, "__version__", "0.0.0+other")
+    assert build._binding_stale() and build.needs_build()
+    monkeypatch.setattr(_lib, "_native", None)
+    with pytest.raises(RuntimeError, match="0.0.0"):
+        _lib.native()
+    monkeypatch.undo()
+    assert _lib.native().built_for == torch.__version__

@@ -171,15 +171,18 @@ def native():
     """The native host path of ``ops`` (csrc/binding.cpp), loaded once; raises if it has not been built."""
     global _native
     if _native is None:
-        import torch  # noqa: F401  (its libraries are what the module is linked against)
+        import torch   # (its libraries are what the module is linked against)
         path = os.path.join(HERE, "_native.so")
         if not os.path.exists(path):
             raise RuntimeError(f"{path} is missing: build it with `python -m xlstm_b200.build` (there is no fallback implementation)")
         lib()
         loader = importlib.machinery.ExtensionFileLoader("xlstm_b200._native", path)
         spec = importlib.util.spec_from_file_location("xlstm_b200._native", path, loader=loader)
-        _native = importlib.util.module_from_spec(spec)
-        loader.exec_module(_native)
+        module = importlib.util.module_from_spec(spec)
+        loader.exec_module(module)
+        if module.built_for != str(torch.__version__):
+            raise RuntimeError(f"{path} was built for PyTorch {module.built_for}, this is {torch.__version__}: run `python -m xlstm_b200.build`")
+        _native = module
     return _native
 
 

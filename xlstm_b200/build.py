@@ -8,7 +8,8 @@ encoder, is looked up at run time) and links the CUDA runtime statically, so
 it loads on a machine without a driver; only launching needs a B200.  The
 binding (`csrc/binding.cpp`, the native host path of `ops.py`) is linked
 against it and against the installed PyTorch.  Sources are compiled one by
-one, in parallel, into `build/`, so a change recompiles only what it touches.
+one, in parallel, into `build/`, so a change recompiles only what it touches;
+another PyTorch or interpreter than the last build's recompiles the binding.
 """
 from __future__ import annotations
 
@@ -25,6 +26,7 @@ OBJ = os.path.join(HERE, "..", "build")
 HEADER = os.path.join(HERE, "..", "include", "xlstm_b200.h")
 LIB = os.path.join(HERE, "libxlstm_b200.so")
 NATIVE = os.path.join(HERE, "_native.so")
+STAMP = os.path.join(OBJ, "binding.stamp")
 SOURCES = ["capi.cu", "mlstm_step.cu", "mlstm_recurrent.cu", "mlstm_chunkwise.cu", "mlstm_parts.cu", "slstm_fwd.cu", "slstm_bwd.cu", "slstm_wgrad.cu", "layer_adjacent.cu", "greedy_head.cu", "peer_reduce.cu", "headwise_proj.cu", "rows_linear.cu"]
 BINDING = "binding.cpp"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -53,16 +55,31 @@ def _headers():
     return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] + [HEADER]
 
 
+def _binding_stamp() -> str:
+    """What the binding is compiled against besides its sources: it is valid for this PyTorch and this interpreter only."""
+    import torch
+    return f"{torch.__version__} {os.path.dirname(torch.__file__)} {sys.version}"
+
+
+def _binding_stale() -> bool:
+    try:
+        with open(STAMP) as fh:
+            return fh.read() != _binding_stamp()
+    except FileNotFoundError:
+        return True
+
+
 def needs_build() -> bool:
     cu = [os.path.join(CSRC, s) for s in SOURCES] + _headers()
-    return _newer(cu, LIB) or _newer([os.path.join(CSRC, BINDING), HEADER], NATIVE)
+    return _newer(cu, LIB) or _newer([os.path.join(CSRC, BINDING), HEADER], NATIVE) or _binding_stale()
 
 
 def _binding_command(obj: str):
     import torch
     inc = os.path.join(os.path.dirname(torch.__file__), "include")
     cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
-    return ["g++", "-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", inc,
+    return ["g++", "-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f'-DXL_BUILT_FOR="{torch.__version__}"', "-I", inc,
             "-I", os.path.join(inc, "torch", "csrc", "api", "include"), "-I", cuda, "-I", sysconfig.get_paths()["include"], "-c",
             os.path.join(CSRC, BINDING), "-o", obj]
 
@@ -80,7 +97,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if force or _newer([src, *_headers()], obj):
             jobs.append([_nvcc(), *extra, *NVCC_FLAGS, "-c", src, "-o", obj])
     bobj = os.path.join(OBJ, BINDING + ".o")
-    if force or _newer([os.path.join(CSRC, BINDING), HEADER], bobj):
+    if force or _newer([os.path.join(CSRC, BINDING), HEADER], bobj) or _binding_stale():
         jobs.append(_binding_command(bobj))
     with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
         for log in pool.map(_run, jobs):
@@ -90,6 +107,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
     _run(["g++", "-shared", "-o", NATIVE, bobj, LIB, "-L", tlib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
           "-Wl,-rpath,$ORIGIN"])
+    with open(STAMP, "w") as fh:
+        fh.write(_binding_stamp())
     return LIB
 
 

@@ -846,4 +846,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Native host path of xls
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__native() {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "built_for", XL_BUILT_FOR) < 0) Py_CLEAR(m);   // the PyTorch it is compiled against
+  return m;
+}

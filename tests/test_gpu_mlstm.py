@@ -499,10 +499,17 @@ def test_chunkwise_without_room_for_its_scratch_keeps_documents_whole():
     assert _lib.lib().xl_mlstm_chunkwise(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
-    # h is 256 MB, c comes out of a 20 MB block, n and m out of a 2 MB one
-    limit = torch.cuda.memory_reserved() + (256 + 20 + 2 + 8 << 20)
+    room = [torch.empty_like(t) for t in want]   # what the outputs will take; everything else is taken now
+    taken = []
+    torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / torch.cuda.get_device_properties(0).total_memory)
+    for size in (256 << 20, 64 << 20, 16 << 20, 4 << 20, 3 << 19):
+        try:
+            while True:
+                taken.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.cuda.OutOfMemoryError:
+            pass
+    del room
     ooms = torch.cuda.memory_stats()["num_ooms"]
-    torch.cuda.set_per_process_memory_fraction(limit / torch.cuda.get_device_properties(0).total_memory)
     try:
         h, st = xlstm_b200.mlstm_sequence(q, k, v, i, f, cu_seqlens=cu, kernel="chunkwise")
     finally:
@@ -533,3 +540,15 @@ def test_host_vectors_are_refused_under_capture():
     torch.cuda.synchronize()
     for (h, st), (h1, st1) in zip(got, want):
         assert torch.equal(h, h1) and all(torch.equal(a, b) for a, b in zip(st, st1))
+
+
+def test_dimensions_of_size_one_in_front_of_the_features():
+    """A step's k and v as (B,NH,1,D) slices of a sequence, a sequence's v as (B,NH,S,1,DHV)."""
+    import xlstm_b200
+    q, k, v, i, f = _cuda(*_inputs(70, 2, 2, 5, 64, 128, torch.bfloat16))
+    c, n, m = _cuda(*_state(71, 2, 2, 64, 128))
+    step = lambda k_, v_: xlstm_b200.mlstm_step(q[:, :, 0], k_, v_, i[:, :, 0], f[:, :, 0], c, n, m, inplace=False)
+    (h, st), (h1, st1) = step(k[:, :, 0], v[:, :, 0]), step(k[:, :, :1], v[:, :, :1])
+    assert h1.shape == h.shape and torch.equal(h, h1) and all(torch.equal(a, b) for a, b in zip(st, st1))
+    (h, st), (h1, st1) = (xlstm_b200.mlstm_sequence(q, k, w, i, f) for w in (v, v[:, :, :, None]))
+    assert h1.shape == h.shape and torch.equal(h, h1) and all(torch.equal(a, b) for a, b in zip(st, st1))

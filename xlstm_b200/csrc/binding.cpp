@@ -82,6 +82,13 @@ Tensor last_contig(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguou
 Tensor as_float(const Tensor& t) { return t.scalar_type() == at::kFloat ? t : t.to(at::kFloat); }
 Tensor float_contig(const Tensor& t) { return as_float(t).contiguous(); }
 
+// `t` without the dimensions of size 1 between its first `lead` and its last
+Tensor drop_units(const Tensor& t, int64_t lead) {
+  Tensor r = t;
+  while (r.dim() > lead + 1 && r.size(lead) == 1) r = r.squeeze(lead);
+  return r;
+}
+
 Tensor empty_on(at::IntArrayRef sizes, at::ScalarType dtype, const Tensor& like) {
   return Tensor(at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt));
 }
@@ -142,14 +149,15 @@ PyObject* pack_pair(PyObject* a, PyObject* b) {
 PyObject* mlstm_sequence(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   want_args(na, 12);
-  const Tensor &q0 = tensor_arg(a[0], "q"), &k0 = tensor_arg(a[1], "k"), &v0 = tensor_arg(a[2], "v");
+  const Tensor &q0 = tensor_arg(a[0], "q"), &k0 = tensor_arg(a[1], "k"), &v_arg = tensor_arg(a[2], "v");
   const Tensor &i0 = tensor_arg(a[3], "i"), &f0 = tensor_arg(a[4], "f");
   const Tensor *c_in = optional_arg(a[5], "c_initial"), *n_in = optional_arg(a[6], "n_initial"), *m_in = optional_arg(a[7], "m_initial");
   const Tensor* cu = optional_arg(a[8], "cu_seqlens");
   const int64_t docs = int_arg(a[9]), choice = int_arg(a[11]);
   const double eps = double_arg(a[10]);
   Unlocked unlocked;
-  for (const Tensor* t : {&q0, &k0, &v0, &i0, &f0, c_in, n_in, m_in, cu}) require_cuda(t);
+  for (const Tensor* t : {&q0, &k0, &v_arg, &i0, &f0, c_in, n_in, m_in, cu}) require_cuda(t);
+  const Tensor v0 = drop_units(v_arg, 3);   // (B,NH,S,1,DHV) is taken, too
   TORCH_CHECK_VALUE(known_dtype(q0) && k0.scalar_type() == q0.scalar_type() && v0.scalar_type() == q0.scalar_type(),
                     "q,k,v must share a dtype (float32 or bfloat16), got ", q0.scalar_type(), ",", k0.scalar_type(), ",", v0.scalar_type());
   TORCH_CHECK_VALUE(q0.dim() == 4 && v0.dim() == 4, "q, k, v must be (B,NH,S,D)");
@@ -222,8 +230,9 @@ struct StepArgs {
   Tensor q, k, v, m_in, slot, c, n, m;
   int64_t B, NH, DQ, DV;
 
-  void fill(xl_mlstm_step_params& p, const Tensor& q0, const Tensor& k0, const Tensor& v0, const Tensor* c0, const Tensor* n0, const Tensor* m0,
+  void fill(xl_mlstm_step_params& p, const Tensor& q0, const Tensor& k_arg, const Tensor& v_arg, const Tensor* c0, const Tensor* n0, const Tensor* m0,
             const Tensor* slot0, double eps, bool inplace) {
+    const Tensor k0 = drop_units(k_arg, 2), v0 = drop_units(v_arg, 2);   // (B,NH,1,D) is taken, too
     TORCH_CHECK_VALUE(q0.dim() == 3 && v0.dim() == 3 && k0.sizes() == q0.sizes() && v0.size(0) == q0.size(0) && v0.size(1) == q0.size(1),
                       "step inputs: q, k (B,NH,DHQK) and v (B,NH,DHV)");
     TORCH_CHECK_VALUE(known_dtype(q0) && k0.scalar_type() == q0.scalar_type() && v0.scalar_type() == q0.scalar_type(),

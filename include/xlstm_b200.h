@@ -96,7 +96,9 @@ int xl_mlstm_chunkwise(const xl_mlstm_seq_params* p, void* cuda_stream);
  * 128-column) chains are cut into parts that run side by side, and packed documents are taken longest first.  `scratch`
  * (device, 16-byte aligned) needs xl_mlstm_chunkwise_scratch_bytes(p) bytes -- a host-only computation from the sizes in
  * `p`, 0 where the split would not pay; contents need not be initialised and are free again when the call's kernels have
- * run.  With scratch == NULL, or where the split would not pay, this is xl_mlstm_chunkwise. */
+ * run.  With scratch == NULL, or where the split would not pay, this is xl_mlstm_chunkwise.  Run to run the results are
+ * the same bits; the cut, and with it the rounding of a document's h and state, depends on B, S and num_docs, where
+ * xl_mlstm_chunkwise gives a document the same bits alone, in a batch and packed. */
 int64_t xl_mlstm_chunkwise_scratch_bytes(const xl_mlstm_seq_params* p);
 int xl_mlstm_chunkwise_parts(const xl_mlstm_seq_params* p, void* scratch, int64_t scratch_bytes, void* cuda_stream);
 

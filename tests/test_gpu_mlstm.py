@@ -472,6 +472,44 @@ def test_recurrent_with_compiled_head_sizes_equals_the_general_kernel(DQ, S, off
         assert float((a - b).norm()) <= TOL_F32 * float(b.norm())
 
 
+def _whole_documents(q, k, v, i, f):
+    """Parameters and outputs of the C entry without scratch: every row one chain."""
+    import ctypes
+    import xlstm_b200
+    from xlstm_b200 import _lib
+    B, NH, S, DQ = q.shape
+    DV = v.shape[3]
+    out = [torch.empty(B, NH, S, DV, dtype=torch.bfloat16, device="cuda"), torch.empty(B, NH, DQ, DV, device="cuda"),
+           torch.empty(B, NH, DQ, device="cuda"), torch.empty(B, NH, 1, device="cuda")]
+    p = _lib.MlstmSeqParams()
+    p.B, p.NH, p.S, p.DHQK, p.DHV, p.num_docs = B, NH, S, DQ, DV, B
+    p.q, p.k, p.v, p.igate, p.fgate = (t.data_ptr() for t in (q, k, v, i, f))
+    p.h, p.c_out, p.n_out, p.m_out = (t.data_ptr() for t in out)
+    p.status = xlstm_b200.ops.status_word("cuda").data_ptr()
+    p.q_sb, p.q_sh, p.q_st = p.k_sb, p.k_sh, p.k_st = q.stride()[:3]
+    p.v_sb, p.v_sh, p.v_st = p.h_sb, p.h_sh, p.h_st = v.stride()[:3]
+    p.g_sb, p.g_sh, p.g_st = i.stride()
+    p.eps, p.dtype = 1e-6, _lib.XL_BF16
+    assert _lib.lib().xl_mlstm_chunkwise(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0
+    return p, out
+
+
+def test_host_buffer_prefill_keeps_documents_whole():
+    """Pieces whose rows would be cut into parts on their own: h and the states are those of the uncut chain, bit for bit."""
+    import ctypes
+    import xlstm_b200
+    from xlstm_b200 import _lib
+    B, NH, S, DQ, DV = 2, 4, 2048, 64, 128
+    q, k, v, i, f = _inputs(72, B, NH, S, DQ, DV, torch.bfloat16)
+    p, want = _whole_documents(*_cuda(q, k, v, i, f))
+    p.B = p.num_docs = 1
+    assert _lib.lib().xl_mlstm_chunkwise_scratch_bytes(ctypes.byref(p)) > 0
+    outs = [torch.empty(t.shape, dtype=t.dtype).pin_memory() for t in want]
+    xlstm_b200.mlstm_sequence_from_host(*(t.pin_memory() for t in (q, k, v, i, f)), *outs)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b.cpu()) for a, b in zip(outs, want))
+
+
 def test_chunkwise_without_room_for_its_scratch_keeps_documents_whole():
     """A packed row of 32768 tokens asks for 37 MB of part states.  With room for the outputs alone the call still works, and
     equals the C entry without scratch bit for bit."""
@@ -483,20 +521,9 @@ def test_chunkwise_without_room_for_its_scratch_keeps_documents_whole():
     q, k, v, i, f = (torch.randn(1, NH, S, *d, generator=g, device="cuda") for d in ((DQ,), (DQ,), (DV,), (), ()))
     q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
     cu = torch.tensor([0, S], dtype=torch.int32, device="cuda")
-    p = _lib.MlstmSeqParams()
-    p.B, p.NH, p.S, p.DHQK, p.DHV, p.num_docs, p.cu_seqlens = 1, NH, S, DQ, DV, 1, cu.data_ptr()
-    need = _lib.lib().xl_mlstm_chunkwise_scratch_bytes(ctypes.byref(p))
-    assert need > 32 << 20
-    want = [torch.empty(1, NH, S, DV, dtype=torch.bfloat16, device="cuda"), torch.empty(1, NH, DQ, DV, device="cuda"),
-            torch.empty(1, NH, DQ, device="cuda"), torch.empty(1, NH, 1, device="cuda")]
-    p.q, p.k, p.v, p.igate, p.fgate = (t.data_ptr() for t in (q, k, v, i, f))
-    p.h, p.c_out, p.n_out, p.m_out = (t.data_ptr() for t in want)
-    p.status = xlstm_b200.ops.status_word("cuda").data_ptr()
-    p.q_sb, p.q_sh, p.q_st = p.k_sb, p.k_sh, p.k_st = q.stride()[:3]
-    p.v_sb, p.v_sh, p.v_st = p.h_sb, p.h_sh, p.h_st = v.stride()[:3]
-    p.g_sb, p.g_sh, p.g_st = i.stride()
-    p.eps, p.dtype = 1e-6, _lib.XL_BF16
-    assert _lib.lib().xl_mlstm_chunkwise(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0
+    p, want = _whole_documents(q, k, v, i, f)
+    p.cu_seqlens = cu.data_ptr()
+    assert _lib.lib().xl_mlstm_chunkwise_scratch_bytes(ctypes.byref(p)) > 32 << 20
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     room = [torch.empty_like(t) for t in want]   # what the outputs will take; everything else is taken now

@@ -145,7 +145,7 @@ PyObject* pack_pair(PyObject* a, PyObject* b) {
 
 // ---------------------------------------------------------------------------------------------- mLSTM over a sequence
 // (q, k, v, i, f, c0, n0, m0, cu_seqlens on the device or None, documents, eps, kernel) -> (h, (c, n, m));
-// kernel: 0 = chosen by shape and dtype, 1 = chunkwise, 2 = recurrent
+// kernel: 0 = chosen by shape and dtype, 1 = chunkwise, 2 = recurrent, 3 = chunkwise with documents whole
 PyObject* mlstm_sequence(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   want_args(na, 12);
@@ -201,10 +201,10 @@ PyObject* mlstm_sequence(PyObject*, PyObject* const* a, Py_ssize_t na) {
   p.g_sb = i.stride(0); p.g_sh = i.stride(1); p.g_st = i.stride(2);
   p.eps = (float)eps; p.dtype = dtype_code(q);
   int rc;
-  if (kernel == 1) {
+  if (kernel != 2) {
     // (stream-ordered: free for the allocator at return.  Where there is no room for it the documents stay whole, as for callers
     // of the C entry without scratch.)
-    int64_t bytes = xl_mlstm_chunkwise_scratch_bytes(&p);
+    int64_t bytes = kernel == 3 ? 0 : xl_mlstm_chunkwise_scratch_bytes(&p);
     Tensor scratch;
     if (bytes) {
       try {
@@ -218,7 +218,7 @@ PyObject* mlstm_sequence(PyObject*, PyObject* const* a, Py_ssize_t na) {
     rc = xl_mlstm_recurrent(&p, stream_of(q));
   }
   unlocked.lock();
-  check(rc, kernel == 1 ? "xl_mlstm_chunkwise" : "xl_mlstm_recurrent");
+  check(rc, kernel != 2 ? "xl_mlstm_chunkwise" : "xl_mlstm_recurrent");
   return pack_pair(THPVariable_Wrap(h), pack({c, n, m}));
   END_HANDLE_TH_ERRORS
 }

@@ -346,7 +346,7 @@ def test_linear_layers_of_the_model_leave_weights_without_row_order_to_the_libra
 
 def test_other_python_threads_run_while_a_launch_waits_for_room_in_the_queue():
     """Behind a kernel of a second or so a thread launches more than a stream's queue holds, so one of its launches blocks.  The
-    other thread must go on: its longest pause is the interpreter's switch interval, not the rest of that second."""
+    other thread must go on: its longest pause is the interpreter's switch interval (and what a busy host adds), not that launch."""
     import threading
     import time
     import xlstm_b200
@@ -380,4 +380,4 @@ def test_other_python_threads_run_while_a_launch_waits_for_room_in_the_queue():
     torch.cuda.synchronize()
     if max(blocked) < 0.2:
         pytest.skip("the queue held every launch")
-    assert pause < 0.2, (pause, max(blocked))
+    assert pause < 0.5 * max(blocked), (pause, max(blocked))

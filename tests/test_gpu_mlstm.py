@@ -529,15 +529,15 @@ def test_chunkwise_without_room_for_its_scratch_keeps_documents_whole():
     room = [torch.empty_like(t) for t in want]   # what the outputs will take; everything else is taken now
     taken = []
     torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / torch.cuda.get_device_properties(0).total_memory)
-    for size in (256 << 20, 64 << 20, 16 << 20, 4 << 20, 3 << 19):
-        try:
-            while True:
-                taken.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
-        except torch.cuda.OutOfMemoryError:
-            pass
-    del room
-    ooms = torch.cuda.memory_stats()["num_ooms"]
     try:
+        for size in (256 << 20, 64 << 20, 16 << 20, 4 << 20, 3 << 19):
+            try:
+                while True:
+                    taken.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.cuda.OutOfMemoryError:
+                pass
+        del room
+        ooms = torch.cuda.memory_stats()["num_ooms"]
         h, st = xlstm_b200.mlstm_sequence(q, k, v, i, f, cu_seqlens=cu, kernel="chunkwise")
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
